@@ -13,6 +13,7 @@
 //                   rounds k_huff_sync_* for archives written by the reference).
 #include <cstdint>
 #include <cstdlib>
+#include <type_traits>
 
 #include "scan.cuh"
 #include "vsz_device.cuh"
@@ -686,6 +687,25 @@ __device__ __forceinline__ uint32_t rd_index(const uint8_t* p, int w) {
     return v;
 }
 
+// The split decoder's image of the tables (HuffTableArgs::win): 1 << kWinBits primary entries, then
+// the first kDec2Smem secondary ones.
+//   (zero << 24) | (symbol << 8) | length   a whole codeword (zero = 1 for symbol 0)
+//   kEntEsc | (off << 8) | (32 - w2)        secondary entry off + the w2 bits after the first kDecBits
+//   kEntEsc                                 neither of them (primary), 0 (secondary): split_long
+constexpr uint32_t kEntEsc = 0x80000000u, kEntZero = 0x01000000u;
+static_assert(kWinBits == kDecBits + 1 && kDec2Max < 32, "one bit of the secondary level joins the primary");
+
+__device__ __forceinline__ uint32_t win_entry(uint32_t e) { return (e >> 8) ? e : e | kEntZero; }
+__device__ __forceinline__ uint32_t win_primary(const uint32_t* table, const uint32_t* table2, uint32_t i) {
+    const uint32_t e = table[i >> 1];
+    if (e & 0x7fu) return win_entry(e);
+    if (!(e & 0x80u)) return kEntEsc;
+    const uint32_t w2 = (e >> 8) & 0xfu, off = e >> 12;
+    const uint32_t e2 = table2[off + ((i & 1u) << (w2 - 1u))];  // the codeword ends with this bit?
+    if ((e2 & 0xffu) == (uint32_t)kWinBits) return win_entry(e2);
+    return off + (1u << w2) <= (uint32_t)kDec2Smem ? kEntEsc | (off << 8) | (32u - w2) : kEntEsc;
+}
+
 // The decode tables of one field, by the whole CTA (1024 threads; returns are block-uniform).
 constexpr int kTableSmemNodes = 4096;
 
@@ -770,6 +790,7 @@ __device__ __forceinline__ void huff_table_run(const HuffTableArgs& a) {
             a.info[0] = 1;  // single-symbol tree: constant output, no bits
             a.info[1] = a.node_sym[0] & 0xffffu;
             a.info[2] = 0;
+            a.info[3] = 0;
         }
         return;
     }
@@ -867,10 +888,24 @@ __device__ __forceinline__ void huff_table_run(const HuffTableArgs& a) {
             }
         }
     }
+    if (a.win) {
+        __syncthreads();
+#pragma unroll
+        for (uint32_t k = 0; k < (1u << kWinBits) / 1024u; k++) {
+            const uint32_t i = k * 1024u + threadIdx.x;
+            a.win[i]         = win_primary(a.table, a.table2, i);
+        }
+        const uint32_t n2 = fits ? min(total, (uint32_t)kDec2Smem) : 0u;
+        for (uint32_t i = threadIdx.x; i < n2; i += 1024u) {
+            const uint32_t e = a.table2[i];
+            a.win[(1u << kWinBits) + i] = (e & 0xffu) ? win_entry(e) : 0u;
+        }
+    }
     if (threadIdx.x == 0) {
         a.info[0] = 0;
         a.info[1] = 0;
         a.info[2] = s_maxlen;
+        a.info[3] = fits ? total : 0u;
     }
 }
 
@@ -1462,6 +1497,245 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// K4b'': split decoder, for fields with fewer chunks than fill the GPU with a lane each.  There
+// the time is one lane's chain of 512 dependent codewords, so a chunk has S lanes here.  Lane i
+// takes the codewords that start in the i-th part of the chunk's bits.  It first decodes from that
+// part's first bit, usually the middle of a codeword; Huffman codes fall into step after a few
+// codewords, so the position it leaves the part at is nearly always the true one.  Each lane then
+// starts again where the lane before it ended, until no start changes (at most S rounds, since a
+// round settles one more lane; one or two in practice).  The codeword counts give every lane's place
+// in the chunk, and a last pass decodes into shared memory, from where the codes are stored whole.
+// About three times the decoding work, S times less of it in a row: 64^3 at 4.4 bits a code 92 -> 27
+// us with S = 16 (8: 37, 32: 21, but 32 is slower from 10 K chunks on).
+//
+// A warp's chunks are consecutive in the stream: their words are loaded once, in bit order, into
+// shared memory (read from global memory where they average more than kSpanBits bits a codeword).
+// Both levels of the tables are in shared memory (win_primary), so the chain never waits for L2.
+// ------------------------------------------------------------------------------------------
+constexpr int kSplitS       = 16;   // lanes per chunk
+constexpr int kSplitThreads = 512;
+constexpr int kSplitBlocks  = 2;    // CTAs per SM
+constexpr int kSpanBits     = 10;
+template <int S>
+struct SplitWarp {
+    static constexpr int kChunks = 32 / S;                                      // chunks per warp
+    static constexpr int kSpan   = kChunks * kChunkSyms * kSpanBits / 32 + 4;   // words
+    // codes of a warp's chunks; lanes write about kChunkSyms / S apart, a word more per such part
+    // keeps them on different banks
+    static constexpr int kPart   = kChunkSyms / S;
+    static constexpr int kOut    = kChunks * (kChunkSyms / 2 + S);              // words
+    uint32_t span[kSpan];
+    uint32_t out[kOut];
+    static __device__ __forceinline__ uint32_t place(uint32_t i) { return i + 2u * (i / (uint32_t)kPart); }
+};
+template <int S>
+constexpr size_t split_smem(int threads) { return 4 * kWinImageWords + (size_t)(threads / 32) * sizeof(SplitWarp<S>); }
+
+// A codeword that the tables in shared memory do not give: the global tables, then the tree bit by
+// bit (up to 64 more bits), from bit p of gb (rem readable bytes).  Returns its entry, or 0 where
+// the bits are not a codeword.  Rare, and kept out of the loops.
+__device__ __noinline__ uint32_t split_long(const uint32_t* table, const uint32_t* table2, const uint32_t* child,
+                                            const uint32_t* node_sym, uint32_t max_nodes, const uint8_t* gb,
+                                            uint32_t rem, uint32_t p) {
+    auto byte_at = [&](uint32_t i) -> uint32_t { return i < rem ? (uint32_t)gb[i] : 0u; };
+    uint32_t w = 0;
+    for (uint32_t k = 0; k < 4; k++) w = (w << 8) | byte_at((p >> 3) + k);
+    w = __funnelshift_l(byte_at((p >> 3) + 4) << 24, w, p & 7u);
+    uint32_t e = table[w >> (32 - kDecBits)];
+    if (e & 0x7fu) return win_entry(e);
+    uint32_t node = e >> 8, used = kDecBits;
+    if (e & 0x80u) {
+        const uint32_t w2 = (e >> 8) & 0xfu;
+        e                 = table2[(e >> 12) + ((w << kDecBits) >> (32u - w2))];
+        if (e & 0xffu) return win_entry(e);
+        node = e >> 8;
+        used = kDecBits + w2;
+    }
+    if (node == 0 || node >= max_nodes) return 0u;
+    for (int d = 0; d < 64; d++) {
+        const uint32_t q = p + used;
+        node = child[2 * (size_t)node + ((byte_at(q >> 3) >> (7u - (q & 7u))) & 1u)];
+        used++;
+        if (node == 0 || node >= max_nodes) return 0u;
+        const uint32_t ns = node_sym[node];
+        if (ns & 0x80000000u) return win_entry(((ns & 0xffffu) << 8) | used);
+    }
+    return 0u;
+}
+
+// Chunks c0 .. c0 + 32 / S - 1 by the calling warp (c0 < a.nchunks).
+template <int S>
+__device__ __forceinline__ void decode_split_warp(const HuffDecodeArgs& a, size_t c0, const uint32_t* s_win,
+                                                  SplitWarp<S>& sw) {
+    using W = SplitWarp<S>;
+    const unsigned lane = threadIdx.x & 31u, seg = lane % S;
+    const size_t j      = c0 + lane / S;
+    const unsigned long long out0 = (unsigned long long)j * kChunkSyms;
+    uint32_t cnt = 0;
+    if (j < a.nchunks && out0 < a.n) cnt = (uint32_t)min((unsigned long long)kChunkSyms, a.n - out0);
+    const uint32_t base0 = (uint32_t)(reinterpret_cast<uintptr_t>(a.payload) & 3u) * 8u;
+    const uint8_t* g4    = reinterpret_cast<const uint8_t*>(reinterpret_cast<uintptr_t>(a.payload) & ~(uintptr_t)3);
+    // readable bytes from g4: the payload plus the 8 bytes past its end that callers provide
+    const unsigned long long readable = base0 / 8u + (a.payload_bits + 7) / 8 + 8;
+    bool bad = false;
+    unsigned long long sb = 0;
+    uint32_t cb = 0;
+    if (cnt) {  // offsets relative to the field's first chunk (a batch scans all fields' indexes at once)
+        sb = a.start_bit[j] - a.start_bit[0];
+        cb = a.chunk_len[j];
+        if (sb + cb > a.payload_bits) bad = true;
+    }
+    // positions are bits from the word that holds the warp's first bit
+    const unsigned long long wb = (base0 + __shfl_sync(0xffffffffu, sb, 0)) >> 5;
+    const uint8_t* gb  = g4 + wb * 4;
+    const uint32_t rem = wb * 4 >= readable ? 0u : (uint32_t)min(readable - wb * 4, 0x7fffffffull);
+    const bool live    = cnt && !bad;
+    const uint32_t p0  = live ? (uint32_t)(base0 + sb - wb * 32) : 0u;
+    const uint32_t pe  = live ? p0 + cb : 0u;
+    const uint32_t nw  = (__reduce_max_sync(0xffffffffu, pe) >> 5) + 2u;  // words a window may read
+    auto word_at = [&](uint32_t i) -> uint32_t {
+        if (4u * i + 4u <= rem) return bswap32(__ldg(reinterpret_cast<const uint32_t*>(gb) + i));
+        uint32_t v = 0;
+        for (uint32_t k = 0; k < 4u; k++) v = (v << 8) | (4u * i + k < rem ? (uint32_t)gb[4u * i + k] : 0u);
+        return v;
+    };
+    const bool in_smem = nw <= (uint32_t)W::kSpan;  // the same for the whole warp
+    if (in_smem) {
+        for (uint32_t i = lane; i < nw; i += 32) sw.span[i] = word_at(i);
+        __syncwarp();
+    }
+    const uint32_t hi = p0 + (seg == S - 1 ? cb : cb * (seg + 1u) / S);
+    auto passes = [&](auto smem_c) {
+        constexpr bool SM = decltype(smem_c)::value;
+        auto entry = [&](uint32_t p) -> uint32_t {  // the codeword at bit p
+            const uint32_t i = p >> 5;
+            const uint32_t w = SM ? __funnelshift_l(sw.span[i + 1], sw.span[i], p)
+                                  : __funnelshift_l(word_at(i + 1), word_at(i), p);
+            uint32_t e = s_win[w >> (32 - kWinBits)];
+            if ((int)e < 0) {
+                uint32_t r = 0;
+                if (e & 31u) r = s_win[(1 << kWinBits) + ((e & ~kEntEsc) >> 8) + __funnelshift_r(w << kDecBits, 0u, e)];
+                if (!(r & 0xffu)) r = split_long(a.table, a.table2, a.child, a.node_sym, a.max_nodes, gb, rem, p);
+                e = r;
+            }
+            return e;
+        };
+        uint32_t n = 0;  // codewords that start in [from, hi)
+        auto walk  = [&](uint32_t from) -> uint32_t {  // their end
+            uint32_t p = from;
+            n          = 0;
+            while (p < hi) {
+                const uint32_t l = entry(p) & 0xffu;
+                p += l ? l : 1u;  // out of step: go on at the next bit
+                n++;
+            }
+            return p;
+        };
+        uint32_t from = p0 + cb * seg / S;
+        uint32_t end  = live ? walk(from) : 0u;
+        // the walk before the current one: in a run of one 2-bit codeword the parts flip between
+        // two starts, round after round, each known after its first walk
+        uint32_t from2 = ~0u, end2 = 0u, n2 = 0u;
+        for (int round = 0; round < S; round++) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, end, 1, S);
+            const bool moved = live && seg != 0 && t != from;
+            if (!__any_sync(0xffffffffu, moved)) break;
+            if (moved) {
+                const uint32_t f = from, e = end, k = n;
+                if (t == from2) {
+                    end = end2;
+                    n   = n2;
+                } else {
+                    end = walk(t);
+                }
+                from  = t;
+                from2 = f;
+                end2  = e;
+                n2    = k;
+            }
+            __syncwarp();
+        }
+        uint32_t incl = n;  // codewords up to and with this lane's
+#pragma unroll
+        for (int o = 1; o < S; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o, S);
+            if (seg >= (unsigned)o) incl += t;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, S - 1, S), last = __shfl_sync(0xffffffffu, end, S - 1, S);
+        if (live && (total != cnt || last != pe)) bad = true;  // a chunk must fill exactly its length
+        uint32_t zeros = 0;
+        if (live && !bad) {
+            uint16_t* out = reinterpret_cast<uint16_t*>(sw.out);
+            uint32_t at   = (lane / S) * kChunkSyms + incl - n, p = from;
+            for (; n; n--, at++) {
+                const uint32_t e = entry(p);
+                if (!(e & 0xffu)) bad = true;
+                p += e & 0xffu;
+                zeros += e >> 24;
+                out[W::place(at)] = (uint16_t)(e >> 8);
+            }
+        }
+        return zeros;
+    };
+    uint32_t zeros = in_smem ? passes(std::true_type{}) : passes(std::false_type{});
+    __syncwarp();
+    if (bad) set_status(a.status, VSZ_ERR_CORRUPT);
+#pragma unroll
+    for (int o = S / 2; o > 0; o >>= 1) zeros += __shfl_xor_sync(0xffffffffu, zeros, o);
+    if (seg == 0 && j < a.nchunks && a.chunk_zero) a.chunk_zero[j] = zeros;
+    // 8 codes a store
+    const unsigned long long first = (unsigned long long)c0 * kChunkSyms;
+    for (uint32_t i = 8u * lane; i < (uint32_t)W::kChunks * kChunkSyms && first + i < a.n; i += 256u) {
+        const uint32_t* s = sw.out + W::place(i) / 2;
+        if (first + i + 8 <= a.n) {
+            *reinterpret_cast<uint4*>(a.codes + first + i) = make_uint4(s[0], s[1], s[2], s[3]);
+        } else {
+            for (uint32_t k = 0; first + i + k < a.n; k++) a.codes[first + i + k] = (uint16_t)(s[k >> 1] >> (16 * (k & 1)));
+        }
+    }
+    __syncwarp();
+}
+
+// The image of one field's tables into shared memory, by the whole CTA.
+__device__ __forceinline__ void split_tables(const HuffDecodeArgs& a, uint32_t* s_win) {
+    const uint32_t n = (1u << kWinBits) + ((min(a.tree_info[3], (uint32_t)kDec2Smem) + 3u) & ~3u);
+    for (uint32_t i = 4u * threadIdx.x; i < n; i += 4u * blockDim.x) cp_async16_zfill(s_win + i, a.win + i, 16u);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+}
+
+// Dynamic shared memory: [table image][SplitWarp per warp] (split_smem bytes).
+template <int S>
+__global__ void __launch_bounds__(kSplitThreads, kSplitBlocks) k_huff_decode_split(HuffDecodeArgs a) {
+    extern __shared__ __align__(16) uint32_t s_split[];
+    if (__syncthreads_or(*a.status != VSZ_OK)) return;  // e.g. the tree failed to parse: no tables
+    split_tables(a, s_split);
+    const unsigned warp = threadIdx.x >> 5;
+    const size_t c0     = (blockIdx.x * (size_t)(blockDim.x >> 5) + warp) * (32 / S);
+    if (c0 < a.nchunks)
+        decode_split_warp<S>(a, c0, s_split, reinterpret_cast<SplitWarp<S>*>(s_split + kWinImageWords)[warp]);
+}
+
+// Many fields: tasks of (field, chunk range), one CTA each.
+template <int S>
+__global__ void __launch_bounds__(kSplitThreads, kSplitBlocks)
+    k_huff_decode_split_batch(const HuffDecodeArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks) {
+    extern __shared__ __align__(16) uint32_t s_split[];
+    const unsigned warp = threadIdx.x >> 5;
+    uint32_t loaded     = 0xffffffffu;  // the field whose tables are in shared memory
+    for (uint32_t t = blockIdx.x; t < ntasks; t += gridDim.x) {
+        const BatchTask tk     = tasks[t];
+        const HuffDecodeArgs& a = args[tk.field];  // read in place: a copy spills
+        if (__syncthreads_or(*a.status != VSZ_OK)) continue;  // the same for the whole CTA
+        if (tk.field != loaded) split_tables(a, s_split);
+        loaded = tk.field;
+        for (size_t c0 = tk.u0 + warp * (32 / S); c0 < tk.u1; c0 += (blockDim.x >> 5) * (32 / S))
+            decode_split_warp<S>(a, c0, s_split, reinterpret_cast<SplitWarp<S>*>(s_split + kWinImageWords)[warp]);
+    }
+}
+
 // One-symbol trees: every code of the chunk is the symbol (src/huffman.hh:348-352); zero counts
 // per chunk for the outlier ranks.
 __global__ void __launch_bounds__(256)
@@ -1487,8 +1761,15 @@ int launch_huff_table_batch(const HuffTableArgs* args, uint32_t nfields, cudaStr
 }
 
 int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks, uint32_t ntasks,
-                             const BatchTask* const_tasks, uint32_t nconst, cudaStream_t st, int num_sms) {
-    if (ntasks) {
+                             const BatchTask* const_tasks, uint32_t nconst, size_t total_chunks, cudaStream_t st, int num_sms) {
+    if (ntasks && total_chunks <= kSplitChunks) {
+        const uint32_t cap  = (uint32_t)num_sms * kSplitBlocks;
+        static std::atomic<unsigned long long> attr{0};
+        smem_limit_once(k_huff_decode_split_batch<kSplitS>, (int)split_smem<kSplitS>(kSplitThreads), attr);
+        k_huff_decode_split_batch<kSplitS><<<ntasks < cap ? ntasks : cap, kSplitThreads,
+                                             split_smem<kSplitS>(kSplitThreads), st>>>(args, tasks, ntasks);
+        count_launch();
+    } else if (ntasks) {
         const uint32_t cap  = (uint32_t)num_sms * kWinMinBlocks;
         const uint32_t grid = ntasks < cap ? ntasks : cap;
         static std::atomic<unsigned long long> attr{0};
@@ -1751,12 +2032,23 @@ int launch_huff_table(HuffTableArgs a, cudaStream_t st) {
     return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }
 
-int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st) {
+int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms) {
     if (a.nchunks == 0) return VSZ_OK;
     int grid = (int)((a.nchunks + 255) / 256);
     const bool indexed = !a.out_begin && !a.nsym && a.chunk_syms == (uint32_t)kChunkSyms &&
                          (reinterpret_cast<uintptr_t>(a.codes) & 15u) == 0 && a.chunk_len;
-    if (indexed) {
+    if (indexed && a.tree_info && a.win) {
+        // whole warps over as many SMs as there are, at most kSplitThreads to a copy of the tables
+        constexpr int kPer = 32 / kSplitS;  // chunks per warp
+        const size_t warps = (a.nchunks + kPer - 1) / kPer;
+        const size_t want  = (warps + (size_t)num_sms * kSplitBlocks - 1) / ((size_t)num_sms * kSplitBlocks);
+        const int threads  = 32 * (int)min((size_t)kSplitThreads / 32, max((size_t)4, want));
+        static std::atomic<unsigned long long> attr{0};
+        smem_limit_once(k_huff_decode_split<kSplitS>, (int)split_smem<kSplitS>(kSplitThreads), attr);
+        k_huff_decode_split<kSplitS><<<(unsigned)((warps * 32 + threads - 1) / threads), threads,
+                                       split_smem<kSplitS>(threads), st>>>(a);
+        count_launch();
+    } else if (indexed) {
         if (a.tree_info) {
             static std::atomic<unsigned long long> attr_win{0};
             smem_limit_once(k_huff_decode_win, (int)kWinSmem, attr_win);

@@ -139,6 +139,7 @@ struct DecompressWs {
     uint32_t* parent;
     uint32_t* walk;
     uint32_t* tinfo;
+    uint32_t* win;
     uint16_t* code;
     uint32_t* seg_zero;
     unsigned long long* seg_off;
@@ -178,6 +179,7 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
     w.parent   = b.take<uint32_t>(maxn);
     w.walk     = b.take<uint32_t>(maxn);
     w.tinfo    = b.take<uint32_t>(4);
+    w.win      = b.take<uint32_t>(n_index_chunks && n_index_chunks <= kSplitMaxChunks ? kWinImageWords : 4);
     w.code     = b.take<uint16_t>(g.n + 8);
     uint32_t nxs = (g.d0 + 255) / 256;
     size_t nsegd = g.nrows * nxs;
@@ -231,6 +233,9 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     ta.walk = w.walk;
     ta.table2 = w.table2;
     ta.info = w.tinfo;
+    // the split decoder's tables, for fields that take it (it copies them 16 bytes at a time)
+    const bool split = chunk_bits && huff_split_applies(n_index_chunks, pbits) && (reinterpret_cast<uintptr_t>(w.win) & 15u) == 0;
+    ta.win = split ? w.win : nullptr;
     ta.status = w.status;
     {
         StageTimer t(kStDecTable, st);
@@ -253,6 +258,7 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     da.d0 = d0;
     da.nxs = nxs;
     da.max_nodes = (uint32_t)(2 * dict - 1);
+    da.win = ta.win;
     da.walk = w.walk;
     da.nodes = node_count;
     da.walk_smem = (dict <= 16384 && node_count < 32768u) ? 1 : 0;
@@ -274,7 +280,7 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
         da.nchunks = n_index_chunks;
         da.chunk_syms = chunk_syms;
         StageTimer t(kStHuffDecode, st);
-        return launch_huff_decode(da, st);
+        return launch_huff_decode(da, st, num_sms());
     }
     // self-synchronising path
     HuffSyncArgs sa{};
@@ -317,7 +323,7 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     da.nsym = w.s_count;
     da.nchunks = sa.nchunks;
     da.chunk_syms = 0;
-    return launch_huff_decode(da, st);
+    return launch_huff_decode(da, st, num_sms());
 }
 
 // ---- Huffman tree on the host, stream-ordered ---------------------------------------------------

@@ -37,7 +37,8 @@ constexpr size_t kDCtlConsts = 0;   // Consts (<= 64 bytes)
 constexpr size_t kDCtlStatus = 64;  // int
 constexpr size_t kDCtlInfo   = 80;  // u32[4] tree info (k_huff_table)
 
-constexpr uint64_t kDecTaskChunks = 256;      // one decoder CTA: lane t decodes chunk u0 + t
+constexpr uint64_t kDecTaskChunks = 256;      // one decoder CTA: lane t decodes chunk u0 + t, or
+constexpr uint64_t kSplitTaskChunks = 64;     // (split decoder) its warps take two chunks at a time
 constexpr uint64_t kCopyTaskBytes = 1 << 18;  // index and outlier copies
 constexpr uint64_t kDqTaskUnits   = 1;        // reverse-Lorenzo warp units per task (one warp's)
 constexpr size_t kDqNextOff       = 64;       // after the batch status in the control tail: one
@@ -160,7 +161,7 @@ struct DLayout {
     uint32_t* all_zero;
     unsigned long long* scan_status;
     uint32_t* scan_counter;
-    std::vector<uint32_t*> table, table2, child, node_sym, parent, walk, redo;
+    std::vector<uint32_t*> table, table2, win, child, node_sym, parent, walk, redo;
     std::vector<uint16_t*> code;
     std::vector<float*> outliers;
     std::vector<size_t> chunk_base;
@@ -188,6 +189,7 @@ DLayout layout_dbatch(const std::vector<DField>& fs, const vsz_dbatch_field* fie
         const DField& f     = fs[i];
         const uint32_t maxn = (uint32_t)(2 * f.nsym);
         L.table.push_back(b.take<uint32_t>(1u << kDecBits));
+        L.win.push_back(T <= kSplitChunks ? b.take<uint32_t>(kWinImageWords) : nullptr);
         L.table2.push_back(b.take<uint32_t>(table2_capacity(maxn - 1)));
         L.child.push_back(b.take<uint32_t>(2 * (size_t)maxn));
         L.node_sym.push_back(b.take<uint32_t>(maxn));
@@ -310,6 +312,7 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         t.parent         = L.parent[f];
         t.walk           = L.walk[f];
         t.table2         = L.table2[f];
+        t.win            = L.win[f];
         t.info           = info;
         t.status         = status;
 
@@ -318,6 +321,7 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         h.payload         = F.d_archive + d.payload_offset;
         h.payload_bits    = (unsigned long long)d.payload_bytes * 8ull;
         h.table           = t.table;
+        h.win             = t.win;
         h.table2          = t.table2;
         h.child           = t.child;
         h.node_sym        = t.node_sym;
@@ -360,16 +364,18 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         ck[f] = DCheck{L.all_zoff + base, G.nch, d.n_outlier, consts, status, d_status + f, L.redo[f]};
     }
     // ---- task lists
+    B->total_chunks       = L.chunk_base.empty() ? 0 : L.chunk_base.back() + fs.back().nch;
+    const uint64_t dec_per = B->total_chunks <= kSplitChunks ? kSplitTaskChunks : kDecTaskChunks;
     B->idx_off = (uint32_t)tasks.size();
     for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, 2 * fs[f].nch, kCopyTaskBytes);
     B->idx_n   = (uint32_t)tasks.size() - B->idx_off;
     B->dec_off = (uint32_t)tasks.size();
     for (uint32_t f = 0; f < nf; f++)
-        if (!fs[f].konst) add_tasks(tasks, f, fs[f].nch, kDecTaskChunks);
+        if (!fs[f].konst) add_tasks(tasks, f, fs[f].nch, dec_per);
     B->dec_n     = (uint32_t)tasks.size() - B->dec_off;
     B->const_off = (uint32_t)tasks.size();
     for (uint32_t f = 0; f < nf; f++)
-        if (fs[f].konst) add_tasks(tasks, f, fs[f].nch, kDecTaskChunks);
+        if (fs[f].konst) add_tasks(tasks, f, fs[f].nch, dec_per);
     B->const_n = (uint32_t)tasks.size() - B->const_off;
     B->out_off = (uint32_t)tasks.size();
     for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, 4 * fields[f].desc.n_outlier, kCopyTaskBytes);
@@ -438,7 +444,6 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     B->all_start    = L.all_start;
     B->all_zero     = L.all_zero;
     B->all_zoff     = L.all_zoff;
-    B->total_chunks = L.chunk_base.empty() ? 0 : L.chunk_base.back() + fs.back().nch;
     B->scan_status  = L.scan_status;
     B->scan_counter = L.scan_counter;
     *out            = B;
@@ -478,7 +483,7 @@ vsz_status vsz_dbatch_decompress(vsz_dbatch* B, void* stream) {
     {
         StageTimer t(kStHuffDecode, st);
         VSZ_TRY(launch_huff_decode_batch(B->dec, B->tasks + B->dec_off, B->dec_n, B->tasks + B->const_off,
-                                         B->const_n, st, sms));
+                                         B->const_n, B->total_chunks, st, sms));
     }
     {
         StageTimer t(kStZeroScan, st);

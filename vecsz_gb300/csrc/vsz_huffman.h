@@ -27,6 +27,19 @@ __host__ __device__ inline size_t table2_capacity(uint32_t max_nodes) {
     const size_t leaves = ((size_t)max_nodes + 1) / 2;
     return ((size_t)(1u << kDec2Max) * leaves + 8) / 9 + 256;
 }
+// The split decoder's tables in shared memory: a primary table one bit wider and the first
+// entries of the secondary one (a 1024-symbol tree of a smooth field has 2.5-4.3 K of them).
+constexpr int kWinBits     = 13;
+constexpr int kDec2Smem    = 3072;
+constexpr size_t kWinImageWords = ((size_t)1 << kWinBits) + kDec2Smem;
+// Whether a stream takes the split decoder (k_huff_decode_split).  It costs about 4 us per 1024
+// chunks over a floor of 20; a lane per chunk costs one lane's chain, 75 us at 1-2 bits a code and
+// 160 at 7 (its secondary table is in L2): 64^3 (512 chunks) 92 -> 27 us, 333x241x187 (29 K chunks, 7 bits)
+// 161 -> 125, but 3600x1800 (12.7 K chunks, 1.5 bits) 75 -> 78.
+constexpr size_t kSplitChunks = size_t(1) << 13, kSplitMaxChunks = size_t(1) << 15;
+inline bool huff_split_applies(size_t nchunks, unsigned long long payload_bits) {
+    return nchunks <= kSplitChunks || (nchunks <= kSplitMaxChunks && payload_bits / 4 >= nchunks * 512);
+}
 constexpr int kChunkSyms   = 512;  // codewords per entry of this library's decode index
 constexpr int kSyncBits    = 8192; // chunk size (bits) of the self-synchronising decoder
 
@@ -85,7 +98,9 @@ struct HuffTableArgs {
     uint32_t* walk;       // max_nodes: both children of an internal node, 16 bits each:
                           // 0x8000 | symbol for a leaf, else the node index (dict <= 16384)
     uint32_t* table2;     // table2_capacity(max_nodes) secondary entries
+    uint32_t* win;        // kWinImageWords, 16-byte aligned: the split decoder's tables, or null
     uint32_t* info;       // [0] single-symbol tree flag [1] its symbol [2] longest codeword (255: > 64)
+                          // [3] entries of table2
     int* status;
 };
 
@@ -111,6 +126,7 @@ struct HuffDecodeArgs {
     uint32_t* seg_zero;                   // zero codes per 256-wide row segment (may be null)
     uint32_t d0, nxs;
     uint32_t max_nodes;                   // node indices past this are a corrupt tree
+    const uint32_t* win;                  // k_huff_table's image for the split decoder, or null
     const uint32_t* tree_info;            // k_huff_table's info ([2] longest codeword), or null
     int* status;
 };
@@ -154,8 +170,9 @@ int launch_huff_table(HuffTableArgs a, cudaStream_t st);
 // constant fill.
 int launch_huff_table_batch(const HuffTableArgs* args, uint32_t nfields, cudaStream_t st, int num_sms);
 int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks, uint32_t ntasks,
-                             const BatchTask* const_tasks, uint32_t nconst, cudaStream_t st, int num_sms);
-int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st);
+                             const BatchTask* const_tasks, uint32_t nconst, size_t total_chunks, cudaStream_t st,
+                             int num_sms);
+int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms);
 int launch_huff_const(uint16_t* codes, size_t n, const uint32_t* info, uint32_t* seg_zero, uint32_t d0, uint32_t nxs,
                       const int* status, cudaStream_t st, int num_sms);
 int launch_huff_sync_init(HuffSyncArgs a, cudaStream_t st);
