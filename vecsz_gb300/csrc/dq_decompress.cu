@@ -9,9 +9,10 @@
 //   s = code == 0 ? outlier : (float)(pred + (float)(code - R))
 //   pred: 1D s[x-1]; 2D (N + W) - NW; 3D XYZ - XY - XZ - YZ + X + Y + Z, left to right
 //   xhat = (float)((double) s * 2eb)                 (dequant(), vsz_device.cuh)
-// The outlier of an element with code 0 is found by its rank among the zero codes in row-major
-// order: seg_off[row segment of 256 columns] (an exclusive scan of the zero counts the Huffman
-// decoder produced) plus the zeros before it inside the segment.
+// The outliers are placed first, as the reference's scatter does: k_outlier_scatter writes each one
+// to its element of the output, where the reverse Lorenzo kernels read it (code 0) before they
+// write the reconstruction there.  So no kernel ranks the zero codes of its rows; the placement
+// reads only the chunks of 512 codes that hold some.
 #include <cstdint>
 #include <cstdlib>
 #include <type_traits>
@@ -22,6 +23,164 @@
 namespace vsz {
 
 constexpr int kDSeg = 256;  // decompress row segment (one warp of 8-wide blocks)
+
+// ------------------------------------------------------------------------------------------
+// Outlier placement.  zero codes per chunk of kOutChunk codes are known (the Huffman decoder counts
+// them, or k_count_zeros_chunk); their exclusive scan gives each chunk's first outlier.  A warp
+// takes a chunk with zero codes 64 codes at a time: ballots rank them, and the outliers, which
+// lie at any byte offset of the archive, are read as two aligned words and a funnel shift -- so
+// reads and writes are contiguous across the warp where outliers are dense.
+// ------------------------------------------------------------------------------------------
+constexpr int kOutChunk = 512;
+
+__device__ __forceinline__ float outlier_at(const uint8_t* o, unsigned long long i, unsigned sh) {
+    // o: the section rounded down to a word; sh: the bits skipped
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(o) + i;
+    const uint32_t lo = __ldg(w);
+    return __uint_as_float(sh ? __funnelshift_r(lo, __ldg(w + 1), sh) : lo);
+}
+
+// The cnt outliers of chunk c, the first of them outlier `rank`, by one warp.  The codes and the
+// outliers (through s_val) are loaded together, all loads before the first store (the compiler
+// cannot move them across it): a load latency a chunk instead of sixteen.
+__device__ __forceinline__ void scatter_chunk(const OutlierArgs& a, size_t c, unsigned long long rank, uint32_t cnt,
+                                              float* s_val) {
+    constexpr int K     = kOutChunk / 64;
+    const unsigned lane = lane_id(), lt = lanemask_lt();
+    const unsigned sh   = (unsigned)(reinterpret_cast<uintptr_t>(a.outliers) & 3u) * 8u;
+    const uint8_t* o    = a.outliers - sh / 8u;
+    const size_t i0     = c * kOutChunk + 2u * lane;
+    const bool whole    = (c + 1) * kOutChunk <= a.n && (reinterpret_cast<uintptr_t>(a.codes) & 3u) == 0;
+    uint32_t w[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const size_t i = i0 + 64u * k;
+        if (whole) w[k] = *reinterpret_cast<const uint32_t*>(a.codes + i);
+        else w[k] = (i < a.n ? a.codes[i] : 1u) | ((i + 1 < a.n ? a.codes[i + 1] : 1u) << 16);
+    }
+    // a corrupt archive has fewer outliers than zero codes
+    cnt = (uint32_t)min((unsigned long long)cnt, rank < a.n_out ? a.n_out - rank : 0ull);
+    const uint32_t* ow = reinterpret_cast<const uint32_t*>(o) + rank;
+    const unsigned next = sh ? 1u : 0u;  // aligned outliers are one word each
+    for (uint32_t i0v = 0; i0v < cnt; i0v += 256) {
+        uint32_t lo[8], hi[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {  // no branch, so that nothing waits for one of them
+            const uint32_t i = min(i0v + 32u * q + lane, cnt - 1u);
+            lo[q] = __ldg(ow + i);
+            hi[q] = __ldg(ow + i + next);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const uint32_t i = i0v + 32u * q + lane;
+            if (i < cnt) s_val[i] = __uint_as_float(__funnelshift_r(lo[q], hi[q], sh));
+        }
+    }
+    __syncwarp();
+    const bool pairs = (reinterpret_cast<uintptr_t>(a.out) & 7u) == 0;
+    uint32_t run     = 0;  // outliers before step k
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const bool z0     = !(w[k] & 0xffffu), z1 = !(w[k] >> 16);
+        const unsigned m0 = __ballot_sync(0xffffffffu, z0), m1 = __ballot_sync(0xffffffffu, z1);
+        const uint32_t r  = run + __popc(m0 & lt) + __popc(m1 & lt), r1 = r + (z0 ? 1u : 0u);
+        float* d          = a.out + i0 + 64u * k;
+        if (z0 && z1 && r1 < cnt && pairs) {
+            *reinterpret_cast<float2*>(d) = make_float2(s_val[r], s_val[r1]);
+        } else {
+            if (z0 && r < cnt) d[0] = s_val[r];
+            if (z1 && r1 < cnt) d[1] = s_val[r1];
+        }
+        run += __popc(m0) + __popc(m1);
+    }
+    __syncwarp();  // s_val is the next chunk's
+}
+
+// One field, over the scan of its counts: CTAs of 8 warps, a warp per chunk and step.  The zero codes
+// must be as many as the outliers (or, not exact, at most as many).  A scan in the same kernel, by
+// look-back over tiles of 64 chunks, left it waiting on the look-back's chain (512^3: 0.05 ms, a scan
+// of its own and this 0.02).
+__global__ void __launch_bounds__(256) k_outlier_scatter(OutlierArgs a) {
+    __shared__ float s_val[8][kOutChunk];
+    if (__syncthreads_or(*a.status != VSZ_OK)) return;  // uniform
+    const unsigned long long all = *a.total;
+    if (a.exact ? all != a.n_out : all > a.n_out) {
+        if (threadIdx.x == 0 && blockIdx.x == 0) set_status(a.status, VSZ_ERR_CORRUPT);
+        return;
+    }
+    if (all == 0) return;
+    const unsigned warp = threadIdx.x >> 5, lane = lane_id();
+    // 32 counts at a time; a warp's chunks are a CTA apart, so that dense ones spread
+    for (size_t c0 = (size_t)blockIdx.x * 8 + warp; c0 < a.nchunks; c0 += (size_t)gridDim.x * 8 * 32) {
+        const size_t c   = c0 + (size_t)lane * gridDim.x * 8;
+        const uint32_t z = c < a.nchunks ? a.chunk_zero[c] : 0u;
+        const unsigned long long off = z ? a.chunk_off[c] : 0ull;
+        for (unsigned m = __ballot_sync(0xffffffffu, z != 0u); m; m &= m - 1u) {
+            const int q = __ffs(m) - 1;
+            scatter_chunk(a, __shfl_sync(0xffffffffu, c, q), __shfl_sync(0xffffffffu, off, q),
+                          __shfl_sync(0xffffffffu, z, q), s_val[warp]);
+        }
+    }
+}
+
+// Many fields: tasks of (field, chunk range), one CTA each, over the scan of all fields' counts.
+__global__ void __launch_bounds__(256)
+    k_outlier_scatter_batch(const OutlierArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks) {
+    __shared__ float s_val[8][kOutChunk];
+    const unsigned warp = threadIdx.x >> 5;
+    for (uint32_t t = blockIdx.x; t < ntasks; t += gridDim.x) {
+        const BatchTask tk   = tasks[t];
+        const OutlierArgs& a = args[tk.field];
+        if (*a.status != VSZ_OK) continue;  // set by earlier kernels only
+        for (size_t c = tk.u0 + warp; c < tk.u1; c += 8) {
+            const uint32_t z = a.chunk_zero[c];  // offsets are relative to the field's first chunk
+            if (z) scatter_chunk(a, c, a.chunk_off[c] - a.chunk_off[0], z, s_val[warp]);
+        }
+    }
+}
+
+// Zero codes per chunk, for codes that no decoder of this library counted.
+__global__ void __launch_bounds__(256) k_count_zeros_chunk(const uint16_t* __restrict__ codes, size_t n, size_t nchunks,
+                                                           uint32_t* __restrict__ chunk_zero) {
+    const unsigned lane = lane_id();
+    const size_t wtot   = (size_t)gridDim.x * (blockDim.x >> 5);
+    for (size_t c = blockIdx.x * (size_t)(blockDim.x >> 5) + (threadIdx.x >> 5); c < nchunks; c += wtot) {
+        uint32_t z = 0;
+#pragma unroll
+        for (int k = 0; k < kOutChunk / 32; k++) {
+            const size_t i = c * kOutChunk + 32u * k + lane;
+            z += (i < n && codes[i] == 0) ? 1u : 0u;
+        }
+        z = __reduce_add_sync(0xffffffffu, z);
+        if (lane == 0) chunk_zero[c] = z;
+    }
+}
+
+int launch_count_zeros_chunk(const uint16_t* codes, size_t n, uint32_t* chunk_zero, cudaStream_t st, int num_sms) {
+    const size_t nchunks = (n + kOutChunk - 1) / kOutChunk;
+    if (nchunks == 0) return VSZ_OK;
+    const size_t want = (nchunks + 7) / 8, cap = (size_t)num_sms * 16;
+    k_count_zeros_chunk<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(codes, n, nchunks, chunk_zero);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
+}
+
+int launch_outlier_scatter(const OutlierArgs& a, cudaStream_t st, int num_sms) {
+    if (a.nchunks == 0) return VSZ_OK;
+    const size_t want = (a.nchunks + 7) / 8, cap = (size_t)num_sms * 5;  // resident CTAs
+    k_outlier_scatter<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>(a);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
+}
+
+int launch_outlier_scatter_batch(const OutlierArgs* args, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st,
+                                 int num_sms) {
+    if (ntasks == 0) return VSZ_OK;
+    const uint32_t cap = (uint32_t)num_sms * 8;
+    k_outlier_scatter_batch<<<ntasks < cap ? ntasks : cap, 256, 0, st>>>(args, tasks, ntasks);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
+}
 
 // ------------------------------------------------------------------------------------------
 // Fast path, block size 8: one lane reconstructs one whole Lorenzo block (8 x by 8 y, plane by
@@ -44,6 +203,50 @@ __device__ __forceinline__ float strict_prequant(float v, uint32_t col, const Dq
     return prequant_vec(v, c.r_f);
 }
 
+// The outliers that k_outlier_scatter put in a row's 8 elements (zm: which of them).
+template <bool VEC>
+__device__ __forceinline__ void load_outliers(const float* p, uint32_t zm, float ov[8]) {
+    if (VEC) {  // 16-byte rows: the other elements hold nothing yet and are not looked at
+        const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+        ov[0] = a.x, ov[1] = a.y, ov[2] = a.z, ov[3] = a.w;
+        ov[4] = b.x, ov[5] = b.y, ov[6] = b.z, ov[7] = b.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++) ov[k] = (zm & (1u << k)) ? p[k] : 0.f;
+    }
+}
+
+// The same from the archive, for blocks that the separable pass has already written over: by rank,
+// the outliers before the chunk plus the zero codes from the chunk's start to the row segment's
+// (q; at most 511 codes, counted by the warp) plus those of the lanes before.  All lanes call it.
+__device__ __forceinline__ void redo_outliers(const DqDecArgs& a, size_t q, uint32_t zm, float ov[8]) {
+    if (!__any_sync(0xffffffffu, zm != 0u)) return;
+    const unsigned lane = lane_id();
+    const uint32_t cnt  = __popc(zm);
+    uint32_t incl       = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (unsigned)o) incl += t;
+    }
+    const size_t lo = (q & ~(size_t)(kOutChunk - 1)) + (size_t)lane * 16;
+    uint32_t zc     = 0;
+#pragma unroll
+    for (int t = 0; t < 16; t++)
+        if (lo + t < q) zc += (a.codes[lo + t] == 0);
+    zc = __reduce_add_sync(0xffffffffu, zc);
+    unsigned long long r = a.chunk_off[q / kOutChunk] - a.chunk_off[0] + zc + (incl - cnt);
+    const unsigned sh    = (unsigned)(reinterpret_cast<uintptr_t>(a.outliers) & 3u) * 8u;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        ov[k] = 0.f;
+        if (!(zm & (1u << k))) continue;
+        if (r < a.n_outliers) ov[k] = outlier_at(a.outliers - sh / 8u, r, sh);
+        else set_status(a.status, VSZ_ERR_CORRUPT);
+        r++;
+    }
+}
+
 typedef float DqPlane[8][8][32];  // one warp's plane of 8 x 8 blocks, [row][column][lane]
 typedef float4 DqPlaneV[8][2][32];  // the same bytes for the separable pass: [row][half][lane] x 4 columns
 
@@ -64,19 +267,12 @@ __device__ __forceinline__ void dq_b8_units(const DqDecArgs& a, uint32_t first, 
     // Narrow rows (a.ygrp > 1, rows of at most 16 blocks): the warp takes ygrp consecutive
     // y-blocks of one z-block, a group of nbx8 lanes per y-block (lanes past ygrp * nbx8 idle), so
     // that its lanes are not spent on columns past the row's end.  A lane still reconstructs one
-    // whole block; the lanes of a group share a row, and outliers are ranked per group.
+    // whole block.
     const uint32_t G   = (REDO || PAD || NDIM == 1) ? 1u : a.ygrp;
     const uint32_t gw  = G > 1 ? a.nbx8 : 32u;  // lanes per group
     const uint32_t grp = G > 1 ? lane / gw : 0u;
     const uint32_t gl0 = grp * gw;              // the group's first lane
     const uint32_t lbx = lane - gl0;            // this lane's block along x in its segment
-    const uint32_t gll = min(gl0 + gw - 1u, 31u);  // the group's last lane
-    const unsigned gmy = (gw >= 32u) ? 0xffffffffu : (((1u << gw) - 1u) << gl0);  // my group's lanes
-    // When a unit spans whole rows (one segment per row), the rows of a block in one plane are
-    // consecutive in the field, so the outlier rank at a row's start is the one at the previous
-    // row's start plus that row's zeros: the zeros from the chunk start are counted once per plane.
-    const bool carry = NDIM >= 2 && a.chunk_off != nullptr && a.nxs == 1u;
-
     // unit indices fit 32 bits (n <= 2^36 elements, 2048 per unit): 32-bit divisions only.
     for (uint32_t ui = first; ui < end; ui += stride) {
         const uint32_t u  = REDO ? a.redo[1 + ui] : ui;
@@ -136,8 +332,6 @@ __device__ __forceinline__ void dq_b8_units(const DqDecArgs& a, uint32_t first, 
             float Zm[8], Zn[8];  // 3D: row y - 1 and row y of plane z - 1
 #pragma unroll
             for (int k = 0; k < 8; k++) Cm[k] = hy;
-            unsigned long long rbase = 0;  // carry: my group's rank at the next row's start, once known
-            bool rknown = false;
 #pragma unroll 2
             for (int y = 0; y < 8; y++) {
                 const bool row_in = y < ny;
@@ -148,60 +342,17 @@ __device__ __forceinline__ void dq_b8_units(const DqDecArgs& a, uint32_t first, 
                 const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
                 auto code_at = [&](int k) -> uint32_t { return (cw[k >> 1] >> (16 * (k & 1))) & 0xffffu; };
                 auto in_at   = [&](int k) -> bool { return all_in || (row_in && x0 + (uint32_t)k < a.d0); };
-                // ---- outliers of this row segment, ranked in row-major order.  Cells outside the
-                // field read code R (never 0), so no range test is needed here or in the row pass:
-                // their values only ever feed other cells outside the field.
+                // outliers of this lane's columns.  Cells outside the field read code R (never 0), so no
+                // range test is needed here or in the row pass: their values only ever feed other
+                // cells outside the field.
                 uint32_t zm = 0;
                 if (zero_halves(cv.x) | zero_halves(cv.y) | zero_halves(cv.z) | zero_halves(cv.w)) {
 #pragma unroll
                     for (int k = 0; k < 8; k++) zm |= (code_at(k) == 0u) ? (1u << k) : 0u;
                 }
-                unsigned long long obase = 0;
-                const unsigned zlanes = __ballot_sync(0xffffffffu, zm != 0u);
-                if (zlanes) {
-                    uint32_t cnt = __popc(zm), incl = cnt;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= (unsigned)o) incl += t;
-                    }
-                    if (G > 1) {  // ranks within my group's row: less the lanes of earlier groups
-                        const uint32_t before = __shfl_sync(0xffffffffu, incl, gl0 ? gl0 - 1 : 0);
-                        if (gl0) incl -= before;
-                    }
-                    unsigned long long seg_base = rbase;
-                    if (a.chunk_off) {
-                        // zeros before this row segment: the chunk's offset plus the zeros between the
-                        // chunk start and the segment start, counted by the warp (at most 511 codes),
-                        // once for each group that has an outlier in this row and no carried rank
-                        const unsigned long long q = row * a.d0 + (unsigned long long)xs * kDSeg;
-                        const unsigned need = carry ? __ballot_sync(0xffffffffu, zm != 0u && !rknown) : zlanes;
-                        for (uint32_t g = 0; g < G; g++) {
-                            const unsigned gmask = (gw >= 32u) ? 0xffffffffu : (((1u << gw) - 1u) << (g * gw));
-                            if (!(need & gmask)) continue;  // the same for the whole warp
-                            const unsigned long long qg = __shfl_sync(0xffffffffu, q, g * gw);
-                            const unsigned long long c0 = qg & ~511ull;
-                            uint32_t zc = 0;
-                            const unsigned long long lo = c0 + (unsigned long long)lane * 16;
-#pragma unroll
-                            for (int t = 0; t < 16; t++)
-                                if (lo + t < qg) zc += (a.codes[lo + t] == 0);
-#pragma unroll
-                            for (int o = 16; o > 0; o >>= 1) zc += __shfl_xor_sync(0xffffffffu, zc, o);
-                            if (g == grp) seg_base = a.chunk_off[qg >> 9] - a.chunk_off[0] + zc;  // relative: batches
-                        }
-                        if (carry) {  // the next row starts this row's zeros later
-                            const uint32_t tot = __shfl_sync(0xffffffffu, incl, gll);
-                            if (zlanes & gmy) {
-                                rbase  = seg_base + tot;
-                                rknown = true;
-                            }
-                        }
-                    } else {
-                        seg_base = a.seg_off[row * a.nxs + xs];
-                    }
-                    obase = seg_base + (incl - cnt);
-                }
+                float ov[8];
+                if (REDO) redo_outliers(a, row * a.d0 + (size_t)xs * kDSeg, zm, ov);
+                else if (zm) load_outliers<VEC>(a.out + row * a.d0 + x0, zm, ov);
                 // ---- reverse Lorenzo along the row; an element with code 0 takes its outlier
                 float C[8];
                 auto row_pass = [&](auto with_outliers) {
@@ -234,10 +385,7 @@ __device__ __forceinline__ void dq_b8_units(const DqDecArgs& a, uint32_t first, 
                         float s = __fadd_rn(pred, __fsub_rn(__uint_as_float(0x4B000000u | cd), rbias));
                         if (decltype(with_outliers)::value) {
                             if (zm & (1u << k)) {
-                                const unsigned long long oi = obase + __popc(zm & ((1u << k) - 1u));
-                                s = 0.f;
-                                if (oi < a.n_outliers) s = a.outliers[oi];
-                                else set_status(a.status, VSZ_ERR_CORRUPT);
+                                s = ov[k];
                                 if (a.strict) s = strict_prequant<NDIM>(s, x0 + (uint32_t)k, a, c);
                             }
                         }
@@ -255,11 +403,7 @@ __device__ __forceinline__ void dq_b8_units(const DqDecArgs& a, uint32_t first, 
                     if (a.strict && zm) {  // strict outliers are output as stored
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
-                            const int kk = 4 * h + k;
-                            if (zm & (1u << kk)) {
-                                const unsigned long long oi = obase + __popc(zm & ((1u << kk) - 1u));
-                                xo[k] = oi < a.n_outliers ? a.outliers[oi] : 0.f;
-                            }
+                            if (zm & (1u << (4 * h + k))) xo[k] = ov[4 * h + k];
                         }
                     }
                     if (VEC && all_in) {
@@ -309,8 +453,6 @@ __global__ void __launch_bounds__(128, 6) k_dq_decompress_b8(DqDecArgs a) {
 // a.redo, and the reference-order kernel redoes it afterwards.
 // ------------------------------------------------------------------------------------------
 // Units u = first, first + stride, ... < end of one field; s_A: A of the previous plane.
-// CARRY: rows of one segment carry their outlier rank (checked at run time).
-template <bool CARRY>
 __device__ __forceinline__ void dq_b8s_units(const DqDecArgs& a, uint32_t first, uint32_t end, uint32_t stride,
                                              DqPlane* s_A, unsigned wib) {
     const Consts c = *a.consts;
@@ -321,9 +463,6 @@ __device__ __forceinline__ void dq_b8s_units(const DqDecArgs& a, uint32_t first,
     const unsigned lane        = lane_id();
     // rows start on 32-byte boundaries (d0 % 8 == 0) when the output does
     const bool out32           = (reinterpret_cast<uintptr_t>(a.out) & 31u) == 0;
-    // one segment per row: a row's outlier rank is the previous row's plus its zeros (as
-    // k_dq_decompress_b8)
-    const bool carry           = CARRY && a.chunk_off != nullptr && a.nxs == 1u;
 
     for (uint32_t u = first; u < end; u += stride) {
         const uint32_t xs = u % a.nxs;
@@ -352,8 +491,6 @@ __device__ __forceinline__ void dq_b8s_units(const DqDecArgs& a, uint32_t first,
             float Bm[8];  // B of the row above (zero above the block)
 #pragma unroll
             for (int k = 0; k < 8; k++) Bm[k] = 0.f;
-            unsigned long long rbase = 0;  // carry: the rank at the next row's start, once known
-            bool rknown = false;
 #pragma unroll 2
             for (int y = 0; y < 8; y++) {
                 const bool row_in = y < ny;
@@ -370,42 +507,10 @@ __device__ __forceinline__ void dq_b8s_units(const DqDecArgs& a, uint32_t first,
                 }
                 const uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
                 auto code_at = [&](int k) -> uint32_t { return (cw[k >> 1] >> (16 * (k & 1))) & 0xffffu; };
-                // outliers of this row segment, ranked in row-major order (as k_dq_decompress_b8)
-                uint32_t zm = 0;
+                uint32_t zm = 0;  // outliers of this lane's columns
                 if (zero_halves(cv.x) | zero_halves(cv.y) | zero_halves(cv.z) | zero_halves(cv.w)) {
 #pragma unroll
                     for (int k = 0; k < 8; k++) zm |= (code_at(k) == 0u) ? (1u << k) : 0u;
-                }
-                unsigned long long obase = 0;
-                if (__any_sync(0xffffffffu, zm != 0u)) {
-                    uint32_t cnt = __popc(zm), incl = cnt;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                        if (lane >= (unsigned)o) incl += t;
-                    }
-                    unsigned long long seg_base = rbase;
-                    if (a.chunk_off) {
-                        if (!rknown) {  // the same for the whole warp
-                            const unsigned long long q  = row * a.d0 + (unsigned long long)xs * kDSeg;
-                            const unsigned long long c0 = q & ~511ull;
-                            uint32_t zc = 0;
-                            const unsigned long long lo = c0 + (unsigned long long)lane * 16;
-#pragma unroll
-                            for (int t = 0; t < 16; t++)
-                                if (lo + t < q) zc += (a.codes[lo + t] == 0);
-#pragma unroll
-                            for (int o = 16; o > 0; o >>= 1) zc += __shfl_xor_sync(0xffffffffu, zc, o);
-                            seg_base = a.chunk_off[q >> 9] - a.chunk_off[0] + zc;  // relative: batches
-                        }
-                        if (carry) {
-                            rbase  = seg_base + __shfl_sync(0xffffffffu, incl, 31);
-                            rknown = true;
-                        }
-                    } else {
-                        seg_base = a.seg_off[row * a.nxs + xs];
-                    }
-                    obase = seg_base + (incl - cnt);
                 }
                 float C[8], Ar[8];  // Ar: A of the row in the previous plane, then of this one
                 {
@@ -414,6 +519,8 @@ __device__ __forceinline__ void dq_b8s_units(const DqDecArgs& a, uint32_t first,
                     Ar[4] = a1.x, Ar[5] = a1.y, Ar[6] = a1.z, Ar[7] = a1.w;
                 }
                 auto row_pass = [&](auto with_outliers) {
+                    float ov[8];
+                    if (decltype(with_outliers)::value) load_outliers<true>(a.out + row * a.d0 + x0, zm, ov);
                     float sl = 0.f;  // s of the element to the left (zero left of the block)
 #pragma unroll
                     for (int k = 0; k < 8; k++) {
@@ -423,10 +530,7 @@ __device__ __forceinline__ void dq_b8s_units(const DqDecArgs& a, uint32_t first,
                         float sv      = __fadd_rn(sl, B);
                         if (decltype(with_outliers)::value) {
                             if (zm & (1u << k)) {
-                                const unsigned long long oi = obase + __popc(zm & ((1u << k) - 1u));
-                                sv = 0.f;
-                                if (oi < a.n_outliers) sv = a.outliers[oi];
-                                else set_status(a.status, VSZ_ERR_CORRUPT);
+                                sv = ov[k];
                                 B = __fsub_rn(sv, sl);
                                 A = __fsub_rn(B, Bm[k]);
                             }
@@ -539,11 +643,10 @@ __global__ void __launch_bounds__(256) k_dq_mul_verify(Consts* __restrict__ c, u
     }
 }
 
-template <bool CARRY>
 __global__ void __launch_bounds__(128, 6) k_dq_decompress_b8s(DqDecArgs a) {
     extern __shared__ __align__(16) uint8_t s_dq_dyn[];
     const unsigned wib = threadIdx.x >> 5;
-    dq_b8s_units<CARRY>(a, blockIdx.x * (blockDim.x >> 5) + wib, (uint32_t)a.nunits, gridDim.x * (blockDim.x >> 5),
+    dq_b8s_units(a, blockIdx.x * (blockDim.x >> 5) + wib, (uint32_t)a.nunits, gridDim.x * (blockDim.x >> 5),
                  reinterpret_cast<DqPlane*>(s_dq_dyn), wib);
 }
 
@@ -555,8 +658,7 @@ __global__ void __launch_bounds__(128, 6) k_dq_decompress_b8s(DqDecArgs a) {
 // step t it reconstructs row (y, z = t - y) from its own row of plane z - 1 (in registers) and
 // lane y - 1's rows of planes z and z - 1 (shuffled one lane up after each step).  15 steps of 8
 // elements per lane instead of 512; the predictor is the reference's, in its FP32 order, so the
-// values are the same bits.  A warp holds 4 blocks along x.  Outliers are ranked from blk_off
-// (zero codes before each row's x-block), so no lane waits on another for a rank.
+// values are the same bits.  A warp holds 4 blocks along x.
 // ------------------------------------------------------------------------------------------
 template <bool VEC>
 __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
@@ -568,7 +670,6 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
     const unsigned lane   = lane_id();
     const int y           = (int)(lane & 7u);  // row of the block
     const uint32_t nxq    = (a.nbx8 + 3) / 4;  // groups of 4 blocks along x
-    const bool ranks      = a.n_outliers != 0;
     const unsigned long long wtot = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     for (unsigned long long u = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
          u < a.nunits; u += wtot) {
@@ -592,14 +693,10 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
             for (int k = 0; k < 8; k++) t[k] = (x0 + k < a.d0) ? (uint32_t)crow[x0 + k] : (uint32_t)R;
             return make_uint4(t[0] | (t[1] << 16), t[2] | (t[3] << 16), t[4] | (t[5] << 16), t[6] | (t[7] << 16));
         };
-        auto load_off = [&](int zz) -> unsigned long long {
-            return (ranks && row_in && zz < nz) ? a.blk_off[row_of(zz) * a.nbx8 + bx] : 0ull;
-        };
         float Zp[8], Y[8], Yp[8];  // own row of plane z - 1; rows y - 1 of planes z and z - 1
 #pragma unroll
         for (int k = 0; k < 8; k++) Zp[k] = Y[k] = Yp[k] = 0.f;
-        uint4 cv               = load_row(0);
-        unsigned long long off = load_off(0);
+        uint4 cv = load_row(0);
         for (int t = 0; t < nz + 7; t++) {
             float up[8];  // lane y - 1's newest row (row y - 1 of the plane this lane takes now)
 #pragma unroll
@@ -607,9 +704,7 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
             const int zz = t - y;
             if (zz >= 0 && zz < nz) {
                 const uint4 cw4 = cv;
-                const unsigned long long obase = off;
-                cv  = load_row(zz + 1);
-                off = load_off(zz + 1);
+                cv = load_row(zz + 1);
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
                     Yp[k] = Y[k];
@@ -622,7 +717,8 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
 #pragma unroll
                     for (int k = 0; k < 8; k++) zm |= (code_at(k) == 0u) ? (1u << k) : 0u;
                 }
-                float C[8];
+                float C[8], ov[8];
+                if (zm) load_outliers<VEC>(a.out + row_of(zz) * a.d0 + x0, zm, ov);
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
                     const float X   = k ? C[k - 1] : 0.f;
@@ -633,10 +729,7 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
                         __fadd_rn(__fadd_rn(__fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(XYZ, XY), XZ), Yp[k]), X), Y[k]), Zp[k]);
                     float s = __fadd_rn(pred, __fsub_rn(__uint_as_float(0x4B000000u | code_at(k)), rbias));
                     if (zm & (1u << k)) {
-                        const unsigned long long oi = obase + __popc(zm & ((1u << k) - 1u));
-                        s = 0.f;
-                        if (oi < a.n_outliers) s = a.outliers[oi];
-                        else set_status(a.status, VSZ_ERR_CORRUPT);
+                        s = ov[k];
                         if (a.strict) s = strict_prequant<3>(s, x0 + (uint32_t)k, a, c);
                     }
                     C[k] = s;
@@ -645,10 +738,7 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
 #pragma unroll
                 for (int k = 0; k < 8; k++) {
                     xo[k] = dequant(C[k], c.c_d, c.c_hi, c.c_lo, c.dq_fast);
-                    if (a.strict && (zm & (1u << k))) {  // strict outliers are output as stored
-                        const unsigned long long oi = obase + __popc(zm & ((1u << k) - 1u));
-                        xo[k] = oi < a.n_outliers ? a.outliers[oi] : 0.f;
-                    }
+                    if (a.strict && (zm & (1u << k))) xo[k] = ov[k];  // strict outliers are output as stored
                 }
                 float* orow = a.out + row_of(zz) * a.d0;
                 if (VEC && all_in) {
@@ -666,33 +756,8 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
     }
 }
 
-// Zero codes per (row, x-block of 8) in row-major order, for k_dq_decompress_w8's ranks.
-__global__ void __launch_bounds__(256) k_count_zeros_b8(const uint16_t* __restrict__ codes, uint32_t d0, uint32_t nbx8,
-                                                        size_t m, uint32_t* __restrict__ blk_zero) {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < m; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t row     = i / nbx8;
-        const uint32_t x0    = (uint32_t)(i - row * nbx8) * 8u;
-        const uint16_t* crow = codes + row * d0;
-        uint32_t z = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < 8; k++) z += (x0 + k < d0 && crow[x0 + k] == 0) ? 1u : 0u;
-        blk_zero[i] = z;
-    }
-}
-
-int launch_count_zeros_b8(const uint16_t* codes, uint32_t d0, size_t nrows, uint32_t* blk_zero, cudaStream_t st,
-                          int num_sms) {
-    const uint32_t nbx8 = (d0 + 7) / 8;
-    const size_t m      = nrows * nbx8;
-    if (m == 0) return VSZ_OK;
-    long long want = (long long)((m + 255) / 256), cap = (long long)num_sms * 8;
-    k_count_zeros_b8<<<(int)(want < cap ? want : cap), 256, 0, st>>>(codes, d0, nbx8, m, blk_zero);
-    count_launch();
-    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
-}
-
 bool dq_w8_applies(const DqDecArgs& a, int ndim) {
-    if (ndim != 3 || a.pad.vals || a.n > kW8MaxN || !(a.blk_off || a.n_outliers == 0)) return false;
+    if (ndim != 3 || a.pad.vals || a.n > kW8MaxN) return false;
     if (getenv("VSZ_DQ_NO_WAVEFRONT") != nullptr) return false;
     // the separable pass catches up with the wavefront between 160^3 and 256^3 (measured: 0.123
     // vs 0.060 ms at 160^3, 0.099 vs 0.127 ms at 256^3, zero scans included)
@@ -706,12 +771,6 @@ bool dq_w8_applies(const DqDecArgs& a, int ndim) {
 // two shared-memory buffers.  A CTA runs G = 128 / bs blocks side by side.
 // 1D: one thread per block, sequential along x.
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t zeros_before(const uint16_t* crow, uint32_t from, uint32_t to) {
-    uint32_t n = 0;
-    for (uint32_t x = from; x < to; x++) n += (crow[x] == 0);
-    return n;
-}
-
 template <int NDIM, int BS, bool PAD = false>
 __global__ void __launch_bounds__(128) k_dq_decompress_gen(DqDecArgs a) {
     constexpr int G = (128 / BS) > 0 ? (128 / BS) : 1;
@@ -723,8 +782,6 @@ __global__ void __launch_bounds__(128) k_dq_decompress_gen(DqDecArgs a) {
         size_t b = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
         size_t x0 = b * BS;
         if (x0 >= a.d0) return;
-        uint32_t seg_x0 = (uint32_t)(x0 & ~(size_t)(kDSeg - 1));
-        uint32_t zb = zeros_before(a.codes, seg_x0, (uint32_t)x0);
         const float hx = PAD ? halo_of(a.pad, 1, (uint32_t)(x0 / BS), 0, 0).x : 0.f;
         float prev = 0.f;
         for (int k = 0; k < BS; k++) {
@@ -733,19 +790,11 @@ __global__ void __launch_bounds__(128) k_dq_decompress_gen(DqDecArgs a) {
             uint32_t cd = a.codes[x];
             float s, xo;
             if (cd == 0u) {
-                if ((x & (kDSeg - 1)) == 0) zb = 0;
-                unsigned long long oi = a.seg_off[x / kDSeg] + zb;
-                if (oi < a.n_outliers) s = a.outliers[oi];
-                else {
-                    s = 0.f;
-                    set_status(a.status, VSZ_ERR_CORRUPT);
-                }
-                zb++;
+                s  = a.out[x];
                 xo = s;  // strict: the stored input value
                 if (a.strict) s = strict_prequant<1>(s, (uint32_t)x, a, c);
                 else xo = dequant(s, c.c_d, c.c_hi, c.c_lo, c.dq_fast);
             } else {
-                if ((x & (kDSeg - 1)) == 0) zb = 0;
                 s  = __fadd_rn(k ? prev : hx, (float)((int)cd - R));
                 xo = dequant(s, c.c_d, c.c_hi, c.c_lo, c.dq_fast);
             }
@@ -774,7 +823,6 @@ __global__ void __launch_bounds__(128) k_dq_decompress_gen(DqDecArgs a) {
     for (int i = t; i < 2 * BS * BS; i += BS) S0[i] = 0.f;
     __syncthreads();
     const int nsteps = (NDIM == 3) ? (BS * BS + BS - 1) : (2 * BS - 1);
-    uint32_t zrun = 0;  // zeros seen in the current row segment before the current x
     for (int step = 0; step < nsteps; step++) {
         const int q = step - t;
         const int lim = (NDIM == 3) ? BS * BS : BS;
@@ -788,8 +836,6 @@ __global__ void __launch_bounds__(128) k_dq_decompress_gen(DqDecArgs a) {
             if (in) {
                 const size_t row     = (size_t)z * a.d1 + y;
                 const uint16_t* crow = a.codes + row * a.d0;
-                if (xl == 0) zrun = zeros_before(crow, x0 & ~(uint32_t)(kDSeg - 1), x0);
-                else if ((x & (kDSeg - 1)) == 0) zrun = 0;
                 uint32_t cd = crow[x];
                 float pred;
                 // halo cells: 2D (x-1, y-1) is the x-halo's, 3D the y-halo's; z - 1 = halo: hz
@@ -809,10 +855,7 @@ __global__ void __launch_bounds__(128) k_dq_decompress_gen(DqDecArgs a) {
                 }
                 float xo;
                 if (cd == 0u) {
-                    unsigned long long oi = a.seg_off[row * a.nxs + (x / kDSeg)] + zrun;
-                    if (oi < a.n_outliers) s = a.outliers[oi];
-                    else set_status(a.status, VSZ_ERR_CORRUPT);
-                    zrun++;
+                    s  = a.out[row * a.d0 + x];
                     xo = s;  // strict: the stored input value
                     if (a.strict) s = strict_prequant<NDIM>(s, x, a, c);
                     else xo = dequant(s, c.c_d, c.c_hi, c.c_lo, c.dq_fast);
@@ -932,7 +975,7 @@ __global__ void __launch_bounds__(128, 6)
     const unsigned wib = threadIdx.x >> 5;
     for (uint32_t t = dq_next_task(next); t < ntasks; t = dq_next_task(next)) {
         const BatchTask tk = tasks[t];
-        dq_b8s_units<true>(args[tk.field], (uint32_t)tk.u0, (uint32_t)tk.u1, 1u, reinterpret_cast<DqPlane*>(s_dq_dyn), wib);
+        dq_b8s_units(args[tk.field], (uint32_t)tk.u0, (uint32_t)tk.u1, 1u, reinterpret_cast<DqPlane*>(s_dq_dyn), wib);
     }
 }
 
@@ -1024,8 +1067,7 @@ int launch_dq_decompress(DqDecArgs a, int ndim, int bs, bool force_general, cuda
                 k_dq_mul_verify<<<(unsigned)num_sms * 4, 256, 0, st>>>(a.consts_rw, a.redo, a.dq_cache);
                 count_launch();
             }
-            // fields of one segment per row carry outlier ranks; wider ones keep the lighter kernel
-            a.nxs == 1 ? go(k_dq_decompress_b8s<true>, 3) : go(k_dq_decompress_b8s<false>, 3);
+            go(k_dq_decompress_b8s, 3);
             go(k_dq_decompress_b8<3, true, false, true>, 3);
         } else {
             if (ndim == 3) vec ? go(k_dq_decompress_b8<3, true>, 3) : go(k_dq_decompress_b8<3, false>, 3);

@@ -1013,14 +1013,6 @@ __global__ void __launch_bounds__(256) k_huff_decode(HuffDecodeArgs a) {
     const uint32_t* gw   = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(a.payload) & ~(uintptr_t)3);
     BitReader br;
     br.init(gw, base0 + a.start_bit[j], base0 + a.payload_bits);
-    // output position -> (row, x) for the per-segment zero counts
-    unsigned long long row = out0 / a.d0;
-    uint32_t x             = (uint32_t)(out0 - row * a.d0);
-    uint32_t zeros         = 0;
-    auto flush = [&]() {
-        if (zeros && a.seg_zero) atomicAdd(&a.seg_zero[row * a.nxs + (x >> 8)], zeros);
-        zeros = 0;
-    };
     uint16_t* out = a.codes + out0;
     for (unsigned long long k = 0; k < cnt; k++) {
         uint32_t s = decode_one(br, s_table, a.table2, a.child, a.node_sym, a.max_nodes);
@@ -1029,20 +1021,7 @@ __global__ void __launch_bounds__(256) k_huff_decode(HuffDecodeArgs a) {
             return;
         }
         out[k] = (uint16_t)s;
-        zeros += (s == 0);
-        x++;
-        if (x == a.d0) {
-            x--;
-            flush();
-            x = 0;
-            row++;
-        } else if ((x & 255u) == 0) {
-            x--;
-            flush();
-            x++;
-        }
     }
-    flush();
 }
 
 // Indexed decode with coalesced output: a warp decodes 32 consecutive chunks of 512 codewords
@@ -1788,17 +1767,11 @@ int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks,
 }
 
 // Constant fill for a one-symbol tree (src/huffman.hh:348-352).
-__global__ void k_huff_const(uint16_t* codes, size_t n, const uint32_t* info, uint32_t* seg_zero, uint32_t d0, uint32_t nxs,
-                             const int* status) {
+__global__ void k_huff_const(uint16_t* codes, size_t n, const uint32_t* info, const int* status) {
     if (*status != VSZ_OK) return;
     const uint16_t c = (uint16_t)info[1];
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         codes[i] = c;
-        if (c == 0 && seg_zero) {
-            size_t row = i / d0;
-            uint32_t x = (uint32_t)(i - row * d0);
-            atomicAdd(&seg_zero[row * nxs + (x >> 8)], 1u);
-        }
     }
 }
 
@@ -2072,11 +2045,10 @@ int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms) {
     return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }
 
-int launch_huff_const(uint16_t* codes, size_t n, const uint32_t* info, uint32_t* seg_zero, uint32_t d0, uint32_t nxs,
-                      const int* status, cudaStream_t st, int num_sms) {
+int launch_huff_const(uint16_t* codes, size_t n, const uint32_t* info, const int* status, cudaStream_t st, int num_sms) {
     int grid = (int)min((long long)((n + 255) / 256), (long long)num_sms * 8);
     if (grid < 1) grid = 1;
-    k_huff_const<<<grid, 256, 0, st>>>(codes, n, info, seg_zero, d0, nxs, status);
+    k_huff_const<<<grid, 256, 0, st>>>(codes, n, info, status);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }

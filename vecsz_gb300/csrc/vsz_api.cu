@@ -1,5 +1,6 @@
 // C ABI of the library (include/vecsz_gb300.h): argument checks, workspace layout and the
 // stream-ordered compress / decompress pipelines built from the kernels in dq_*.cu and huffman.cu.
+#include <algorithm>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -141,9 +142,9 @@ struct DecompressWs {
     uint32_t* tinfo;
     uint32_t* win;
     uint16_t* code;
-    uint32_t* seg_zero;
+    uint32_t* seg_zero;  // f64 fields: zero codes per 256-wide row segment, and their scan
     unsigned long long* seg_off;
-    uint32_t* chunk_zero;
+    uint32_t* chunk_zero;  // zero codes per 512 codes, and their scan
     unsigned long long* chunk_off;
     unsigned long long* scan_status;
     uint32_t* scan_counter;
@@ -155,15 +156,12 @@ struct DecompressWs {
     uint32_t* s_count;
     unsigned long long* s_out_begin;
     int* s_changed;
-    float* outliers;
-    uint32_t* blk_zero;             // zero codes per (row, x-block of 8): small 3D fields only
-    unsigned long long* blk_off;    // their exclusive scan (outlier rank of each row's block)
     uint32_t* redo;  // units of the separable reverse Lorenzo that the reference-order kernel redoes
     unsigned long long* dq_cache;  // the last dequantization check (k_dq_mul_verify), at a fixed offset
     size_t bytes;
 };
 
-DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes, size_t n_out, size_t n_index_chunks,
+DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes, size_t n_index_chunks, bool f64,
                                uint8_t* base, size_t cap) {
     Bump b{base, cap};
     DecompressWs w{};
@@ -182,18 +180,13 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
     w.win      = b.take<uint32_t>(n_index_chunks && n_index_chunks <= kSplitMaxChunks ? kWinImageWords : 4);
     w.code     = b.take<uint16_t>(g.n + 8);
     uint32_t nxs = (g.d0 + 255) / 256;
-    size_t nsegd = g.nrows * nxs;
+    const size_t nsegd = f64 ? g.nrows * nxs : 0, nch = (g.n + kChunkSyms - 1) / kChunkSyms;
     w.seg_zero = b.take<uint32_t>(nsegd + 1);
     w.seg_off  = b.take<unsigned long long>(nsegd + 1);
-    w.chunk_zero = b.take<uint32_t>(n_index_chunks + 1);
-    w.chunk_off  = b.take<unsigned long long>(n_index_chunks + 1);
-    const size_t nblk = (g.ndim == 3 && g.n <= kW8MaxN) ? g.nrows * ((g.d0 + 7) / 8) : 0;
-    w.blk_zero = b.take<uint32_t>(nblk + 1);
-    w.blk_off  = b.take<unsigned long long>(nblk + 1);
+    w.chunk_zero = b.take<uint32_t>(nch + 1);
+    w.chunk_off  = b.take<unsigned long long>(nch + 1);
     size_t nsync = (payload_bytes * 8 + kSyncBits - 1) / kSyncBits + 1;
-    size_t scan_n = nsegd > nblk ? nsegd : nblk;
-    if (n_index_chunks > scan_n) scan_n = n_index_chunks;
-    if (nsync > scan_n) scan_n = nsync;
+    const size_t scan_n = std::max(std::max(nsegd, nch), nsync);
     w.scan_status  = b.take<unsigned long long>(scan_tmp_tiles(scan_n) + 1);
     w.scan_counter = b.take<uint32_t>(4);
     w.scan_total   = b.take<unsigned long long>(1);
@@ -204,7 +197,6 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
     w.s_count      = b.take<uint32_t>(nsync);
     w.s_out_begin  = b.take<unsigned long long>(nsync);
     w.s_changed    = b.take<int>(4);
-    w.outliers     = b.take<float>(n_out + 4);
     {
         const size_t units8 = (size_t)nxs * ((g.d1 + 7) / 8) * ((g.d2 + 7) / 8);  // block-8 warp units
         w.redo = b.take<uint32_t>(units8 + 2);
@@ -216,11 +208,10 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
 // Decode n codes from a Huffman section at d_huff.  Index path when chunk_bits != null.
 int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, size_t tree_bytes, size_t n, int dict,
                  const uint16_t* chunk_bits, size_t n_index_chunks, uint32_t chunk_syms, const DecompressWs& w,
-                 uint32_t* seg_zero, uint32_t d0, cudaStream_t st) {
+                 cudaStream_t st) {
     const uint8_t* payload   = d_huff + 8 + tree_bytes;
     size_t payload_bytes     = huff_bytes - 8 - tree_bytes;
     unsigned long long pbits = (unsigned long long)payload_bytes * 8ull;
-    uint32_t nxs             = (d0 + 255) / 256;
     HuffTableArgs ta{};
     ta.huff = d_huff;
     ta.huff_bytes = huff_bytes;
@@ -243,7 +234,7 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     }
     if (node_count == 1) {
         // one-symbol tree: constant output (src/huffman.hh:348-352)
-        return launch_huff_const(w.code, n, w.tinfo, seg_zero, d0, nxs, w.status, st, num_sms());
+        return launch_huff_const(w.code, n, w.tinfo, w.status, st, num_sms());
     }
     HuffDecodeArgs da{};
     da.payload = payload;
@@ -254,9 +245,6 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     da.node_sym = w.node_sym;
     da.codes = w.code;
     da.n = n;
-    da.seg_zero = seg_zero;
-    da.d0 = d0;
-    da.nxs = nxs;
     da.max_nodes = (uint32_t)(2 * dict - 1);
     da.win = ta.win;
     da.walk = w.walk;
@@ -852,7 +840,7 @@ vsz_status vsz_huffman_encode(const uint16_t* d_code, size_t n, const void* d_co
 size_t vsz_huffman_decode_tmp_bytes(size_t huff_bytes, size_t n, int dict_size) {
     size_t dims[3] = {n, 1, 1};
     Geometry g = make_geometry(1, dims);
-    return layout_decompress(g, dict_size, huff_bytes, 0, 0, nullptr, 0).bytes;
+    return layout_decompress(g, dict_size, huff_bytes, 0, false, nullptr, 0).bytes;
 }
 
 vsz_status vsz_huffman_decode(const uint8_t* d_huff, size_t huff_bytes, size_t n, int dict_size, uint16_t* d_code,
@@ -863,7 +851,7 @@ vsz_status vsz_huffman_decode(const uint8_t* d_huff, size_t huff_bytes, size_t n
     if (tmp_bytes < need) return VSZ_ERR_CAPACITY;
     size_t dims[3] = {n, 1, 1};
     Geometry g = make_geometry(1, dims);
-    DecompressWs w = layout_decompress(g, dict_size, huff_bytes, 0, 0, reinterpret_cast<uint8_t*>(d_tmp), tmp_bytes);
+    DecompressWs w = layout_decompress(g, dict_size, huff_bytes, 0, false, reinterpret_cast<uint8_t*>(d_tmp), tmp_bytes);
     // node count / tree size from the big-endian header on the device: copy 4 bytes
     uint8_t h4[4];
     VSZ_CUDA(cudaMemcpyAsync(h4, d_huff, 4, cudaMemcpyDeviceToHost, S(stream)));
@@ -872,8 +860,7 @@ vsz_status vsz_huffman_decode(const uint8_t* d_huff, size_t huff_bytes, size_t n
     if (nc == 0 || nc > (uint32_t)(2 * dict_size - 1) || 8 + tree_bytes_size(nc) > huff_bytes) return VSZ_ERR_CORRUPT;
     VSZ_CUDA(cudaMemsetAsync(w.status, 0, sizeof(int), S(stream)));
     // decode into w.code, then copy to the caller (w.code is sized for n)
-    int rc = decode_codes(d_huff, huff_bytes, nc, tree_bytes_size(nc), n, dict_size, nullptr, 0, 0, w, nullptr,
-                          (uint32_t)n, S(stream));
+    int rc = decode_codes(d_huff, huff_bytes, nc, tree_bytes_size(nc), n, dict_size, nullptr, 0, 0, w, S(stream));
     if (rc) return rc;
     VSZ_CUDA(cudaMemcpyAsync(d_code, w.code, n * sizeof(uint16_t), cudaMemcpyDeviceToDevice, S(stream)));
     int st = 0;
@@ -884,10 +871,9 @@ vsz_status vsz_huffman_decode(const uint8_t* d_huff, size_t huff_bytes, size_t n
 
 size_t vsz_dualquant_decompress_tmp_bytes(int ndim, const size_t dims[3]) {
     if (!valid_dims(ndim, dims)) return 0;
-    Geometry g = make_geometry(ndim, dims);
-    uint32_t nxs = (g.d0 + 255) / 256;
-    size_t nsegd = g.nrows * nxs;
-    return 1024 + 4 * (nsegd + 64) + 8 * (nsegd + 64) + 8 * (scan_tmp_tiles(nsegd) + 2) + 1024;
+    Geometry g       = make_geometry(ndim, dims);
+    const size_t nch = (g.n + kChunkSyms - 1) / kChunkSyms;
+    return 2048 + 12 * (nch + 32) + 8 * (scan_tmp_tiles(nch) + 1);
 }
 
 vsz_status vsz_dualquant_decompress(int ndim, const size_t dims[3], int block_size, int dict_size,
@@ -898,23 +884,33 @@ vsz_status vsz_dualquant_decompress(int ndim, const size_t dims[3], int block_si
     if (!valid_bs(block_size)) return VSZ_ERR_UNSUPPORTED;
     if (tmp_bytes < vsz_dualquant_decompress_tmp_bytes(ndim, dims)) return VSZ_ERR_CAPACITY;
     Geometry g = make_geometry(ndim, dims);
-    uint32_t nxs = (g.d0 + 255) / 256;
-    size_t nsegd = g.nrows * nxs;
+    const size_t nch = (g.n + kChunkSyms - 1) / kChunkSyms;
     Bump b{reinterpret_cast<uint8_t*>(d_tmp), tmp_bytes};
-    int* status = b.take<int>(4);
-    uint32_t* counter = b.take<uint32_t>(4);
-    uint32_t* seg_zero = b.take<uint32_t>(nsegd + 1);
-    unsigned long long* seg_off = b.take<unsigned long long>(nsegd + 1);
-    unsigned long long* tstat = b.take<unsigned long long>(scan_tmp_tiles(nsegd) + 1);
+    OutlierArgs o{};
+    o.codes       = d_code;
+    o.n           = g.n;
+    o.nchunks     = nch;
+    o.outliers    = reinterpret_cast<const uint8_t*>(d_outliers);
+    o.n_out       = n_outlier;
+    o.out         = d_out;
+    int* status   = b.take<int>(4);
+    o.status      = status;
+    uint32_t* counter    = b.take<uint32_t>(4);
+    unsigned long long* total      = b.take<unsigned long long>(1);
+    unsigned long long* tiles      = b.take<unsigned long long>(scan_tmp_tiles(nch) + 1);
+    uint32_t* chunk_zero           = b.take<uint32_t>(nch);
+    unsigned long long* chunk_off  = b.take<unsigned long long>(nch);
+    o.chunk_zero  = chunk_zero;
+    o.chunk_off   = chunk_off;
+    o.total       = total;
     VSZ_CUDA(cudaMemsetAsync(status, 0, sizeof(int), S(stream)));
-    VSZ_TRY(launch_count_zeros(d_code, g.d0, g.nrows, seg_zero, S(stream), num_sms()));
-    VSZ_TRY(launch_scan_u32(seg_zero, seg_off, nsegd, tstat, counter, nullptr, status, S(stream)));
+    VSZ_TRY(launch_count_zeros_chunk(d_code, g.n, chunk_zero, S(stream), num_sms()));
+    VSZ_TRY(launch_scan_u32(chunk_zero, chunk_off, nch, tiles, counter, total, status, S(stream)));
+    VSZ_TRY(launch_outlier_scatter(o, S(stream), num_sms()));
     DqDecArgs a{};
     a.codes      = d_code;
-    a.outliers   = d_outliers;
     a.n_outliers = n_outlier;
     a.status     = status;
-    a.seg_off    = seg_off;
     a.consts     = reinterpret_cast<const Consts*>(d_consts);
     a.out        = d_out;
     a.d0 = g.d0;
@@ -1234,6 +1230,11 @@ static PadView pad_view_of(const vsz_archive_desc* d, int bs, const uint8_t* d_a
     return v;
 }
 
+// Whether the decoder of this archive counts the zero codes of each chunk: the indexed ones do.
+static bool indexed_counts(const vsz_archive_desc* d) {
+    return d->has_trailer && d->node_count > 1;
+}
+
 vsz_status vsz_decompress_bounds(const vsz_archive_desc* d, const vsz_decompress_opts* o, size_t* ws_bytes) {
     if (!d) return VSZ_ERR_INVALID;
     int dict, bs;
@@ -1242,8 +1243,8 @@ vsz_status vsz_decompress_bounds(const vsz_archive_desc* d, const vsz_decompress
     size_t dims[3] = {d->dims[0], d->dims[1], d->dims[2]};
     Geometry g = make_geometry(d->ndim, dims);
     if (ws_bytes)
-        *ws_bytes = layout_decompress(g, decode_symbols(d, dict), d->payload_bytes, d->n_outlier,
-                                      d->has_trailer ? d->n_chunks : 0, nullptr, 0).bytes;
+        *ws_bytes = layout_decompress(g, decode_symbols(d, dict), d->payload_bytes, d->has_trailer ? d->n_chunks : 0,
+                                      false, nullptr, 0).bytes;
     return VSZ_OK;
 }
 
@@ -1258,36 +1259,48 @@ vsz_status vsz_decompress(const vsz_archive_desc* d, const vsz_decompress_opts* 
     Geometry g = make_geometry(d->ndim, dims);
     const int nsym = decode_symbols(d, dict);
     if (d->node_count > (uint32_t)(2 * nsym - 1)) return VSZ_ERR_CORRUPT;
-    DecompressWs w = layout_decompress(g, nsym, d->payload_bytes, d->n_outlier, d->has_trailer ? d->n_chunks : 0,
+    DecompressWs w = layout_decompress(g, nsym, d->payload_bytes, d->has_trailer ? d->n_chunks : 0, false,
                                        reinterpret_cast<uint8_t*>(d_ws), ws_bytes);
     if (w.bytes > ws_bytes) return VSZ_ERR_CAPACITY;
     cudaStream_t st = S(stream);
-    uint32_t nxs = (g.d0 + 255) / 256;
-    size_t nsegd = g.nrows * nxs;
     VSZ_CUDA(cudaMemsetAsync(w.status, 0, sizeof(int), st));
-    VSZ_CUDA(cudaMemsetAsync(w.seg_zero, 0, 4 * nsegd, st));
     VSZ_TRY(launch_eb_setup(VSZ_MODE_ABS, ebf, nullptr, 0, w.consts, w.mm, st, w.status));
     const uint16_t* idx = d->has_trailer ? reinterpret_cast<const uint16_t*>(d_archive + d->index_offset) : nullptr;
     VSZ_TRY(decode_codes(d_archive + d->huff_offset, d->huff_bytes, d->node_count, d->tree_bytes, g.n, nsym, idx,
-                         d->has_trailer ? d->n_chunks : 0, d->chunk_syms, w, idx ? nullptr : w.seg_zero, g.d0, st));
-    // outlier ranks: per 512-code chunk from the indexed decoder (block size 8), else per 256-wide
-    // row segment
+                         d->has_trailer ? d->n_chunks : 0, d->chunk_syms, w, st));
+    // the outliers to their elements of the output: the indexed decoders count the zero codes of each
+    // chunk, other codes are counted here
+    OutlierArgs oa{};
+    oa.codes       = w.code;
+    oa.n           = g.n;
+    oa.nchunks     = (g.n + kChunkSyms - 1) / kChunkSyms;
+    oa.chunk_zero  = w.chunk_zero;
+    oa.chunk_off   = w.chunk_off;
+    oa.outliers    = d_archive + d->outlier_offset;
+    oa.n_out       = d->n_outlier;
+    oa.exact       = 1;
+    oa.out         = d_out;
+    oa.total       = w.scan_total;
+    oa.status      = w.status;
+    {
+        StageTimer t(kStZeroScan, st);
+        if (!indexed_counts(d)) VSZ_TRY(launch_count_zeros_chunk(w.code, g.n, w.chunk_zero, st, num_sms()));
+        VSZ_TRY(launch_scan_u32(w.chunk_zero, w.chunk_off, oa.nchunks, w.scan_status, w.scan_counter, w.scan_total,
+                                w.status, st));
+    }
+    {
+        StageTimer t(kStOutlierCopy, st);
+        VSZ_TRY(launch_outlier_scatter(oa, st, num_sms()));
+    }
     // VSZ_FORCE_GENERAL_DECOMPRESS: the general reverse-Lorenzo kernel for every block size (tests
-    // of that path); it ranks outliers by row segment only
+    // of that path)
     const bool force_general = getenv("VSZ_FORCE_GENERAL_DECOMPRESS") != nullptr;
-    // the block-8 kernel ranks outliers from the decoder's per-chunk zero counts directly, which
-    // costs a recount from the chunk start in every row segment holding outliers; with dense
-    // outliers (over 1 in 1024 elements) the per-segment zero counts are cheaper
-    const bool dense_outliers = d->n_outlier > g.n / 1024;
-    const bool chunk_rank     = idx != nullptr && bs == 8 && d->node_count > 1 && !force_general && !dense_outliers;
-    // the reverse Lorenzo's arguments (the outlier rank source is set after the zero scan)
     DqDecArgs a{};
     a.codes = w.code;
-    a.outliers = w.outliers;
+    a.outliers = oa.outliers;
     a.n_outliers = d->n_outlier;
     a.status = w.status;
-    a.seg_off = w.seg_off;
-    a.chunk_off = chunk_rank ? w.chunk_off : nullptr;
+    a.chunk_off = w.chunk_off;
     a.consts = w.consts;
     a.out = d_out;
     a.d0 = g.d0;
@@ -1301,32 +1314,6 @@ vsz_status vsz_decompress(const vsz_archive_desc* d, const vsz_decompress_opts* 
     a.redo   = w.redo;
     a.consts_rw = w.consts;
     a.dq_cache  = w.dq_cache;
-    // small 3D fields (the wavefront pass): zeros before each row's x-block of 8
-    a.blk_off = w.blk_off;
-    const bool blk_rank = bs == 8 && !force_general && d->n_outlier != 0 && dq_w8_applies(a, g.ndim);
-    {
-        StageTimer t(kStZeroScan, st);
-        if (blk_rank) {
-            VSZ_TRY(launch_count_zeros_b8(w.code, g.d0, g.nrows, w.blk_zero, st, num_sms()));
-            VSZ_TRY(launch_scan_u32(w.blk_zero, w.blk_off, g.nrows * ((g.d0 + 7) / 8), w.scan_status, w.scan_counter,
-                                    w.scan_total, w.status, st));
-        } else if (chunk_rank) {
-            VSZ_TRY(launch_scan_u32(w.chunk_zero, w.chunk_off, d->n_chunks, w.scan_status, w.scan_counter,
-                                    w.scan_total, w.status, st));
-        } else {
-            if (idx) VSZ_TRY(launch_count_zeros(w.code, g.d0, g.nrows, w.seg_zero, st, num_sms()));
-            VSZ_TRY(launch_scan_u32(w.seg_zero, w.seg_off, nsegd, w.scan_status, w.scan_counter, w.scan_total,
-                                    w.status, st));
-        }
-        k_check_zeros<<<1, 1, 0, st>>>(w.scan_total, d->n_outlier, w.status);
-        count_launch();
-    }
-    if (d->n_outlier) {
-        StageTimer t(kStOutlierCopy, st);
-        VSZ_CUDA(cudaMemcpyAsync(w.outliers, d_archive + d->outlier_offset, 4 * d->n_outlier, cudaMemcpyDeviceToDevice,
-                                 st));
-    }
-    a.blk_off = blk_rank ? w.blk_off : nullptr;
     {
         StageTimer t(kStLorenzoDecompress, st);
         VSZ_TRY(launch_dq_decompress(a, d->ndim, bs, force_general, st, num_sms()));
@@ -1574,7 +1561,7 @@ vsz_status vsz_decompress_f64_bounds(const vsz_archive_desc* d, size_t* ws_bytes
     size_t dims[3] = {d->dims[0], d->dims[1], d->dims[2]};
     if (!valid_dims(d->ndim, dims) || !valid_dict(d->dict_size) || !valid_bs(d->block_size)) return VSZ_ERR_CORRUPT;
     Geometry g = make_geometry(d->ndim, dims);
-    if (ws_bytes) *ws_bytes = layout_decompress(g, d->dict_size, d->payload_bytes, 0, d->n_chunks, nullptr, 0).bytes;
+    if (ws_bytes) *ws_bytes = layout_decompress(g, d->dict_size, d->payload_bytes, d->n_chunks, true, nullptr, 0).bytes;
     return VSZ_OK;
 }
 
@@ -1588,7 +1575,7 @@ vsz_status vsz_decompress_f64(const vsz_archive_desc* d, const uint8_t* d_archiv
     const int dict = d->dict_size;
     if (d->node_count > (uint32_t)(2 * dict - 1)) return VSZ_ERR_CORRUPT;
     Geometry g     = make_geometry(d->ndim, dims);
-    DecompressWs w = layout_decompress(g, dict, d->payload_bytes, 0, d->n_chunks, reinterpret_cast<uint8_t*>(d_ws),
+    DecompressWs w = layout_decompress(g, dict, d->payload_bytes, d->n_chunks, true, reinterpret_cast<uint8_t*>(d_ws),
                                        ws_bytes);
     if (w.bytes > ws_bytes) return VSZ_ERR_CAPACITY;
     cudaStream_t st    = S(stream);
@@ -1598,7 +1585,7 @@ vsz_status vsz_decompress_f64(const vsz_archive_desc* d, const uint8_t* d_archiv
                                 reinterpret_cast<unsigned long long*>(w.mm), w.status, st, num_sms()));
     const uint16_t* idx = reinterpret_cast<const uint16_t*>(d_archive + d->index_offset);
     VSZ_TRY(decode_codes(d_archive + d->huff_offset, d->huff_bytes, d->node_count, d->tree_bytes, g.n, dict, idx,
-                         d->n_chunks, d->chunk_syms, w, nullptr, g.d0, st));
+                         d->n_chunks, d->chunk_syms, w, st));
     {
         StageTimer t(kStZeroScan, st);
         VSZ_TRY(launch_count_zeros(w.code, g.d0, g.nrows, w.seg_zero, st, num_sms()));

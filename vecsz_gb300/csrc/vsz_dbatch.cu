@@ -39,12 +39,13 @@ constexpr size_t kDCtlInfo   = 80;  // u32[4] tree info (k_huff_table)
 
 constexpr uint64_t kDecTaskChunks = 256;      // one decoder CTA: lane t decodes chunk u0 + t, or
 constexpr uint64_t kSplitTaskChunks = 64;     // (split decoder) its warps take two chunks at a time
-constexpr uint64_t kCopyTaskBytes = 1 << 18;  // index and outlier copies
+constexpr uint64_t kCopyTaskBytes = 1 << 12;  // index copies: a few KB a CTA, so that they spread
+constexpr uint64_t kOutTaskChunks = 64;       // outlier placement
 constexpr uint64_t kDqTaskUnits   = 1;        // reverse-Lorenzo warp units per task (one warp's)
 constexpr size_t kDqNextOff       = 64;       // after the batch status in the control tail: one
 constexpr size_t kDqMaxClasses    = 16;       // task counter per reverse-Lorenzo class
 
-// A byte range copied into an aligned buffer (the archive's index and outlier sections).
+// A byte range copied into an aligned buffer (the archive's index).
 struct DCopy {
     const uint8_t* src;
     uint8_t* dst;
@@ -163,12 +164,11 @@ struct DLayout {
     uint32_t* scan_counter;
     std::vector<uint32_t*> table, table2, win, child, node_sym, parent, walk, redo;
     std::vector<uint16_t*> code;
-    std::vector<float*> outliers;
     std::vector<size_t> chunk_base;
     size_t bytes;
 };
 
-DLayout layout_dbatch(const std::vector<DField>& fs, const vsz_dbatch_field* fields, uint8_t* base, size_t cap) {
+DLayout layout_dbatch(const std::vector<DField>& fs, uint8_t* base, size_t cap) {
     Bump b{base, cap};
     DLayout L{};
     const size_t nf = fs.size();
@@ -196,7 +196,6 @@ DLayout layout_dbatch(const std::vector<DField>& fs, const vsz_dbatch_field* fie
         L.parent.push_back(b.take<uint32_t>(maxn));
         L.walk.push_back(b.take<uint32_t>(maxn));
         L.code.push_back(b.take<uint16_t>(f.g.n + 8));
-        L.outliers.push_back(b.take<float>(fields[i].desc.n_outlier + 4));
         L.redo.push_back(f.sep ? b.take<uint32_t>(f.units + 2) : nullptr);
     }
     L.bytes = b.off + 256;
@@ -244,7 +243,7 @@ struct vsz_dbatch {
     const HuffDecodeArgs* dec = nullptr;
     const DqDecArgs* dq = nullptr;
     const DCopy* copy_index = nullptr;
-    const DCopy* copy_out = nullptr;
+    const OutlierArgs* outliers = nullptr;
     const DCheck* check = nullptr;
     const BatchTask* tasks = nullptr;
     uint32_t idx_off = 0, idx_n = 0, dec_off = 0, dec_n = 0, const_off = 0, const_n = 0, out_off = 0, out_n = 0;
@@ -266,7 +265,7 @@ extern "C" {
 vsz_status vsz_dbatch_workspace_bytes(const vsz_dbatch_field* fields, int nfields, size_t* ws_bytes) {
     std::vector<DField> fs;
     VSZ_TRY(dfields(fields, nfields, fs));
-    if (ws_bytes) *ws_bytes = layout_dbatch(fs, fields, nullptr, 0).bytes;
+    if (ws_bytes) *ws_bytes = layout_dbatch(fs, nullptr, 0).bytes;
     return VSZ_OK;
 }
 
@@ -276,14 +275,15 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     *out = nullptr;
     std::vector<DField> fs;
     VSZ_TRY(dfields(fields, nfields, fs));
-    DLayout L = layout_dbatch(fs, fields, reinterpret_cast<uint8_t*>(d_ws), ws_bytes);
+    DLayout L = layout_dbatch(fs, reinterpret_cast<uint8_t*>(d_ws), ws_bytes);
     if (L.bytes > ws_bytes) return VSZ_ERR_CAPACITY;
     const uint32_t nf = (uint32_t)nfields;
     std::vector<ConstsField> cs(nf);
     std::vector<HuffTableArgs> ta(nf);
     std::vector<HuffDecodeArgs> da(nf);
     std::vector<DqDecArgs> qa(nf);
-    std::vector<DCopy> ci(nf), co(nf);
+    std::vector<DCopy> ci(nf);
+    std::vector<OutlierArgs> oa(nf);
     std::vector<DCheck> ck(nf);
     std::vector<BatchTask> tasks;
     vsz_dbatch* B = new vsz_dbatch();
@@ -334,8 +334,6 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         h.chunk_syms      = kChunkSyms;
         h.codes           = L.code[f];
         h.n               = G.g.n;
-        h.d0              = G.g.d0;
-        h.nxs             = (G.g.d0 + 255) / 256;
         h.max_nodes       = (uint32_t)(2 * G.nsym - 1);
         h.tree_info       = info;
         h.status          = status;
@@ -343,7 +341,7 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         DqDecArgs& q  = qa[f];
         q             = DqDecArgs{};
         q.codes       = L.code[f];
-        q.outliers    = L.outliers[f];
+        q.outliers    = F.d_archive + d.outlier_offset;
         q.n_outliers  = d.n_outlier;
         q.status      = status;
         q.chunk_off   = L.all_zoff + base;
@@ -360,7 +358,17 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         if (!G.sep) dq_b8_narrow(q, G.g.ndim);
 
         ci[f] = DCopy{F.d_archive + d.index_offset, reinterpret_cast<uint8_t*>(L.all_bits + base), status};
-        co[f] = DCopy{F.d_archive + d.outlier_offset, reinterpret_cast<uint8_t*>(L.outliers[f]), status};
+        OutlierArgs& o = oa[f];
+        o              = OutlierArgs{};
+        o.codes        = L.code[f];
+        o.n            = G.g.n;
+        o.nchunks      = G.nch;
+        o.chunk_zero   = L.all_zero + base;
+        o.chunk_off    = L.all_zoff + base;
+        o.outliers     = F.d_archive + d.outlier_offset;
+        o.n_out        = d.n_outlier;
+        o.out          = F.d_out;
+        o.status       = status;
         ck[f] = DCheck{L.all_zoff + base, G.nch, d.n_outlier, consts, status, d_status + f, L.redo[f]};
     }
     // ---- task lists
@@ -378,7 +386,8 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         if (fs[f].konst) add_tasks(tasks, f, fs[f].nch, dec_per);
     B->const_n = (uint32_t)tasks.size() - B->const_off;
     B->out_off = (uint32_t)tasks.size();
-    for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, 4 * fields[f].desc.n_outlier, kCopyTaskBytes);
+    for (uint32_t f = 0; f < nf; f++)
+        if (fields[f].desc.n_outlier) add_tasks(tasks, f, fs[f].nch, kOutTaskChunks);
     B->out_n = (uint32_t)tasks.size() - B->out_off;
     std::map<std::tuple<int, bool, bool>, std::vector<uint32_t>> classes;
     for (uint32_t f = 0; f < nf; f++) classes[std::make_tuple(fs[f].g.ndim, fs[f].vec, fs[f].sep)].push_back(f);
@@ -409,7 +418,7 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     };
     const size_t o_cs = place(sizeof(ConstsField) * nf), o_ta = place(sizeof(HuffTableArgs) * nf),
                  o_da = place(sizeof(HuffDecodeArgs) * nf), o_qa = place(sizeof(DqDecArgs) * nf),
-                 o_ci = place(sizeof(DCopy) * nf), o_co = place(sizeof(DCopy) * nf), o_ck = place(sizeof(DCheck) * nf),
+                 o_ci = place(sizeof(DCopy) * nf), o_oa = place(sizeof(OutlierArgs) * nf), o_ck = place(sizeof(DCheck) * nf),
                  o_tk = place(sizeof(BatchTask) * std::max<size_t>(tasks.size(), 1));
     const size_t table_bytes = off + 256;
     std::vector<uint8_t> h(table_bytes, 0);
@@ -418,7 +427,7 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     memcpy(h.data() + o_da, da.data(), sizeof(HuffDecodeArgs) * nf);
     memcpy(h.data() + o_qa, qa.data(), sizeof(DqDecArgs) * nf);
     memcpy(h.data() + o_ci, ci.data(), sizeof(DCopy) * nf);
-    memcpy(h.data() + o_co, co.data(), sizeof(DCopy) * nf);
+    memcpy(h.data() + o_oa, oa.data(), sizeof(OutlierArgs) * nf);
     memcpy(h.data() + o_ck, ck.data(), sizeof(DCheck) * nf);
     if (!tasks.empty()) memcpy(h.data() + o_tk, tasks.data(), sizeof(BatchTask) * tasks.size());
     if (cudaMalloc(reinterpret_cast<void**>(&B->d_tables), table_bytes) != cudaSuccess) {
@@ -434,7 +443,7 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     B->dec          = reinterpret_cast<const HuffDecodeArgs*>(B->d_tables + o_da);
     B->dq           = reinterpret_cast<const DqDecArgs*>(B->d_tables + o_qa);
     B->copy_index   = reinterpret_cast<const DCopy*>(B->d_tables + o_ci);
-    B->copy_out     = reinterpret_cast<const DCopy*>(B->d_tables + o_co);
+    B->outliers     = reinterpret_cast<const OutlierArgs*>(B->d_tables + o_oa);
     B->check        = reinterpret_cast<const DCheck*>(B->d_tables + o_ck);
     B->tasks        = reinterpret_cast<const BatchTask*>(B->d_tables + o_tk);
     B->ctl          = L.ctl;
@@ -494,9 +503,7 @@ vsz_status vsz_dbatch_decompress(vsz_dbatch* B, void* stream) {
     }
     if (B->out_n) {
         StageTimer t(kStOutlierCopy, st);
-        k_dbatch_copy<<<std::min<uint32_t>(B->out_n, (uint32_t)sms * 8), 256, 0, st>>>(B->copy_out,
-                                                                                      B->tasks + B->out_off, B->out_n);
-        count_launch();
+        VSZ_TRY(launch_outlier_scatter_batch(B->outliers, B->tasks + B->out_off, B->out_n, st, sms));
     }
     {
         StageTimer t(kStLorenzoDecompress, st);

@@ -123,8 +123,6 @@ struct HuffDecodeArgs {
     uint32_t chunk_syms;
     uint16_t* codes;
     size_t n;
-    uint32_t* seg_zero;                   // zero codes per 256-wide row segment (may be null)
-    uint32_t d0, nxs;
     uint32_t max_nodes;                   // node indices past this are a corrupt tree
     const uint32_t* win;                  // k_huff_table's image for the split decoder, or null
     const uint32_t* tree_info;            // k_huff_table's info ([2] longest codeword), or null
@@ -173,8 +171,7 @@ int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks,
                              const BatchTask* const_tasks, uint32_t nconst, size_t total_chunks, cudaStream_t st,
                              int num_sms);
 int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms);
-int launch_huff_const(uint16_t* codes, size_t n, const uint32_t* info, uint32_t* seg_zero, uint32_t d0, uint32_t nxs,
-                      const int* status, cudaStream_t st, int num_sms);
+int launch_huff_const(uint16_t* codes, size_t n, const uint32_t* info, const int* status, cudaStream_t st, int num_sms);
 int launch_huff_sync_init(HuffSyncArgs a, cudaStream_t st);
 int launch_huff_sync_round(HuffSyncArgs a, const unsigned long long* exit_in, unsigned long long* exit_out,
                            int* changed, cudaStream_t st);

@@ -130,13 +130,27 @@ struct GatherArgs {
 };
 
 // ---- dual-quant decompress ----------------------------------------------------------------
+// Outlier placement (k_outlier_scatter): out[i] = the next outlier for every code 0.
+struct OutlierArgs {
+    const uint16_t* codes;
+    size_t n;
+    size_t nchunks;                      // of 512 codes
+    const uint32_t* chunk_zero;          // zero codes per chunk
+    const unsigned long long* chunk_off; // their exclusive scan (a batch: relative to chunk_off[0])
+    const unsigned long long* total;     // and its total (one field only)
+    const uint8_t* outliers;             // f32 values at any byte address (4 readable bytes past them)
+    unsigned long long n_out;            // their number
+    int exact;                           // 1: other counts of zero codes are VSZ_ERR_CORRUPT, 0: larger ones
+    float* out;
+    int* status;
+};
+
 struct DqDecArgs {
     const uint16_t* codes;
-    const float* outliers;               // compact outlier values (aligned copy)
-    unsigned long long n_outliers;       // entries of `outliers`; a rank past it is VSZ_ERR_CORRUPT
+    const uint8_t* outliers;             // separable pass: the archive's outlier section (any alignment)
+    unsigned long long n_outliers;       // outliers of the field
     int* status;
-    const unsigned long long* seg_off;   // exclusive zero-code offsets per 256-wide row segment, or
-    const unsigned long long* chunk_off; // exclusive zero-code offsets per 512-code chunk (block 8),
+    const unsigned long long* chunk_off; // separable pass: outliers before each 512-code chunk,
                                          // relative to chunk_off[0]
     const Consts* consts;
     float* out;
@@ -159,16 +173,20 @@ struct DqDecArgs {
                                          // large field records its dequantization check there (or null)
     unsigned long long* dq_cache;        // 4 words kept across calls: the last check's c_d and result
                                          // (or null)
-    const unsigned long long* blk_off;   // 3D block 8, fields of at most kW8MaxN elements: exclusive
-                                         // zero-code offsets per (row, x-block of 8), or null
 };
 
 // 3D block-8 fields up to this many elements take the wavefront reverse Lorenzo
-// (k_dq_decompress_w8), which ranks outliers from per-(row, x-block) zero offsets.
+// (k_dq_decompress_w8).
 constexpr size_t kW8MaxN = size_t(1) << 24;
 // ... and those that would take the separable pass only up to this many.
 constexpr size_t kW8MaxSeparableN = size_t(1) << 23;
 
+// Zero codes per 512-code chunk; the placement of one field's outliers; of many fields' (tasks of
+// (field, chunk range)).  Both after the scan of the counts.  The reverse Lorenzo launchers below expect it done.
+int launch_count_zeros_chunk(const uint16_t* codes, size_t n, uint32_t* chunk_zero, cudaStream_t st, int num_sms);
+int launch_outlier_scatter(const OutlierArgs& a, cudaStream_t st, int num_sms);
+int launch_outlier_scatter_batch(const OutlierArgs* args, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st,
+                                 int num_sms);
 int launch_dq_decompress(DqDecArgs a, int ndim, int bs, bool force_general, cudaStream_t st, int num_sms);
 // Block size 8: unit geometry (nxs, nyb, nunits), whether the 16-byte row path applies, and
 // whether the separable pass does (3D, vector rows, not strict, no padding, under 1 outlier in 64).
@@ -179,11 +197,8 @@ void dq_b8_narrow(DqDecArgs& a, int ndim);
 bool dq_b8_vec(const DqDecArgs& a);
 bool dq_b8_separable(const DqDecArgs& a, int ndim);
 // The wavefront pass applies: 3D, no padding, at most kW8MaxN elements (kW8MaxSeparableN for a
-// field the separable pass takes), blk_off given (or no outliers), VSZ_DQ_NO_WAVEFRONT unset.
+// field the separable pass takes), VSZ_DQ_NO_WAVEFRONT unset.
 bool dq_w8_applies(const DqDecArgs& a, int ndim);
-// Zero codes per (row, x-block of 8), row-major: nrows * ceil(d0 / 8) counts.
-int launch_count_zeros_b8(const uint16_t* codes, uint32_t d0, size_t nrows, uint32_t* blk_zero, cudaStream_t st,
-                          int num_sms);
 // Many fields of one class (ndim, vec, separable), block size 8, no padding: tasks of (field,
 // unit range), one warp each, handed out through the counter `next` (zero on entry; the class's
 // own word).  A separable class is followed by launch_dq_redo_batch over its fields.
