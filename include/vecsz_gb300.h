@@ -284,8 +284,8 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
                             uint64_t* d_results, vsz_batch** batch);
 vsz_status vsz_batch_compress(vsz_batch* batch, void* stream);
 void vsz_batch_destroy(vsz_batch* batch);
-/* Work per block-wide task: dual-quant warp units (default 32) and encoder 512-code chunks
- * (default 64).  Rebuilds and uploads the task lists (synchronous): call before capturing
+/* Work per block-wide task: dual-quant warp units (by default at most 32) and encoder 512-code chunks
+ * (at most 64; fewer where the batch would not fill the GPU).  Rebuilds and uploads the task lists (synchronous): call before capturing
  * vsz_batch_compress in a graph.  vsz_batch_autotune times vsz_batch_compress over dual-quant sizes
  * {8, 16, 32, 64, 128}, then encoder sizes {16, 32, 64, 128, 256} (`iterations` timed runs each
  * after one warm-up, CUDA events on `stream`, synchronising), keeps the fastest pair and reports it;

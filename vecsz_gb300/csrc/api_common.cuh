@@ -103,6 +103,7 @@ inline DqArgs make_dq_args(const Geometry& g, int bs, int dict, const float* x, 
     a.nxt = g.nxt;
     a.nyg = (g.d1 + 7) / 8;
     a.nzb = (g.ndim == 3) ? (g.d2 + bs - 1) / bs : 1;
+    a.zlen = (g.ndim == 3) ? (uint32_t)bs : 1u;
     a.xtail = (g.d0 % 8) ? (g.d0 & ~7u) : g.d0;
     a.R = dict / 2;
     a.dict = dict;

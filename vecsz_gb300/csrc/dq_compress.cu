@@ -246,8 +246,8 @@ __device__ __forceinline__ int code_of(float e, float rmagic) {
 }
 
 template <int NDIM, bool TAIL>
-__device__ __forceinline__ float prequant_at(float v, uint32_t col, uint32_t xtail, float r_f, double r_d) {
-    if (NDIM == 3 && TAIL && col >= xtail) return prequant_scalar(v, r_d);
+__device__ __forceinline__ float prequant_at(float v, uint32_t col, uint32_t xtail, float r_f, const ScalarMul& sm) {
+    if (NDIM == 3 && TAIL && col >= xtail) return prequant_scalar(v, r_f, sm.r_lo, sm.split, sm.r_d);
     return prequant_vec(v, r_f);
 }
 
@@ -270,18 +270,21 @@ __device__ __forceinline__ float4 load_raw(const DqArgs& a, size_t row, bool row
 
 // Prequantized values of a raw row; zero outside the field.
 template <int NDIM, bool TAIL, bool FULL = false>
-__device__ __forceinline__ void prequant_row(const DqArgs& a, float4 v, bool row_in, uint32_t xb, float r_f, double r_d,
+__device__ __forceinline__ void prequant_row(const DqArgs& a, float4 v, bool row_in, uint32_t xb, float r_f, const ScalarMul& sm,
                                              float S[4]) {
     const float t[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const bool in = FULL || (row_in && (xb + j < a.d0));
-        S[j]          = in ? prequant_at<NDIM, TAIL>(t[j], xb + j, a.xtail, r_f, r_d) : 0.0f;
+        S[j]          = in ? prequant_at<NDIM, TAIL>(t[j], xb + j, a.xtail, r_f, sm) : 0.0f;
     }
 }
 
-// 2D / 3D.  Work unit = one warp tile: 128 consecutive x (4 per lane) by 8 rows (y) by one
-// Lorenzo block of planes (z).  Rows are processed one at a time (the next row's values are
+// 2D / 3D.  Work unit = one warp tile: 128 consecutive x (4 per lane) by 8 rows (y) by a.zlen planes
+// (z) of one Lorenzo block.  A field with fewer units than the GPU holds warps is bound by a unit's
+// chain of rows (64^3: 64 units of 64 rows, 38 us), so its blocks are split along z (dq_set_zlen): a
+// unit that does not start its block first prequantizes the plane before it, which costs 1 / zlen
+// of the loads and prequantizations again.  Rows are processed one at a time (the next row's values are
 // loaded while the current one is coded); a lane keeps in registers only its 4 values of the
 // current row and of the row above, in this plane and in the previous one.  The previous plane's
 // 8 rows live in shared memory [row][column][lane] (conflict-free), each row overwritten by the
@@ -320,7 +323,7 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
                                            unsigned long long u1, unsigned long long ustep, uint32_t* s_hist,
                                            PrevRows* s_prev, HistAcc& h) {
     const float r_f     = c.r_f;
-    const double r_d    = c.r_d;
+    const ScalarMul sm  = (NDIM == 3 && TAIL) ? scalar_mul(c.r_d, r_f) : ScalarMul{};
     const float Rf      = (float)a.R;
     const float rmagic  = Rf + 12582912.0f;
     const unsigned lane = lane_id();
@@ -335,12 +338,12 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
         const uint32_t xt = u % a.nxt;
         const uint32_t r = u / a.nxt;
         const uint32_t yg = r % a.nyg;
-        const uint32_t zb = r / a.nyg;
         const uint32_t xb = xt * kTileX + lane * 4;
         const uint32_t y0 = yg * 8;
         const bool yhalo  = (BS > 8) && (y0 % BS) != 0;  // the row above is inside the block
-        const uint32_t z0 = (NDIM == 3) ? zb * BS : 0;
-        const int nz      = (NDIM == 3) ? (int)min((uint32_t)BS, a.d2 - z0) : 1;
+        const uint32_t z0 = (NDIM == 3) ? (r / a.nyg) * a.zlen : 0;
+        const int nz      = (NDIM == 3) ? (int)min(a.zlen, a.d2 - z0) : 1;
+        const bool zin    = NDIM == 3 && (z0 % BS) != 0;  // the plane before is inside the block
 
         // a tile wholly inside the field (the common case) runs without per-element range checks
         const bool full = VEC && (xt + 1) * kTileX <= a.d0 && y0 + 8 <= a.d1;
@@ -352,7 +355,7 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
             // cell of the lane to the left, same block
             float hx = 0.f, hy = 0.f, hz = 0.f;
             if (PAD && xb < a.d0) {
-                const Halo hv = halo_of(a.pad, NDIM, xb / BS, y0 / BS, zb);
+                const Halo hv = halo_of(a.pad, NDIM, xb / BS, y0 / BS, z0 / BS);
                 hx = hv.x;
                 hy = hv.y;
                 hz = hv.z;
@@ -360,14 +363,34 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
             const float hxy = (xbound && NDIM == 2) ? hx : hy;
 
             float Ph[4] = {hz, hz, hz, hz}, PhL = hz;  // previous plane's halo row (y0 - 1)
+            if (NDIM == 3 && zin) {
+                const size_t rp = (size_t)(z0 - 1) * a.d1 + y0;
+                float4 raw[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) raw[i] = load_raw<VEC, FULL>(a, rp + i, y0 + i < a.d1, xb);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    float S[4];
+                    prequant_row<NDIM, TAIL, FULL>(a, raw[i], y0 + i < a.d1, xb, r_f, sm, S);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) s_prev[wib][i][j][lane] = S[j];
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) Ph[j] = hy;
+                PhL = hxy;
+                if (yhalo) {
+                    prequant_row<NDIM, TAIL, FULL>(a, load_raw<VEC, FULL>(a, rp - 1, true, xb), true, xb, r_f, sm, Ph);
+                    PhL = left(Ph[3], hx);
+                }
+            }
             float4 nxt = load_raw<VEC, FULL>(a, (size_t)z0 * a.d1 + y0, y0 < a.d1, xb);
             for (int zz = 0; zz < nz; zz++) {
                 const uint32_t z = z0 + zz;
-                const bool zp    = zz > 0;  // a previous plane inside the block
+                const bool zp    = zin || zz > 0;  // a previous plane inside the block
                 float Sp[4] = {hy, hy, hy, hy}, SpL = hxy;  // row above, this plane (halo row at i = 0)
                 if (yhalo) {
                     prequant_row<NDIM, TAIL, FULL>(a, load_raw<VEC, FULL>(a, (size_t)z * a.d1 + (y0 - 1), true, xb), true, xb, r_f,
-                                             r_d, Sp);
+                                             sm, Sp);
                     SpL = left(Sp[3], hx);
                 }
                 const float ShNext[4] = {Sp[0], Sp[1], Sp[2], Sp[3]};
@@ -385,7 +408,7 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
                         nxt = more ? load_raw<VEC, FULL>(a, (size_t)zn * a.d1 + yn, yn < a.d1, xb) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
                     float S[4];
-                    prequant_row<NDIM, TAIL, FULL>(a, raw, row_in, xb, r_f, r_d, S);
+                    prequant_row<NDIM, TAIL, FULL>(a, raw, row_in, xb, r_f, sm, S);
                     const float SL = left(S[3], hx);
                     float Pc[4] = {hz, hz, hz, hz}, PcL = hz;  // this row, previous plane
                     if (NDIM == 3) {
@@ -484,39 +507,11 @@ __global__ void __launch_bounds__(256, 4) k_dq_compress_23d(DqArgs a) {
     hist_flush_block(a, s_hist, h);
 }
 
-// Many fields in one launch: block-wide tasks (one field, a range of its warp units), each taken
-// by the next free block (`next`: the launch's task counter, zero at launch), so that blocks do
-// not idle behind uneven tasks.  hist_words = shared-memory histogram words reserved before the
-// planes.
 __device__ __forceinline__ uint32_t dq_block_next_task(uint32_t* next, uint32_t* s_task) {
     __syncthreads();  // every thread has read the previous task number
     if (threadIdx.x == 0) *s_task = atomicAdd(next, 1u);
     __syncthreads();
     return *s_task;
-}
-
-template <int NDIM, int BS, bool VEC, bool TAIL>
-__global__ void __launch_bounds__(256, 3)
-    k_dq_compress_23d_batch(const DqArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks,
-                            uint32_t hist_words, uint32_t* __restrict__ next) {
-    extern __shared__ __align__(16) uint32_t s_dyn[];
-    __shared__ uint32_t s_task;
-    PrevRows* s_prev = reinterpret_cast<PrevRows*>(s_dyn + hist_words);
-    for (uint32_t t = dq_block_next_task(next, &s_task); t < ntasks; t = dq_block_next_task(next, &s_task)) {
-        const BatchTask tk = tasks[t];
-        const DqArgs& a    = args[tk.field];  // read-only table: loads stay cached
-        const Consts c     = *a.consts;
-        if (c.status != VSZ_OK) continue;  // uniform: the whole block is on this task
-        uint32_t* s_hist = a.smem_hist ? s_dyn : nullptr;
-        if (s_hist) {
-            for (int i = threadIdx.x; i < a.dict; i += blockDim.x) s_hist[i] = 0u;
-            __syncthreads();
-        }
-        HistAcc h;
-        dq23_units<NDIM, BS, VEC, TAIL>(a, c, tk.u0 + (threadIdx.x >> 5), tk.u1, blockDim.x >> 5, s_hist, s_prev, h);
-        hist_flush_block(a, s_hist, h);
-        __syncthreads();  // the next task reuses shared memory
-    }
 }
 
 // 1D: 4 consecutive 128-element tiles per warp unit; the x - 1 neighbour comes from the lane to
@@ -540,7 +535,7 @@ __device__ __forceinline__ void dq1d_units(const DqArgs& a, const Consts& c, uns
             const uint32_t xb = xt * kTileX + lane * 4;
             const float4 rw   = load_raw<VEC>(a, 0, xt < a.nxt, xb);
             if (STRICT) RW[STRICT ? t : 0] = rw;
-            prequant_row<1, false>(a, rw, xt < a.nxt, xb, r_f, 0.0, S[t]);
+            prequant_row<1, false>(a, rw, xt < a.nxt, xb, r_f, ScalarMul{}, S[t]);
         }
 #pragma unroll
         for (int t = 0; t < U; t++) {
@@ -604,26 +599,45 @@ __global__ void __launch_bounds__(256) k_dq_compress_1d(DqArgs a) {
     hist_flush_block(a, s_hist, h);
 }
 
-template <int BS, bool VEC>
-__global__ void __launch_bounds__(256)
-    k_dq_compress_1d_batch(const DqArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks,
-                           uint32_t* __restrict__ next) {
-    extern __shared__ uint32_t s_hist_dyn[];
+// Many fields in one launch: block-wide tasks (one field, a range of its warp units), each taken
+// by the next free block (`next`: the launch's task counter, zero at launch), so that blocks do
+// not idle behind uneven tasks.  Fields of every dimensionality and alignment share the launch (the
+// task names its class): a launch per class ran one after another, most of them too small to fill
+// the GPU (60 mixed fields: 8 launches, 1.37 ms).  hist_words = shared-memory histogram words
+// reserved before the planes.
+template <int BS>
+__global__ void __launch_bounds__(256, 3)
+    k_dq_compress_batch(const DqArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks,
+                        uint32_t hist_words, uint32_t* __restrict__ next) {
+    extern __shared__ __align__(16) uint32_t s_dyn[];
     __shared__ uint32_t s_task;
+    PrevRows* s_prev = reinterpret_cast<PrevRows*>(s_dyn + hist_words);
     for (uint32_t t = dq_block_next_task(next, &s_task); t < ntasks; t = dq_block_next_task(next, &s_task)) {
         const BatchTask tk = tasks[t];
-        const DqArgs& a    = args[tk.field];
+        const DqArgs& a    = args[tk.field];  // read-only table: loads stay cached
         const Consts c     = *a.consts;
-        if (c.status != VSZ_OK) continue;
-        uint32_t* s_hist = a.smem_hist ? s_hist_dyn : nullptr;
+        if (c.status != VSZ_OK) continue;  // uniform: the whole block is on this task
+        uint32_t* s_hist = a.smem_hist ? s_dyn : nullptr;
         if (s_hist) {
             for (int i = threadIdx.x; i < a.dict; i += blockDim.x) s_hist[i] = 0u;
             __syncthreads();
         }
         HistAcc h;
-        dq1d_units<BS, VEC>(a, c, tk.u0 + (threadIdx.x >> 5), tk.u1, blockDim.x >> 5, s_hist, h);
+        const unsigned long long u0 = tk.u0 + (threadIdx.x >> 5), us = blockDim.x >> 5;
+        switch (tk.pad) {
+            case 4 + 0: case 4 + 1: dq1d_units<BS, false>(a, c, u0, tk.u1, us, s_hist, h); break;
+            case 4 + 2: case 4 + 3: dq1d_units<BS, true>(a, c, u0, tk.u1, us, s_hist, h); break;
+            case 8 + 0: dq23_units<2, BS, false, false>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+            case 8 + 1: dq23_units<2, BS, false, true>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+            case 8 + 2: dq23_units<2, BS, true, false>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+            case 8 + 3: dq23_units<2, BS, true, true>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+            case 12 + 0: dq23_units<3, BS, false, false>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+            case 12 + 1: dq23_units<3, BS, false, true>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+            case 12 + 2: dq23_units<3, BS, true, false>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+            case 12 + 3: dq23_units<3, BS, true, true>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+        }
         hist_flush_block(a, s_hist, h);
-        __syncthreads();
+        __syncthreads();  // the next task reuses shared memory
     }
 }
 
@@ -638,37 +652,59 @@ constexpr int kGatherThreads = 256;
 constexpr int kGatherPerThread = 16;
 constexpr int kGatherTile = kGatherThreads * kGatherPerThread;  // segments per tile
 
-// One tile of 4096 row segments of one field: the next ticket of the field's look-back.  The
-// status is read once per block, so the early exit is uniform.
-// Copies the n outliers of segment s from scratch to outlier index dst0 of the destination (one
-// warp).  A byte destination is written as whole aligned words, each the bytes of two neighbouring
-// values (funnel shift); only the partial words at the run's two ends, shared with the
-// neighbouring runs, are written byte by byte.
-__device__ __forceinline__ void copy_segment(const GatherArgs& g, uint8_t* out_bytes, size_t s, uint32_t n,
-                                             unsigned long long dst0) {
+// Copies the outliers of 32 consecutive segments (lane l: cn of segment s0 + l, the group's first one
+// outlier dst0 of the destination), by one warp.  They are consecutive in the destination, so a lane
+// takes every 32nd of them, whatever segment it lies in (found by bisection of the segments' ends over
+// the lanes): a load latency per 32 outliers, not per segment.  A byte destination is written as
+// whole aligned words, each the bytes of two neighbouring values (funnel shift); only the partial
+// words at the run's two ends, shared with the neighbouring runs, are written byte by byte.
+__device__ __forceinline__ void copy_segments(const GatherArgs& g, uint8_t* out_bytes, size_t s0, uint32_t cn,
+                                              unsigned long long dst0) {
     const unsigned lane = lane_id();
-    const float* src    = g.scratch + s * kSegX;
+    uint32_t incl       = cn;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (unsigned)o) incl += t;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    if (total == 0) return;
+    auto value = [&](uint32_t t) -> uint32_t {  // outlier t of the group (t < total, all lanes call it)
+        uint32_t k = 0;                           // its segment: the first that ends past t
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            if (__shfl_sync(0xffffffffu, incl, k + o - 1) <= t) k += o;
+        const uint32_t before = __shfl_sync(0xffffffffu, incl - cn, k);
+        return __float_as_uint(g.scratch[(s0 + k) * kSegX + (t - before)]);
+    };
     if (g.out_f32) {
-        for (uint32_t i = lane; i < n; i += 32) g.out_f32[dst0 + i] = src[i];
+        for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+            const uint32_t t = t0 + lane, v = value(min(t, total - 1));
+            if (t < total) g.out_f32[dst0 + t] = __uint_as_float(v);
+        }
         return;
     }
-    uint8_t* d          = out_bytes + 4 * dst0;
-    const uint32_t a    = (uint32_t)(reinterpret_cast<uintptr_t>(d) & 3u);
-    const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src);
-    if (a == 0) {
-        uint32_t* dw = reinterpret_cast<uint32_t*>(d);
-        for (uint32_t i = lane; i < n; i += 32) dw[i] = s32[i];
-        return;
-    }
-    uint32_t* dw = reinterpret_cast<uint32_t*>(d + (4 - a));  // word j: top a bytes of value j, low 4 - a of j + 1
-    for (uint32_t j = lane; j + 1 < n; j += 32) dw[j] = __funnelshift_r(s32[j], s32[j + 1], 8 * (4 - a));
-    if (lane == 0) {
-        const uint32_t b0 = s32[0], bl = s32[n - 1];
-        for (uint32_t t = 0; t < 4 - a; t++) d[t] = (uint8_t)(b0 >> (8 * t));                    // value 0, low bytes
-        for (uint32_t t = 0; t < a; t++) d[4 * n - a + t] = (uint8_t)(bl >> (8 * (4 - a + t)));  // value n-1, top bytes
+    uint8_t* d       = out_bytes + 4 * dst0;
+    const uint32_t a = (uint32_t)(reinterpret_cast<uintptr_t>(d) & 3u);
+    // word t of dw: the top a bytes of value t and the low 4 - a bytes of value t + 1 (a = 0: value t)
+    uint32_t* dw = reinterpret_cast<uint32_t*>(a ? d + (4 - a) : d);
+    const uint32_t step = a ? 31u : 32u;
+    for (uint32_t t0 = 0; t0 < total; t0 += step) {
+        const uint32_t t = t0 + lane, v = value(min(t, total - 1)), vn = __shfl_down_sync(0xffffffffu, v, 1);
+        if (a == 0) {
+            if (t < total) dw[t] = v;
+        } else {
+            if (lane < 31 && t + 1 < total) dw[t] = __funnelshift_r(v, vn, 8 * (4 - a));
+            if (t == 0)
+                for (uint32_t q = 0; q < 4 - a; q++) d[q] = (uint8_t)(v >> (8 * q));  // value 0, low bytes
+            if (t == total - 1)  // the last value's top bytes
+                for (uint32_t q = 0; q < a; q++) d[4 * total - a + q] = (uint8_t)(v >> (8 * (4 - a + q)));
+        }
     }
 }
 
+// One tile of 4096 row segments of one field: the next ticket of the field's look-back.  The
+// status is read once per block, so the early exit is uniform.
 __device__ __forceinline__ void gather_tile(const GatherArgs& g) {
     __shared__ uint32_t s_off[kGatherTile];
     __shared__ uint8_t s_cnt[kGatherTile];
@@ -745,40 +781,40 @@ __device__ __forceinline__ void gather_tile(const GatherArgs& g) {
         return;
     }
     uint8_t* out_bytes = g.out_bytes ? g.out_bytes + g.out_off.eval() : nullptr;
-    // warp-cooperative copies of the non-empty segments: each warp scans 32 segment counts at a
-    // time from shared memory and visits only those with outliers
-    for (int k0 = w * 32; k0 < kGatherTile; k0 += kGatherThreads) {
+    for (int k0 = w * 32; k0 < kGatherTile; k0 += kGatherThreads) {  // 32 segments of each warp at a time
         const int kk = k0 + (int)lane;
-        const bool has = (tseg0 + kk < g.nseg) && s_cnt[kk] != 0;
-        unsigned nz = __ballot_sync(0xffffffffu, has);
-        while (nz) {
-            const int k = k0 + __ffs(nz) - 1;
-            nz &= nz - 1;
-            copy_segment(g, out_bytes, tseg0 + k, s_cnt[k], base + s_off[k]);
-        }
+        copy_segments(g, out_bytes, tseg0 + k0, (tseg0 + kk < g.nseg) ? s_cnt[kk] : 0u, base + s_off[k0]);
     }
 }
 
 __global__ void __launch_bounds__(kGatherThreads) k_outlier_gather(GatherArgs g) { gather_tile(g); }
 
-// Split copy: every warp of the grid takes 32 segments at a time and copies the non-empty ones.
+// Split copy: every warp of the grid takes 32 segments at a time (which never straddle a tile).
+__device__ __forceinline__ void copy_group(const GatherArgs& g, uint8_t* out_bytes, size_t s0, size_t s1) {
+    const size_t s    = s0 + lane_id();
+    const uint32_t cn = (s < s1) ? g.seg_count[s] : 0u;
+    if (!__any_sync(0xffffffffu, cn != 0u)) return;
+    copy_segments(g, out_bytes, s0, cn, g.tile_base[s0 / kGatherTile] + g.seg_off[s0]);
+}
+
 __global__ void __launch_bounds__(256) k_outlier_copy(GatherArgs g) {
     if (*g.status != VSZ_OK || *g.total == 0) return;  // a field without outliers returns at once
-    const unsigned lane = lane_id();
     uint8_t* out_bytes  = g.out_bytes ? g.out_bytes + g.out_off.eval() : nullptr;
     const size_t nwarps = (size_t)gridDim.x * (blockDim.x >> 5);
-    for (size_t s0 = ((size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; s0 < g.nseg;
-         s0 += nwarps * 32) {
-        const size_t s    = s0 + lane;
-        const uint32_t cn = (s < g.nseg) ? g.seg_count[s] : 0u;
-        unsigned nz       = __ballot_sync(0xffffffffu, cn != 0u);
-        while (nz) {
-            const int k = __ffs(nz) - 1;
-            nz &= nz - 1;
-            const size_t sk = s0 + k;
-            const uint32_t n = __shfl_sync(0xffffffffu, cn, k);
-            copy_segment(g, out_bytes, sk, n, g.tile_base[sk / kGatherTile] + g.seg_off[sk]);
-        }
+    for (size_t s0 = ((size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; s0 < g.nseg; s0 += nwarps * 32)
+        copy_group(g, out_bytes, s0, g.nseg);
+}
+
+// Many fields: tasks of (field, kCopySegs segments), 32 of them to a warp.
+static_assert(kCopySegs == 8 * 32 && kGatherTile % kCopySegs == 0, "a CTA's warps take one group each");
+__global__ void __launch_bounds__(256)
+    k_outlier_copy_batch(const GatherArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks) {
+    for (uint32_t t = blockIdx.x; t < ntasks; t += gridDim.x) {
+        const BatchTask tk  = tasks[t];
+        const GatherArgs& g = args[tk.field];
+        if (*g.status != VSZ_OK || *g.total == 0) continue;  // set by earlier kernels only
+        const size_t s0 = tk.u0 + (threadIdx.x >> 5) * 32;
+        if (s0 < tk.u1) copy_group(g, g.out_bytes + g.out_off.eval(), s0, tk.u1);
     }
 }
 
@@ -875,6 +911,7 @@ int launch_eb_setup(int mode, double eb, const float* d_in, size_t n, Consts* d_
 // The most dynamic shared memory a dual-quant kernel takes: a shared histogram of up to 16384
 // bins and the 3D previous planes.  Every kernel is opted in to it once, so that a later launch
 // with a larger dictionary than the first still fits.
+constexpr int kDqFillWarps = 24;
 constexpr int kDqSmemMax = 16384 * 4 + 8 * (int)sizeof(PrevRows);
 
 template <int NDIM, int BS>
@@ -932,7 +969,18 @@ static int dispatch_bs(const DqArgs& a, int bs, bool vec, int grid, size_t smem,
     return VSZ_OK;
 }
 
+// Blocks are split along z until a launch has a unit for each of kDqFillWarps warps per SM.
+int dq_zlen_halvings(unsigned long long units, int bs, int num_sms) {
+    int h = 0;
+    while (units < (unsigned long long)num_sms * kDqFillWarps && (bs >> h) > 1) {
+        units *= 2;
+        h++;
+    }
+    return h;
+}
+
 int launch_dq_compress(DqArgs a, int ndim, int bs, cudaStream_t st, int num_sms) {
+    if (ndim == 3) dq_set_zlen(a, bs, dq_zlen_halvings(a.nunits, bs, num_sms));
     const bool vec = (a.d0 % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.x) & 15u) == 0) &&
                      ((reinterpret_cast<uintptr_t>(a.code) & 7u) == 0);
     if (a.nunits == 0) return VSZ_OK;
@@ -980,48 +1028,33 @@ int launch_consts_batch(const ConstsField* f, uint32_t nfields, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }
 
-int launch_dq_compress_batch(const DqArgs* args, const BatchTask* tasks, uint32_t ntasks, int ndim, int bs, bool vec,
-                             bool tail, uint32_t hist_words, uint32_t* next, cudaStream_t st, int num_sms) {
+int launch_dq_compress_batch(const DqArgs* args, const BatchTask* tasks, uint32_t ntasks, int bs, bool any3d,
+                             uint32_t hist_words, uint32_t* next, cudaStream_t st, int num_sms) {
     if (ntasks == 0) return VSZ_OK;
-    size_t smem = (size_t)hist_words * sizeof(uint32_t);
-    if (ndim == 3) smem += sizeof(PrevRows) * 8;
-    const uint32_t cap = (uint32_t)num_sms * (ndim == 1 ? 8u : 3u);
+    const size_t smem   = (size_t)hist_words * sizeof(uint32_t) + (any3d ? sizeof(PrevRows) * 8 : 0);
+    const uint32_t cap  = (uint32_t)num_sms * 3u;
     const uint32_t grid = ntasks < cap ? ntasks : cap;
-    int rc = VSZ_OK;
-    auto go23 = [&](auto kern, std::atomic<unsigned long long>& attr) {
-        smem_limit_once(kern, kDqSmemMax, attr);
+    static std::atomic<unsigned long long> attr[4];
+    auto go = [&](auto kern, std::atomic<unsigned long long>& at) {
+        smem_limit_once(kern, kDqSmemMax, at);
         kern<<<grid, 256, smem, st>>>(args, tasks, ntasks, hist_words, next);
     };
-    auto go1 = [&](auto kern, std::atomic<unsigned long long>& attr) {
-        smem_limit_once(kern, kDqSmemMax, attr);
-        kern<<<grid, 256, smem, st>>>(args, tasks, ntasks, next);
-    };
-    auto pick = [&](auto nd_c, auto bs_c) {
-        constexpr int ND = decltype(nd_c)::value, B = decltype(bs_c)::value;
-        static std::atomic<unsigned long long> attr[4];
-        if constexpr (ND == 1) {
-            if (vec) go1(k_dq_compress_1d_batch<B, true>, attr[0]);
-            else go1(k_dq_compress_1d_batch<B, false>, attr[1]);
-        } else {
-            if (vec && !tail) go23(k_dq_compress_23d_batch<ND, B, true, false>, attr[0]);
-            else if (vec) go23(k_dq_compress_23d_batch<ND, B, true, true>, attr[1]);
-            else if (!tail) go23(k_dq_compress_23d_batch<ND, B, false, false>, attr[2]);
-            else go23(k_dq_compress_23d_batch<ND, B, false, true>, attr[3]);
-        }
-    };
-    auto by_bs = [&](auto nd_c) {
-        switch (bs) {
-            case 8: pick(nd_c, std::integral_constant<int, 8>{}); break;
-            case 16: pick(nd_c, std::integral_constant<int, 16>{}); break;
-            case 32: pick(nd_c, std::integral_constant<int, 32>{}); break;
-            case 64: pick(nd_c, std::integral_constant<int, 64>{}); break;
-            default: rc = VSZ_ERR_UNSUPPORTED;
-        }
-    };
-    if (ndim == 1) by_bs(std::integral_constant<int, 1>{});
-    else if (ndim == 2) by_bs(std::integral_constant<int, 2>{});
-    else by_bs(std::integral_constant<int, 3>{});
-    if (rc) return rc;
+    switch (bs) {
+        case 8: go(k_dq_compress_batch<8>, attr[0]); break;
+        case 16: go(k_dq_compress_batch<16>, attr[1]); break;
+        case 32: go(k_dq_compress_batch<32>, attr[2]); break;
+        case 64: go(k_dq_compress_batch<64>, attr[3]); break;
+        default: return VSZ_ERR_UNSUPPORTED;
+    }
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
+}
+
+int launch_outlier_copy_batch(const GatherArgs* args, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st,
+                              int num_sms) {
+    if (ntasks == 0) return VSZ_OK;
+    const uint32_t cap = (uint32_t)num_sms * 8;
+    k_outlier_copy_batch<<<ntasks < cap ? ntasks : cap, 256, 0, st>>>(args, tasks, ntasks);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }

@@ -11,7 +11,6 @@
 #include <cstdint>
 #include <cstring>
 #include <map>
-#include <tuple>
 #include <vector>
 
 #include "api_common.cuh"
@@ -34,21 +33,19 @@ constexpr size_t kCtlInfo    = 80;   // u32[4] tree info
 constexpr size_t kCtlBits    = 96;   // u64 payload bits
 constexpr size_t kCtlNOut    = 104;  // u64 outliers
 constexpr size_t kCtlTicket  = 112;  // u32 gather look-back ticket
-// after the per-field records: the batch status, then one dual-quant task counter per class
-// (dimensionality x block size x aligned or not x tail or not: at most 48)
+// after the per-field records: the batch status, then one dual-quant task counter per block size
 constexpr size_t kDqNextOff  = 64;
-static_assert(kDqNextOff + 4 * 48 <= 256, "the counters fit the control tail");
 
-// Work per task (defaults; vsz_batch_autotune searches the first two): dual-quant warp units,
-// encoder chunks, min/max elements.
+// Work per task (vsz_batch_autotune searches the first two): dual-quant warp units and encoder chunks
+// (at most these many by default, fewer where the batch would not fill the GPU), min/max elements.
 constexpr uint64_t kDqUnitsPerTask  = 32;
 constexpr uint64_t kEncChunksPerTask = 64;
-constexpr uint64_t kMinmaxPerTask    = 1 << 20;
+constexpr uint64_t kMinmaxPerTask    = 1 << 15;
 constexpr uint64_t kGatherTileSegs   = 4096;  // k_outlier_gather's tile
 
-struct DqGroup {
-    int ndim, bs;
-    bool vec, tail;
+struct DqGroup {  // the fields of one block size
+    int bs;
+    bool any3d;
     uint32_t hist_words;
     uint32_t task_off, ntasks;
 };
@@ -75,13 +72,14 @@ struct vsz_batch {
     int build_dict_max = 0;
     uint32_t enc_off = 0, enc_n = 0;
     int cb_dict_max = 0;
-    uint32_t gather_off = 0, gather_n = 0;
+    uint32_t gather_off = 0, gather_n = 0, copy_off = 0, copy_n = 0;
     size_t total_chunks = 0;
     // task lists (own buffer, rebuilt by vsz_batch_set_task_sizes) and what they are built from
     BatchTask* d_tasks = nullptr;
     size_t tasks_cap   = 0;
-    uint64_t dq_per = 32, enc_per = 64;
-    std::vector<uint64_t> minmax_units, dq_units, enc_units, gather_units;  // per field
+    uint64_t dq_per = 0, enc_per = 0;  // 0: by the batch's size
+    std::vector<uint64_t> minmax_units, dq_units, enc_units, gather_units, copy_units;  // per field
+    std::vector<uint32_t> dq_class;
     std::vector<std::pair<DqGroup, std::vector<uint32_t>>> classes;
     // workspace regions zeroed per call
     uint8_t* ctl = nullptr;
@@ -123,6 +121,8 @@ struct BatchLayout {
     std::vector<uint8_t*> build_scratch;
     std::vector<unsigned long long*> edge_idx;
     std::vector<uint32_t*> edge_bits;
+    std::vector<uint32_t*> seg_off;               // gather: offsets of the segments in their tiles
+    std::vector<unsigned long long*> tile_base;   // and the tiles' first outliers
     std::vector<size_t> hist_off, gstat_off, chunk_base;
     size_t bytes;
 };
@@ -157,6 +157,8 @@ BatchLayout layout_batch(const std::vector<FieldGeom>& fg, uint8_t* base, size_t
                                                                      : b.take<uint8_t>(huff_build_scratch_bytes(f.p.dict_size)));
         L.edge_idx.push_back(b.take<unsigned long long>(2 * f.nch + 2));
         L.edge_bits.push_back(b.take<uint32_t>(2 * f.nch + 2));
+        L.seg_off.push_back(b.take<uint32_t>(f.g.nseg + 1));
+        L.tile_base.push_back(b.take<unsigned long long>(f.ntiles + 1));
     }
     L.bytes = b.off + 256;
     return L;
@@ -181,12 +183,13 @@ int field_geoms(const vsz_batch_field* fields, int nfields, std::vector<FieldGeo
     return VSZ_OK;
 }
 
-void add_tasks(std::vector<BatchTask>& t, uint32_t field, uint64_t units, uint64_t per) {
+void add_tasks(std::vector<BatchTask>& t, uint32_t field, uint64_t units, uint64_t per, uint32_t cls = 0) {
     for (uint64_t u = 0; u < units; u += per) {
         BatchTask k{};
         k.u0    = u;
         k.u1    = std::min(units, u + per);
         k.field = field;
+        k.pad   = cls;
         t.push_back(k);
     }
 }
@@ -213,19 +216,32 @@ int upload_tasks(vsz_batch* B) {
         if (B->minmax_units[f]) add_tasks(tasks, f, B->minmax_units[f], kMinmaxPerTask);
     B->minmax_n = (uint32_t)tasks.size();
     B->dq_groups.clear();
+    // default task sizes: a few tasks for each CTA the stage can hold, so that the last ones to finish
+    // leave little idle (8 units: one for each warp of the block)
+    auto per_task = [&](uint64_t set, uint64_t units, uint64_t ctas, uint64_t most) {
+        return set ? set : std::max<uint64_t>(8, std::min<uint64_t>(most, units / (4 * ctas) / 8 * 8));
+    };
+    const uint64_t sms = (uint64_t)num_sms();
     for (auto& kv : B->classes) {
         DqGroup grp  = kv.first;
         grp.task_off = (uint32_t)tasks.size();
-        for (uint32_t f : kv.second) add_tasks(tasks, f, B->dq_units[f], B->dq_per);
+        uint64_t units = 0;
+        for (uint32_t f : kv.second) units += B->dq_units[f];
+        const uint64_t per = per_task(B->dq_per, units, 3 * sms, kDqUnitsPerTask);
+        for (uint32_t f : kv.second) add_tasks(tasks, f, B->dq_units[f], per, B->dq_class[f]);
         grp.ntasks = (uint32_t)tasks.size() - grp.task_off;
         B->dq_groups.push_back(grp);
     }
     B->enc_off = (uint32_t)tasks.size();
-    for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, B->enc_units[f], B->enc_per);
+    const uint64_t enc_per = per_task(B->enc_per, B->total_chunks, 4 * sms, kEncChunksPerTask);
+    for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, B->enc_units[f], enc_per);
     B->enc_n      = (uint32_t)tasks.size() - B->enc_off;
     B->gather_off = (uint32_t)tasks.size();
     for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, B->gather_units[f], 1);
     B->gather_n = (uint32_t)tasks.size() - B->gather_off;
+    B->copy_off = (uint32_t)tasks.size();
+    for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, B->copy_units[f], kCopySegs);
+    B->copy_n = (uint32_t)tasks.size() - B->copy_off;
     if (tasks.size() > B->tasks_cap) {
         if (B->d_tasks) cudaFree(B->d_tasks);
         B->d_tasks   = nullptr;
@@ -346,6 +362,8 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
         g.tile_counter = ticket;
         g.status      = status;
         g.ntiles      = (uint32_t)G.ntiles;
+        g.seg_off     = L.seg_off[f];
+        g.tile_base   = L.tile_base[f];
 
         FinalizeArgs& fa = fin[f];
         fa               = FinalizeArgs{};
@@ -368,29 +386,36 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
         fa.chunk_bits    = he.chunk_bits;
         fa.n_chunks      = G.nch;
     }
-    // ---- what the task lists are built from
+    // ---- what the task lists are built from: fields by block size, 3D blocks split along z where the
+    // fields of one block size would not fill the GPU
+    std::map<int, std::vector<uint32_t>> classes;
+    for (uint32_t f = 0; f < nf; f++) classes[fg[f].p.block_size].push_back(f);
+    for (auto& kv : classes) {
+        unsigned long long units = 0;
+        for (uint32_t f : kv.second) units += dq[f].nunits;
+        const int halvings = dq_zlen_halvings(units, kv.first, num_sms());
+        for (uint32_t f : kv.second)
+            if (fg[f].g.ndim == 3) dq_set_zlen(dq[f], kv.first, halvings);
+    }
     for (uint32_t f = 0; f < nf; f++) {
+        const Geometry& g = fg[f].g;
+        const bool vec    = (g.d0 % 4 == 0) && ((reinterpret_cast<uintptr_t>(fields[f].d_in) & 15u) == 0);
+        B->dq_class.push_back(dq_class_of(g.ndim, vec, g.ndim >= 2 && (g.d0 % 8) != 0));
         B->minmax_units.push_back(fg[f].r2r ? fg[f].g.n : 0);
         B->dq_units.push_back(dq[f].nunits);
         B->enc_units.push_back(fg[f].nch);
         B->gather_units.push_back(fg[f].ntiles);
-    }
-    std::map<std::tuple<int, int, bool, bool>, std::vector<uint32_t>> classes;
-    for (uint32_t f = 0; f < nf; f++) {
-        const FieldGeom& G = fg[f];
-        const bool vec     = (G.g.d0 % 4 == 0) && ((reinterpret_cast<uintptr_t>(fields[f].d_in) & 15u) == 0);
-        const bool tail    = G.g.ndim >= 2 && (G.g.d0 % 8) != 0;
-        classes[std::make_tuple(G.g.ndim, G.p.block_size, vec, tail)].push_back(f);
+        B->copy_units.push_back(g.nseg);
     }
     for (auto& kv : classes) {
         DqGroup grp{};
-        std::tie(grp.ndim, grp.bs, grp.vec, grp.tail) = kv.first;
-        for (uint32_t f : kv.second)
+        grp.bs = kv.first;
+        for (uint32_t f : kv.second) {
             if (dq[f].smem_hist) grp.hist_words = std::max(grp.hist_words, (uint32_t)((dq[f].dict + 3) & ~3));
+            grp.any3d = grp.any3d || fg[f].g.ndim == 3;
+        }
         B->classes.emplace_back(grp, kv.second);
     }
-    B->dq_per  = kDqUnitsPerTask;
-    B->enc_per = kEncChunksPerTask;
     B->total_chunks = L.chunk_base.empty() ? 0 : L.chunk_base.back() + fg.back().nch;
     // ---- upload
     std::vector<HuffBuildArgs> build = build_smem;
@@ -480,7 +505,7 @@ vsz_status vsz_batch_autotune(vsz_batch* B, int iterations, int* best_dq_units, 
     // coordinate search: dual-quant task size first, then the encoder's
     static const uint64_t kDq[]  = {8, 16, 32, 64, 128};
     static const uint64_t kEnc[] = {16, 32, 64, 128, 256};
-    uint64_t bdq = B->dq_per, benc = B->enc_per;
+    uint64_t bdq = B->dq_per ? B->dq_per : kDqUnitsPerTask, benc = B->enc_per ? B->enc_per : kEncChunksPerTask;
     float best = 3.4e38f, ms = 0.f;
     int rc = VSZ_OK;
     for (uint64_t dq : kDq) {
@@ -529,8 +554,8 @@ vsz_status vsz_batch_compress(vsz_batch* B, void* stream) {
         uint32_t* next = reinterpret_cast<uint32_t*>(B->ctl + (size_t)nf * kCtlBytes + kDqNextOff);
         for (size_t i = 0; i < B->dq_groups.size(); i++) {
             const DqGroup& g = B->dq_groups[i];
-            VSZ_TRY(launch_dq_compress_batch(B->dq, B->tasks + g.task_off, g.ntasks, g.ndim, g.bs, g.vec, g.tail,
-                                             g.hist_words, next + i, st, sms));
+            VSZ_TRY(launch_dq_compress_batch(B->dq, B->tasks + g.task_off, g.ntasks, g.bs, g.any3d, g.hist_words,
+                                             next + i, st, sms));
         }
     }
     {
@@ -545,6 +570,7 @@ vsz_status vsz_batch_compress(vsz_batch* B, void* stream) {
     {
         StageTimer t(kStOutlierGather, st);
         VSZ_TRY(launch_outlier_gather_batch(B->gather, B->tasks + B->gather_off, B->gather_n, st, sms));
+        VSZ_TRY(launch_outlier_copy_batch(B->gather, B->tasks + B->copy_off, B->copy_n, st, sms));
     }
     {
         StageTimer t(kStFinalize, st);

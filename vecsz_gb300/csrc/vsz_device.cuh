@@ -73,6 +73,34 @@ __device__ __forceinline__ float prequant_scalar(float x, double r_d) {
     return __double2float_rn(round(__dmul_rn((double)x, r_d)));
 }
 
+// The same value without FP64 where that is certain.  GB300 issues a warp's double multiply in 16
+// cycles per SM, and a row's tail columns took a handful each: that alone was 70 of the 98 us of a
+// 333x241x187 dual-quant.  With r_d = r_hi + r_lo (+ less than 2^-48 of it), x * r_d is p + t + less
+// than 2^-23 for |p| < 2^22: p = RN32(x r_hi), t = RN32(x r_lo + (x r_hi - p)).  So the nearest
+// integer of RN64(x * r_d) is rint(p) moved by d = (p - rint(p)) + t, unless d is within 2^-16 of a
+// half: those, larger values and unusable splits (`split` = 0) take the double operations.
+__device__ __forceinline__ float prequant_scalar(float x, float r_hi, float r_lo, bool split, double r_d) {
+    const float p  = __fmul_rn(x, r_hi);
+    const float t  = __fmaf_rn(x, r_lo, __fmaf_rn(x, r_hi, -p));
+    const float q  = rintf(p);
+    const float d  = __fadd_rn(__fsub_rn(p, q), t);
+    const float ad = fabsf(d);
+    if (split && fabsf(p) < 4194304.0f && fabsf(__fsub_rn(ad, 0.5f)) > 1.52587890625e-5f)
+        return copysignf(ad > 0.5f ? __fadd_rn(q, copysignf(1.0f, d)) : q, x);  // round(-0.3) is -0
+    return prequant_scalar(x, r_d);
+}
+
+// Multiplier of prequant_scalar above, from r_d: valid while both parts are far from the ends of
+// the FP32 range.
+struct ScalarMul {
+    double r_d;
+    float r_lo;
+    bool split;
+};
+__device__ __forceinline__ ScalarMul scalar_mul(double r_d, float r_hi) {
+    return ScalarMul{r_d, __double2float_rn(__dsub_rn(r_d, (double)r_hi)), r_hi > 1e-18f && r_hi < 1e30f};
+}
+
 // ------------------------------------------------------------------------------------------
 // Dequantization: (float)((double)s * c_d)   (src/dualquant.hh:941,980,1038)
 //

@@ -72,7 +72,7 @@ __device__ __forceinline__ Halo halo_of(const PadView& p, int ndim, uint32_t bx,
 struct BatchTask {
     unsigned long long u0, u1;
     uint32_t field;
-    uint32_t pad;
+    uint32_t pad;  // dual-quant tasks: the field's kernel class
 };
 
 struct MinmaxField {
@@ -100,7 +100,8 @@ struct DqArgs {
     uint32_t d0, d1, d2;
     uint32_t nxt;                // 128-wide x tiles per row
     uint32_t nyg;                // groups of 8 rows
-    uint32_t nzb;                // Lorenzo blocks along z (3D) or 1
+    uint32_t nzb;                // units along z (3D): slabs of zlen planes; or 1
+    uint32_t zlen;               // 3D: planes per unit, the block size or that halved (dq_set_zlen)
     uint32_t xtail;              // first tail column: d0 & ~7 when d0 % 8 != 0, else d0
     int R;                       // radius = dict / 2
     int dict;
@@ -231,6 +232,14 @@ int launch_dq_compress_f64(F64Args a, int ndim, cudaStream_t st, int num_sms);
 int launch_gather_f64(F64Args a, const unsigned long long* seg_off, DevOffset out_off, cudaStream_t st, int num_sms);
 int launch_dq_decompress_f64(F64Args a, int ndim, const unsigned long long* seg_off, cudaStream_t st);
 
+// Planes per 3D unit: block_size halved `halvings` times (and nzb, nunits for it).  dq_zlen_halvings:
+// for a launch whose units number `units` at whole blocks.
+inline void dq_set_zlen(DqArgs& a, int bs, int halvings) {
+    a.zlen   = (uint32_t)bs >> halvings;
+    a.nzb    = (a.d2 + a.zlen - 1) / a.zlen;
+    a.nunits = (unsigned long long)a.nxt * a.nyg * a.nzb;
+}
+int dq_zlen_halvings(unsigned long long units, int bs, int num_sms);
 int launch_eb_setup(int mode, double eb, const float* d_in, size_t n, Consts* d_consts, uint32_t* d_mm,
                     cudaStream_t st, int* status_word = nullptr);
 int launch_dq_compress(DqArgs a, int ndim, int bs, cudaStream_t st, int num_sms);
@@ -253,16 +262,21 @@ size_t pad_ws_bytes();
 size_t pad_count(int ndim, const uint32_t d[3], int bs, int mode);
 int launch_pad_values(const PadArgs& a, cudaStream_t st, int num_sms);
 
-// Batched launchers (device arrays of per-field arguments and of tasks).  A dual-quant batch
-// holds fields of one kernel class: ndim, block size, vec (d0 % 4 == 0 and aligned), tail
-// (d0 % 8 != 0); hist_words = shared-memory histogram words (0 when no field uses one); next =
-// the launch's task counter (zero on entry), through which free blocks take tasks.
+// Batched launchers (device arrays of per-field arguments and of tasks).  A dual-quant launch
+// holds the fields of one block size; a task's pad word is its field's kernel class (dq_class_of).
+// hist_words = shared-memory histogram words (0 when no field uses one); any3d: some field is 3D;
+// next = the launch's task counter (zero on entry), through which free blocks take tasks.
+inline uint32_t dq_class_of(int ndim, bool vec, bool tail) { return (uint32_t)ndim * 4u + (vec ? 2u : 0u) + (tail ? 1u : 0u); }
 int launch_minmax_batch(const MinmaxField* f, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st, int num_sms);
 int launch_consts_batch(const ConstsField* f, uint32_t nfields, cudaStream_t st);
-int launch_dq_compress_batch(const DqArgs* args, const BatchTask* tasks, uint32_t ntasks, int ndim, int bs, bool vec,
-                             bool tail, uint32_t hist_words, uint32_t* next, cudaStream_t st, int num_sms);
+int launch_dq_compress_batch(const DqArgs* args, const BatchTask* tasks, uint32_t ntasks, int bs, bool any3d,
+                             uint32_t hist_words, uint32_t* next, cudaStream_t st, int num_sms);
 int launch_outlier_gather_batch(const GatherArgs* args, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st,
                                 int num_sms);
+// ... then the values, by tasks of (field, segment range) (kCopySegs segments a CTA).
+constexpr unsigned kCopySegs = 256;
+int launch_outlier_copy_batch(const GatherArgs* args, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st,
+                              int num_sms);
 size_t gather_tmp_bytes(size_t nseg);
 int set_spin_limit_dq(long long polls);  // test hook: this unit's look-back spin limit
 
