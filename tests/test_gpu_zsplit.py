@@ -77,3 +77,11 @@ def test_tail_columns_near_halves(cuda, eb):
     x[2::197] = 3e38
     x = np.where(np.isfinite(x), x, np.float32(1.0)).astype(np.float32)
     check(cuda, x, dims, 8, eb)
+
+
+@pytest.mark.parametrize("d0", [1, 3, 7, 8, 9, 16, 23, 31, 33, 40, 50, 56, 60, 63, 64, 65])
+@pytest.mark.parametrize("rest", [(1,), (7,), (50,), (9, 3), (37, 17)])
+def test_narrow_rows(cuda, d0, rest):
+    """Rows of at most 64 columns: several groups of 8 rows to a warp."""
+    dims = (d0,) + rest
+    check(cuda, smooth(dims, d0, 0.02) if len(dims) == 3 else smooth(dims + (1,), d0, 0.02), dims, 8)

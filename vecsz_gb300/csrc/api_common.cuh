@@ -102,6 +102,8 @@ inline DqArgs make_dq_args(const Geometry& g, int bs, int dict, const float* x, 
     a.d2 = g.d2;
     a.nxt = g.nxt;
     a.nyg = (g.d1 + 7) / 8;
+    a.lpr = 32;
+    a.grp = 1;
     a.nzb = (g.ndim == 3) ? (g.d2 + bs - 1) / bs : 1;
     a.zlen = (g.ndim == 3) ? (uint32_t)bs : 1u;
     a.xtail = (g.d0 % 8) ? (g.d0 & ~7u) : g.d0;

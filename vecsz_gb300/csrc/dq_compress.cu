@@ -167,26 +167,33 @@ struct HistAcc {
     }
 };
 
-// One row of 4 elements per lane: store codes, count histogram, rank and write outliers.
+// Columns [xb, xb + 4) of a lane in a row: n of them lie in the row.  FULL: all four in every lane
+// (whole tiles); VEC (rows of 16-byte multiples): all four or none.
+template <bool VEC, bool FULL>
+__device__ __forceinline__ bool col_in(uint32_t n, int j) {
+    return FULL || (VEC ? n != 0u : (uint32_t)j < n);
+}
+__device__ __forceinline__ uint32_t cols_of(uint32_t xb, uint32_t d0) { return xb >= d0 ? 0u : min(4u, d0 - xb); }
+
+// One row of 4 elements per lane: store codes, count histogram, rank and write outliers.  x, crow:
+// the lane's first column; seg: the row segment.  gmask: the lanes of this lane's row, lead: it is the
+// first of them.  Rows outside the field have n = 0.
 template <bool VEC, bool FULL = false>
-__device__ __forceinline__ void emit_row(const DqArgs& a, size_t row, uint32_t xb, uint32_t xt, bool row_in,
-                                         const int code[4], const float outv[4], HistAcc& h, uint32_t* s_hist) {
-    const unsigned lane = lane_id();
-    if (FULL) row_in = true;
+__device__ __forceinline__ void emit_row(const DqArgs& a, const float* x, uint16_t* crow, size_t seg, uint32_t n,
+                                         const int code[4], const float outv[4], HistAcc& h, uint32_t* s_hist,
+                                         unsigned gmask, bool lead) {
     bool in[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) in[j] = FULL || (row_in && (xb + j < a.d0));
-    uint16_t* crow = a.code + row * a.d0;
+    for (int j = 0; j < 4; j++) in[j] = col_in<VEC, FULL>(n, j);
     if (VEC && in[0]) {
-        // d0 % 4 == 0: all four columns are in range together; 8-byte aligned store.
         uint2 v;
         v.x = (uint32_t)code[0] | ((uint32_t)code[1] << 16);
         v.y = (uint32_t)code[2] | ((uint32_t)code[3] << 16);
-        *reinterpret_cast<uint2*>(crow + xb) = v;
+        *reinterpret_cast<uint2*>(crow) = v;
     } else {
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (in[j]) crow[xb + j] = (uint16_t)code[j];
+            if (in[j]) crow[j] = (uint16_t)code[j];
     }
     if (s_hist) {
         // predicated, not branched: the zero-residual code counts in a register, the others in the
@@ -207,35 +214,29 @@ __device__ __forceinline__ void emit_row(const DqArgs& a, size_t row, uint32_t x
     bool o[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) o[j] = in[j] && code[j] == 0;
-    const size_t seg = row * a.nxt + xt;
     if (!__any_sync(0xffffffffu, o[0] | o[1] | o[2] | o[3])) {
-        if (row_in && lane == 0) a.seg_count[seg] = 0;
+        if (lead && (FULL || n)) a.seg_count[seg] = 0;
         return;
     }
     unsigned m[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) m[j] = __ballot_sync(0xffffffffu, o[j]);
-    if (!row_in) return;
+    for (int j = 0; j < 4; j++) m[j] = __ballot_sync(0xffffffffu, o[j]) & gmask;
     const unsigned lt = lanemask_lt();
-    unsigned before   = __popc(m[0] & lt) + __popc(m[1] & lt) + __popc(m[2] & lt) + __popc(m[3] & lt);
-    unsigned total    = __popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]);
-    if (lane == 0) a.seg_count[seg] = (uint8_t)total;
-    if (total) {
-        float* dst = a.scratch + seg * kSegX;
-        unsigned r = before;
+    unsigned r        = __popc(m[0] & lt) + __popc(m[1] & lt) + __popc(m[2] & lt) + __popc(m[3] & lt);
+    if (lead && (FULL || n)) a.seg_count[seg] = (uint8_t)(__popc(m[0]) + __popc(m[1]) + __popc(m[2]) + __popc(m[3]));
+    float* dst = a.scratch + seg * kSegX;
 #pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (o[j]) {
-                float v = outv[j];
-                // a NaN input's prequantized value is that NaN, quieted (the GPU multiply would
-                // give its canonical NaN); strict outliers are input values already
-                if (v != v && !a.strict) {
-                    const float xv = a.x[row * a.d0 + xb + j];
-                    if (xv != xv) v = quiet_nan(xv);
-                }
-                dst[r++] = v;
+    for (int j = 0; j < 4; j++)
+        if (o[j]) {
+            float v = outv[j];
+            // a NaN input's prequantized value is that NaN, quieted (the GPU multiply would
+            // give its canonical NaN); strict outliers are input values already
+            if (v != v && !a.strict) {
+                const float xv = x[j];
+                if (xv != xv) v = quiet_nan(xv);
             }
-    }
+            dst[r++] = v;
+        }
 }
 
 // (int)(e + R) for an integer-valued residual with |e| < R <= 32768: e + R + 1.5 * 2^23 is exact
@@ -245,38 +246,33 @@ __device__ __forceinline__ int code_of(float e, float rmagic) {
     return __float_as_int(__fadd_rn(e, rmagic)) - 0x4B400000;
 }
 
-template <int NDIM, bool TAIL>
-__device__ __forceinline__ float prequant_at(float v, uint32_t col, uint32_t xtail, float r_f, const ScalarMul& sm) {
-    if (NDIM == 3 && TAIL && col >= xtail) return prequant_scalar(v, r_f, sm.r_lo, sm.split, sm.r_d);
-    return prequant_vec(v, r_f);
-}
-
-// Raw values of 4 consecutive columns [xb, xb+4) of one row (zeros outside the field).
+// Raw values of a lane's 4 columns from p on (zeros outside the row).
 template <bool VEC, bool FULL = false>
-__device__ __forceinline__ float4 load_raw(const DqArgs& a, size_t row, bool row_in, uint32_t xb) {
+__device__ __forceinline__ float4 load_raw(const float* p, uint32_t n) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (!FULL && !row_in) return v;
-    const float* rowp = a.x + row * a.d0;
     if (VEC) {
-        if (FULL || xb < a.d0) v = __ldcs(reinterpret_cast<const float4*>(rowp + xb));
+        if (FULL || n) v = __ldcs(reinterpret_cast<const float4*>(p));
     } else {
-        if (xb < a.d0) v.x = __ldcs(rowp + xb);
-        if (xb + 1 < a.d0) v.y = __ldcs(rowp + xb + 1);
-        if (xb + 2 < a.d0) v.z = __ldcs(rowp + xb + 2);
-        if (xb + 3 < a.d0) v.w = __ldcs(rowp + xb + 3);
+        if (col_in<false, FULL>(n, 0)) v.x = __ldcs(p);
+        if (col_in<false, FULL>(n, 1)) v.y = __ldcs(p + 1);
+        if (col_in<false, FULL>(n, 2)) v.z = __ldcs(p + 2);
+        if (col_in<false, FULL>(n, 3)) v.w = __ldcs(p + 3);
     }
     return v;
 }
 
-// Prequantized values of a raw row; zero outside the field.
-template <int NDIM, bool TAIL, bool FULL = false>
-__device__ __forceinline__ void prequant_row(const DqArgs& a, float4 v, bool row_in, uint32_t xb, float r_f, const ScalarMul& sm,
-                                             float S[4]) {
+// Prequantized values of a raw row.  Cells outside the field need no care: their values only ever
+// feed other cells outside it.  scalar: the lane's columns are 3D tail columns (all or none of a
+// lane's are: tails start at multiples of 8).
+template <bool TAIL>
+__device__ __forceinline__ void prequant_row(float4 v, bool scalar, float r_f, const ScalarMul& sm, float S[4]) {
     const float t[4] = {v.x, v.y, v.z, v.w};
+    if (TAIL && scalar) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const bool in = FULL || (row_in && (xb + j < a.d0));
-        S[j]          = in ? prequant_at<NDIM, TAIL>(t[j], xb + j, a.xtail, r_f, sm) : 0.0f;
+        for (int j = 0; j < 4; j++) S[j] = prequant_scalar(t[j], r_f, sm.r_lo, sm.split, sm.r_d);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) S[j] = prequant_vec(t[j], r_f);
     }
 }
 
@@ -284,7 +280,9 @@ __device__ __forceinline__ void prequant_row(const DqArgs& a, float4 v, bool row
 // (z) of one Lorenzo block.  A field with fewer units than the GPU holds warps is bound by a unit's
 // chain of rows (64^3: 64 units of 64 rows, 38 us), so its blocks are split along z (dq_set_zlen): a
 // unit that does not start its block first prequantizes the plane before it, which costs 1 / zlen
-// of the loads and prequantizations again.  Rows are processed one at a time (the next row's values are
+// of the loads and prequantizations again.  Rows of at most 64 columns would leave most lanes idle
+// (23 columns: 82 %), so a warp takes a.grp groups of 8 of them (dq_set_narrow), a.lpr lanes each.
+// Rows are processed one at a time (the next row's values are
 // loaded while the current one is coded); a lane keeps in registers only its 4 values of the
 // current row and of the row above, in this plane and in the previous one.  The previous plane's
 // 8 rows live in shared memory [row][column][lane] (conflict-free), each row overwritten by the
@@ -318,7 +316,8 @@ __device__ __forceinline__ void hist_flush_block(const DqArgs& a, uint32_t* s_hi
 
 // Warp units u0, u0 + ustep, ... < u1 of one field.  STRICT: the strict error-bound mode (see
 // strict_keep).  PAD: padding (-p), the halo of each block from a.pad instead of zeros.
-template <int NDIM, int BS, bool VEC, bool TAIL, bool STRICT = false, bool PAD = false>
+// NARROW: a.grp row groups to a warp.
+template <int NDIM, int BS, bool VEC, bool TAIL, bool STRICT = false, bool PAD = false, bool NARROW = false>
 __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, unsigned long long u0,
                                            unsigned long long u1, unsigned long long ustep, uint32_t* s_hist,
                                            PrevRows* s_prev, HistAcc& h) {
@@ -328,8 +327,9 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
     const float rmagic  = Rf + 12582912.0f;
     const unsigned lane = lane_id();
     const unsigned wib  = threadIdx.x >> 5;
-    const bool xbound   = ((lane * 4) % BS) == 0;  // my first column starts a Lorenzo block
-    auto left = [&](float v, float halo) {         // x - 1 neighbour of my first column
+    const uint32_t gi   = NARROW ? lane / a.lpr : 0u, lx = NARROW ? lane % a.lpr : lane;  // my row group, lane in it
+    const bool xbound   = ((lx * 4) % BS) == 0;  // my first column starts a Lorenzo block
+    auto left = [&](float v, float halo) {       // x - 1 neighbour of my first column
         const float t = __shfl_up_sync(0xffffffffu, v, 1);
         return xbound ? halo : t;
     };
@@ -338,17 +338,31 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
         const uint32_t xt = u % a.nxt;
         const uint32_t r = u / a.nxt;
         const uint32_t yg = r % a.nyg;
-        const uint32_t xb = xt * kTileX + lane * 4;
-        const uint32_t y0 = yg * 8;
+        const uint32_t xb = xt * kTileX + lx * 4;
+        const uint32_t y0 = NARROW ? (yg * a.grp + gi) * 8 : yg * 8;
         const bool yhalo  = (BS > 8) && (y0 % BS) != 0;  // the row above is inside the block
         const uint32_t z0 = (NDIM == 3) ? (r / a.nyg) * a.zlen : 0;
         const int nz      = (NDIM == 3) ? (int)min(a.zlen, a.d2 - z0) : 1;
         const bool zin    = NDIM == 3 && (z0 % BS) != 0;  // the plane before is inside the block
 
+        const uint32_t nc  = (NARROW && gi >= a.grp) ? 0u : cols_of(xb, a.d0);
+        const bool lane_tl = TAIL && xb >= a.xtail;  // my columns are tail columns
         // a tile wholly inside the field (the common case) runs without per-element range checks
-        const bool full = VEC && (xt + 1) * kTileX <= a.d0 && y0 + 8 <= a.d1;
+        const bool full    = (xt + 1) * kTileX <= a.d0 && y0 + 8 <= a.d1;
         auto unit_body = [&](auto full_c) {
             constexpr bool FULL = decltype(full_c)::value;
+            // rows of my group, and of the warp's first one (the others have no more)
+            const int nyl = FULL ? 8 : (y0 < a.d1 ? (int)min(8u, a.d1 - y0) : 0);
+            const int ny  = FULL ? 8 : (NARROW ? (int)min(8u, a.d1 - yg * a.grp * 8) : nyl);
+            auto cols     = [&](int i) { return NARROW && i >= nyl ? 0u : nc; };  // my columns in row i
+            // my columns of row i of plane z (row and element indices are computed where they are used:
+            // kept as running pointers they spill)
+            auto row_of   = [&](uint32_t z, int i) { return (size_t)z * a.d1 + (y0 + i); };
+            auto load     = [&](uint32_t z, int i) {
+                return load_raw<VEC, FULL>(a.x + row_of(z, i) * a.d0 + xb, cols(max(i, 0)));
+            };
+            const unsigned gmask = NARROW ? ((1u << a.lpr) - 1u) << (gi * a.lpr) : 0xffffffffu;
+            auto prequant = [&](float4 v, float S[4]) { prequant_row<TAIL && NDIM == 3>(v, lane_tl, r_f, sm, S); };
             // halo values of my block: x-, y- and z-halo cells (zero without padding; lanes past the
             // field read none); hxy: the (x-1, y-1) neighbour of my first column when the row above is
             // the halo row -- the corner cell at a block start (2D: x-halo, 3D: y-halo), else a y-halo
@@ -361,17 +375,15 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
                 hz = hv.z;
             }
             const float hxy = (xbound && NDIM == 2) ? hx : hy;
-
             float Ph[4] = {hz, hz, hz, hz}, PhL = hz;  // previous plane's halo row (y0 - 1)
             if (NDIM == 3 && zin) {
-                const size_t rp = (size_t)(z0 - 1) * a.d1 + y0;
                 float4 raw[8];
 #pragma unroll
-                for (int i = 0; i < 8; i++) raw[i] = load_raw<VEC, FULL>(a, rp + i, y0 + i < a.d1, xb);
+                for (int i = 0; i < 8; i++) raw[i] = i < ny ? load(z0 - 1, i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     float S[4];
-                    prequant_row<NDIM, TAIL, FULL>(a, raw[i], y0 + i < a.d1, xb, r_f, sm, S);
+                    prequant(raw[i], S);
 #pragma unroll
                     for (int j = 0; j < 4; j++) s_prev[wib][i][j][lane] = S[j];
                 }
@@ -379,36 +391,31 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
                 for (int j = 0; j < 4; j++) Ph[j] = hy;
                 PhL = hxy;
                 if (yhalo) {
-                    prequant_row<NDIM, TAIL, FULL>(a, load_raw<VEC, FULL>(a, rp - 1, true, xb), true, xb, r_f, sm, Ph);
+                    prequant(load(z0 - 1, -1), Ph);
                     PhL = left(Ph[3], hx);
                 }
             }
-            float4 nxt = load_raw<VEC, FULL>(a, (size_t)z0 * a.d1 + y0, y0 < a.d1, xb);
+            float4 nxt = load(z0, 0);
             for (int zz = 0; zz < nz; zz++) {
                 const uint32_t z = z0 + zz;
                 const bool zp    = zin || zz > 0;  // a previous plane inside the block
                 float Sp[4] = {hy, hy, hy, hy}, SpL = hxy;  // row above, this plane (halo row at i = 0)
                 if (yhalo) {
-                    prequant_row<NDIM, TAIL, FULL>(a, load_raw<VEC, FULL>(a, (size_t)z * a.d1 + (y0 - 1), true, xb), true, xb, r_f,
-                                             sm, Sp);
+                    prequant(load(z, -1), Sp);
                     SpL = left(Sp[3], hx);
                 }
                 const float ShNext[4] = {Sp[0], Sp[1], Sp[2], Sp[3]};
                 const float ShNextL   = SpL;
                 float Pp[4] = {Ph[0], Ph[1], Ph[2], Ph[3]}, PpL = PhL;  // row above, previous plane
-#pragma unroll 2
-                for (int i = 0; i < 8; i++) {
-                    const uint32_t y  = y0 + i;
-                    const bool row_in = y < a.d1;
-                    const float4 raw  = nxt;
-                    {  // the next row of this plane, or the first row of the next plane
-                        const bool last_row = (i == 7);
-                        const uint32_t zn = last_row ? z + 1 : z, yn = last_row ? y0 : y + 1;
-                        const bool more = !last_row || zz + 1 < nz;
-                        nxt = more ? load_raw<VEC, FULL>(a, (size_t)zn * a.d1 + yn, yn < a.d1, xb) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
+                constexpr int kUnroll = FULL && VEC ? 2 : 1;
+#pragma unroll kUnroll
+                for (int i = 0; i < ny; i++) {
+                    const float4 raw = nxt;
+                    // the next row of this plane, or the first row of the next plane
+                    const bool last_row = i + 1 == ny, more = !last_row || zz + 1 < nz;
+                    nxt = more ? load(last_row ? z + 1 : z, last_row ? 0 : i + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
                     float S[4];
-                    prequant_row<NDIM, TAIL, FULL>(a, raw, row_in, xb, r_f, sm, S);
+                    prequant(raw, S);
                     const float SL = left(S[3], hx);
                     float Pc[4] = {hz, hz, hz, hz}, PcL = hz;  // this row, previous plane
                     if (NDIM == 3) {
@@ -418,23 +425,22 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
                     }
                     int code[4];
                     float outv[4];
+                    auto residuals = [&](auto tail_c) {
+                        constexpr bool TL = decltype(tail_c)::value;
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const uint32_t col = xb + j;
-                        const float cur    = S[j];
-                        const float X      = j ? S[j - 1] : SL;
-                        const float Y      = Sp[j];
-                        const float XY     = j ? Sp[j - 1] : SpL;
-                        const bool tail    = TAIL && col >= a.xtail;
-                        float pred;
-                        if (NDIM == 2) {
-                            pred = __fadd_rn(X, __fsub_rn(Y, XY));  // W + (N - NW)
-                        } else {
+                        for (int j = 0; j < 4; j++) {
+                            const float cur = S[j];
+                            const float X   = j ? S[j - 1] : SL;
+                            const float Y   = Sp[j];
+                            const float XY  = j ? Sp[j - 1] : SpL;
                             const float Z   = Pc[j];
                             const float XZ  = j ? Pc[j - 1] : PcL;
                             const float YZ  = Pp[j];
                             const float XYZ = j ? Pp[j - 1] : PpL;
-                            if (!tail) {
+                            float pred;
+                            if (NDIM == 2) {
+                                pred = __fadd_rn(X, __fsub_rn(Y, XY));  // W + (N - NW)
+                            } else if (!TL) {
                                 float dist1 = __fadd_rn(X, __fadd_rn(Y, Z));
                                 float dist2 = __fadd_rn(XY, __fadd_rn(XZ, YZ));
                                 pred        = __fadd_rn(__fsub_rn(XYZ, dist2), dist1);
@@ -442,34 +448,32 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
                                 pred = __fadd_rn(__fadd_rn(__fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(XYZ, XY), XZ), YZ), X), Y),
                                                  Z);
                             }
-                        }
-                        const float e = __fsub_rn(cur, pred);
-                        const bool q  = fabsf(e) < Rf;
-                        code[j]       = q ? code_of(e, rmagic) : 0;
-                        outv[j]       = cur;
-                        if (STRICT) {
-                            const float xr = j == 0 ? raw.x : (j == 1 ? raw.y : (j == 2 ? raw.z : raw.w));
-                            float pd;  // the decompressor's prediction from the same (in-step) neighbours
-                            if (NDIM == 2) {
-                                pd = __fsub_rn(__fadd_rn(Y, X), XY);
-                            } else {
-                                const float Z   = Pc[j];
-                                const float XZ  = j ? Pc[j - 1] : PcL;
-                                const float YZ  = Pp[j];
-                                const float XYZ = j ? Pp[j - 1] : PpL;
-                                pd = __fadd_rn(__fadd_rn(__fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(XYZ, XY), XZ), YZ), X), Y), Z);
+                            const float e = __fsub_rn(cur, pred);
+                            const bool q  = fabsf(e) < Rf;
+                            code[j]       = q ? code_of(e, rmagic) : 0;
+                            outv[j]       = cur;
+                            if (STRICT) {
+                                const float xv = j == 0 ? raw.x : (j == 1 ? raw.y : (j == 2 ? raw.z : raw.w));
+                                // the decompressor's prediction from the same (in-step) neighbours
+                                const float pd =
+                                    NDIM == 2 ? __fsub_rn(__fadd_rn(Y, X), XY)
+                                              : __fadd_rn(__fadd_rn(__fadd_rn(__fsub_rn(__fsub_rn(__fsub_rn(XYZ, XY), XZ), YZ), X), Y), Z);
+                                if (!strict_keep(q, pd, e, cur, xv, c)) code[j] = 0;
+                                outv[j] = xv;  // strict outliers carry the input value
+                            } else if (NDIM == 2 && TL) {
+                                code[j] = 0;
+                                outv[j] = 0.0f;
                             }
-                            if (!strict_keep(q, pd, e, cur, xr, c)) code[j] = 0;
-                            outv[j] = xr;  // strict outliers carry the input value
-                        } else if (NDIM == 2 && tail) {
-                            code[j] = 0;
-                            outv[j] = 0.0f;
                         }
-                    }
-                    emit_row<VEC, FULL>(a, (size_t)z * a.d1 + y, xb, xt, row_in, code, outv, h, s_hist);
+                    };
+                    if (TAIL && lane_tl) residuals(std::true_type{});
+                    else residuals(std::false_type{});
+                    const size_t row = row_of(z, i), off = row * a.d0 + xb;
+                    emit_row<VEC, FULL>(a, a.x + off, a.code + off, row * a.nxt + xt, cols(i), code, outv, h, s_hist,
+                                        gmask, lx == 0);
                     if (NDIM == 3) {
 #pragma unroll
-                        for (int j = 0; j < 4; j++) s_prev[wib][i][j][lane] = S[j];  // row i of plane z
+                        for (int j = 0; j < 4; j++) s_prev[wib][i][j][lane] = S[j];  // row i of this plane
                     }
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
@@ -484,12 +488,12 @@ __device__ __forceinline__ void dq23_units(const DqArgs& a, const Consts& c, uns
                 PhL = ShNextL;
             }
         };
-        if (full) unit_body(std::true_type{});
+        if (!NARROW && full) unit_body(std::integral_constant<bool, !NARROW>{});
         else unit_body(std::false_type{});
     }
 }
 
-template <int NDIM, int BS, bool VEC, bool TAIL, bool STRICT = false, bool PAD = false>
+template <int NDIM, int BS, bool VEC, bool TAIL, bool STRICT = false, bool PAD = false, bool NARROW = false>
 __global__ void __launch_bounds__(256, 4) k_dq_compress_23d(DqArgs a) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
     uint32_t* s_hist = a.smem_hist ? s_dyn : nullptr;
@@ -503,7 +507,7 @@ __global__ void __launch_bounds__(256, 4) k_dq_compress_23d(DqArgs a) {
     const unsigned long long warps_total = (unsigned long long)gridDim.x * (blockDim.x >> 5);
     const unsigned long long warp0       = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     HistAcc h;
-    dq23_units<NDIM, BS, VEC, TAIL, STRICT, PAD>(a, c, warp0, a.nunits, warps_total, s_hist, s_prev, h);
+    dq23_units<NDIM, BS, VEC, TAIL, STRICT, PAD, NARROW>(a, c, warp0, a.nunits, warps_total, s_hist, s_prev, h);
     hist_flush_block(a, s_hist, h);
 }
 
@@ -533,9 +537,9 @@ __device__ __forceinline__ void dq1d_units(const DqArgs& a, const Consts& c, uns
         for (int t = 0; t < U; t++) {
             const uint32_t xt = (uint32_t)(u * U + t);
             const uint32_t xb = xt * kTileX + lane * 4;
-            const float4 rw   = load_raw<VEC>(a, 0, xt < a.nxt, xb);
+            const float4 rw   = load_raw<VEC>(a.x + xb, cols_of(xb, a.d0));
             if (STRICT) RW[STRICT ? t : 0] = rw;
-            prequant_row<1, false>(a, rw, xt < a.nxt, xb, r_f, ScalarMul{}, S[t]);
+            prequant_row<false>(rw, false, r_f, ScalarMul{}, S[t]);
         }
 #pragma unroll
         for (int t = 0; t < U; t++) {
@@ -577,7 +581,7 @@ __device__ __forceinline__ void dq1d_units(const DqArgs& a, const Consts& c, uns
                     outv[j] = xr;
                 }
             }
-            emit_row<VEC>(a, 0, xb, xt, xt < a.nxt, code, outv, h, s_hist);
+            emit_row<VEC>(a, a.x + xb, a.code + xb, xt, cols_of(xb, a.d0), code, outv, h, s_hist, 0xffffffffu, lane == 0);
         }
     }
 }
@@ -624,17 +628,30 @@ __global__ void __launch_bounds__(256, 3)
         }
         HistAcc h;
         const unsigned long long u0 = tk.u0 + (threadIdx.x >> 5), us = blockDim.x >> 5;
+        auto units = [&](auto nd_c, auto vec_c, auto tail_c, auto narrow_c) {
+            dq23_units<decltype(nd_c)::value, BS, decltype(vec_c)::value, decltype(tail_c)::value, false, false,
+                       decltype(narrow_c)::value>(a, c, u0, tk.u1, us, s_hist, s_prev, h);
+        };
+        using std::false_type;
+        using std::true_type;
+        constexpr std::integral_constant<int, 2> d2{};
+        constexpr std::integral_constant<int, 3> d3{};
+        constexpr std::integral_constant<bool, BS == 8> narrow{};  // of block size 8 only
         switch (tk.pad) {
             case 4 + 0: case 4 + 1: dq1d_units<BS, false>(a, c, u0, tk.u1, us, s_hist, h); break;
             case 4 + 2: case 4 + 3: dq1d_units<BS, true>(a, c, u0, tk.u1, us, s_hist, h); break;
-            case 8 + 0: dq23_units<2, BS, false, false>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
-            case 8 + 1: dq23_units<2, BS, false, true>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
-            case 8 + 2: dq23_units<2, BS, true, false>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
-            case 8 + 3: dq23_units<2, BS, true, true>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
-            case 12 + 0: dq23_units<3, BS, false, false>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
-            case 12 + 1: dq23_units<3, BS, false, true>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
-            case 12 + 2: dq23_units<3, BS, true, false>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
-            case 12 + 3: dq23_units<3, BS, true, true>(a, c, u0, tk.u1, us, s_hist, s_prev, h); break;
+            case 8 + 0: units(d2, false_type{}, false_type{}, false_type{}); break;
+            case 8 + 1: units(d2, false_type{}, true_type{}, false_type{}); break;
+            case 8 + 2: units(d2, true_type{}, false_type{}, false_type{}); break;
+            case 8 + 3: units(d2, true_type{}, true_type{}, false_type{}); break;
+            case 12 + 0: units(d3, false_type{}, false_type{}, false_type{}); break;
+            case 12 + 1: units(d3, false_type{}, true_type{}, false_type{}); break;
+            case 12 + 2: units(d3, true_type{}, false_type{}, false_type{}); break;
+            case 12 + 3: units(d3, true_type{}, true_type{}, false_type{}); break;
+            // narrow rows: the general loads and tails take them all
+            default:
+                if (tk.pad & 4) units(d3, false_type{}, true_type{}, narrow);
+                else units(d2, false_type{}, true_type{}, narrow);
         }
         hist_flush_block(a, s_hist, h);
         __syncthreads();  // the next task reuses shared memory
@@ -926,10 +943,11 @@ static void launch_23d(const DqArgs& a, bool vec, int grid, size_t smem, cudaStr
         smem_limit_once(kern, kDqSmemMax, at);
         kern<<<grid, 256, smem, st>>>(a);
     };
-    static std::atomic<unsigned long long> attr_strict{0}, attr_pad{0};
-    // strict and padded fields: general loads, tail columns decided at run time
+    static std::atomic<unsigned long long> attr_strict{0}, attr_pad{0}, attr_narrow{0};
+    // strict, padded and narrow fields: general loads, tail columns decided at run time
     if (a.strict) go(k_dq_compress_23d<NDIM, BS, false, true, true>, attr_strict);
     else if (a.pad.vals) go(k_dq_compress_23d<NDIM, BS, false, true, false, true>, attr_pad);
+    else if (a.grp > 1) go(k_dq_compress_23d<NDIM, BS, false, true, false, false, BS == 8>, attr_narrow);
     else if (vec && !tail) go(k_dq_compress_23d<NDIM, BS, true, false>, attr[0]);
     else if (vec) go(k_dq_compress_23d<NDIM, BS, true, true>, attr[1]);
     else if (!tail) go(k_dq_compress_23d<NDIM, BS, false, false>, attr[2]);
@@ -980,6 +998,7 @@ int dq_zlen_halvings(unsigned long long units, int bs, int num_sms) {
 }
 
 int launch_dq_compress(DqArgs a, int ndim, int bs, cudaStream_t st, int num_sms) {
+    dq_set_narrow(a, ndim, bs);
     if (ndim == 3) dq_set_zlen(a, bs, dq_zlen_halvings(a.nunits, bs, num_sms));
     const bool vec = (a.d0 % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.x) & 15u) == 0) &&
                      ((reinterpret_cast<uintptr_t>(a.code) & 7u) == 0);

@@ -312,6 +312,7 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
         mm[f] = MinmaxField{F.d_in, mmw};
         cs[f] = ConstsField{G.p.mode, G.p.eb, mmw, F.d_in, consts, status};
         dq[f] = make_dq_args(G.g, G.p.block_size, dict, F.d_in, consts, L.code[f], L.scratch[f], L.seg_count[f], hist);
+        dq_set_narrow(dq[f], G.g.ndim, G.p.block_size);
 
         HuffBuildArgs hb{};
         hb.hist    = hist;
@@ -400,7 +401,7 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
     for (uint32_t f = 0; f < nf; f++) {
         const Geometry& g = fg[f].g;
         const bool vec    = (g.d0 % 4 == 0) && ((reinterpret_cast<uintptr_t>(fields[f].d_in) & 15u) == 0);
-        B->dq_class.push_back(dq_class_of(g.ndim, vec, g.ndim >= 2 && (g.d0 % 8) != 0));
+        B->dq_class.push_back(dq_class_of(g.ndim, vec, g.ndim >= 2 && (g.d0 % 8) != 0, dq[f].grp > 1));
         B->minmax_units.push_back(fg[f].r2r ? fg[f].g.n : 0);
         B->dq_units.push_back(dq[f].nunits);
         B->enc_units.push_back(fg[f].nch);

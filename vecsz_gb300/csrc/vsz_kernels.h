@@ -99,7 +99,8 @@ struct DqArgs {
     const Consts* consts;
     uint32_t d0, d1, d2;
     uint32_t nxt;                // 128-wide x tiles per row
-    uint32_t nyg;                // groups of 8 rows
+    uint32_t nyg;                // groups of 8 rows (narrow rows: of grp x 8)
+    uint32_t lpr, grp;           // narrow rows (dq_set_narrow): lanes per row and row groups per warp; else 32, 1
     uint32_t nzb;                // units along z (3D): slabs of zlen planes; or 1
     uint32_t zlen;               // 3D: planes per unit, the block size or that halved (dq_set_zlen)
     uint32_t xtail;              // first tail column: d0 & ~7 when d0 % 8 != 0, else d0
@@ -232,6 +233,15 @@ int launch_dq_compress_f64(F64Args a, int ndim, cudaStream_t st, int num_sms);
 int launch_gather_f64(F64Args a, const unsigned long long* seg_off, DevOffset out_off, cudaStream_t st, int num_sms);
 int launch_dq_decompress_f64(F64Args a, int ndim, const unsigned long long* seg_off, cudaStream_t st);
 
+// Narrow rows (block size 8, 2D / 3D, rows of at most 64): a warp takes grp groups of 8 rows side by
+// side, lpr lanes each.  Before dq_set_zlen.
+inline void dq_set_narrow(DqArgs& a, int ndim, int bs) {
+    if (ndim < 2 || bs != 8 || a.d0 > 64 || a.strict || a.pad.vals) return;
+    a.lpr    = (a.d0 + 7) / 8 * 2;
+    a.grp    = 32 / a.lpr;
+    a.nyg    = ((a.d1 + 7) / 8 + a.grp - 1) / a.grp;
+    a.nunits = (unsigned long long)a.nxt * a.nyg * a.nzb;
+}
 // Planes per 3D unit: block_size halved `halvings` times (and nzb, nunits for it).  dq_zlen_halvings:
 // for a launch whose units number `units` at whole blocks.
 inline void dq_set_zlen(DqArgs& a, int bs, int halvings) {
@@ -266,7 +276,9 @@ int launch_pad_values(const PadArgs& a, cudaStream_t st, int num_sms);
 // holds the fields of one block size; a task's pad word is its field's kernel class (dq_class_of).
 // hist_words = shared-memory histogram words (0 when no field uses one); any3d: some field is 3D;
 // next = the launch's task counter (zero on entry), through which free blocks take tasks.
-inline uint32_t dq_class_of(int ndim, bool vec, bool tail) { return (uint32_t)ndim * 4u + (vec ? 2u : 0u) + (tail ? 1u : 0u); }
+inline uint32_t dq_class_of(int ndim, bool vec, bool tail, bool narrow) {
+    return (narrow ? 16u : 0u) + (uint32_t)ndim * 4u + (vec ? 2u : 0u) + (tail ? 1u : 0u);
+}
 int launch_minmax_batch(const MinmaxField* f, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st, int num_sms);
 int launch_consts_batch(const ConstsField* f, uint32_t nfields, cudaStream_t st);
 int launch_dq_compress_batch(const DqArgs* args, const BatchTask* tasks, uint32_t ntasks, int bs, bool any3d,
