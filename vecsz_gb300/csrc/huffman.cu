@@ -85,10 +85,13 @@ struct HeapKey {
     }
 };
 
-// The reference's heap, operation for operation (src/huffman.hh:169-192, 248-262).  Returns the
-// number of nodes created.
+// The reference's heap, operation for operation (src/huffman.hh:169-192, 248-262), by one thread.
+// Returns the number of nodes created.  Each operation depends on the one before: 20 levels a merge at
+// 65 cycles each.  Slower for 1024 symbols (0.63 ms): three levels a step with their 14 frequencies
+// loaded together (0.74), a warp taking five levels a step by ballots (0.98), two lanes running the two
+// removals of a merge two levels apart (1.39) -- branches and votes cost more than the loads they save.
 template <bool K32>
-__device__ __forceinline__ int heap_replay(BuildWs& w, int nused, int* fail) {
+__device__ __forceinline__ int heap_replay(BuildWs& w, int nused) {
     using K  = HeapKey<K32>;
     int qend = 1;
     for (int i = 0; i < nused; i++) {  // leaves: qinsert(new_node(freq, i)) in symbol order
@@ -144,7 +147,6 @@ __device__ __forceinline__ int heap_replay(BuildWs& w, int nused, int* fail) {
         }
         w.heap[ii] = key;
     }
-    (void)fail;
     return nnodes;
 }
 
@@ -197,41 +199,59 @@ __device__ __forceinline__ void build_field(const HuffBuildArgs& a, uint8_t* s_b
     if (threadIdx.x == 0) {
         unsigned long long total = 0;
         for (int i = 0; i < (int)(blockDim.x >> 5); i++) total += s_fsum[i];
-        int nnodes = nused;
-        if (nused == 0) s_fail = VSZ_ERR_INVALID;
-        else if (total >= (1ull << (64 - kKeyShift))) s_fail = VSZ_ERR_UNSUPPORTED;
-        else if (total < (1ull << 32)) nnodes = heap_replay<true>(w, nused, &s_fail);
-        else nnodes = heap_replay<false>(w, nused, &s_fail);
-        uint32_t node_count = 0, max_len = 0;
-        if (!s_fail) {
-            const int nint = nnodes - nused;
-            // subtree sizes bottom-up (children are always created before their parent)
-            for (int i = 0; i < nused; i++) w.size[i] = 1u;
-            for (int k = 0; k < nint; k++) w.size[nused + k] = 1u + w.size[w.lchild[k]] + w.size[w.rchild[k]];
-            // root = the last node created (a one-leaf tree: the leaf); preorder numbering of
-            // pad_tree_* (src/huffman.hh:374-423) and codewords of build_code (:200-227) top-down
-            const int root = nnodes - 1;
-            w.pre[root]   = 0u;
-            w.code[root]  = 0ull;
-            w.depth[root] = 0u;
-            for (int k = nint - 1; k >= 0; k--) {
-                const int v = nused + k, l = w.lchild[k], r = w.rchild[k];
-                const uint32_t pv = w.pre[v], dv = w.depth[v] + 1u;
-                const unsigned long long cv = w.code[v] << 1;
-                w.pre[l]   = pv + 1u;
-                w.pre[r]   = pv + 1u + w.size[l];
-                w.code[l]  = cv;
-                w.code[r]  = cv | 1ull;
-                w.depth[l] = dv;
-                w.depth[r] = dv;
-                if (dv > max_len) max_len = dv;
-            }
-            node_count = (uint32_t)nnodes;
-        }
+        int nnodes = nused, fail = 0;
+        if (nused == 0) fail = VSZ_ERR_INVALID;
+        else if (total >= (1ull << (64 - kKeyShift))) fail = VSZ_ERR_UNSUPPORTED;
+        else if (total < (1ull << 32)) nnodes = heap_replay<true>(w, nused);
+        else nnodes = heap_replay<false>(w, nused);
+        const uint32_t node_count = fail ? 0u : (uint32_t)nnodes;
+        s_fail    = fail;
         s_info[0] = node_count;
         s_info[1] = (uint32_t)tree_bytes_size(node_count);
-        s_info[2] = max_len;
+        s_info[2] = 0u;
         s_info[3] = (uint32_t)nnodes;
+    }
+    __syncthreads();
+    if (!s_fail) {
+        // every node on its own, by the way up to the root (the last node created; a one-leaf tree:
+        // the leaf): subtree sizes, then the preorder index of pad_tree_* (src/huffman.hh:374-423) and
+        // the codeword of build_code (:200-227)
+        const int nn = (int)s_info[0], root = nn - 1;
+        uint32_t* parent = reinterpret_cast<uint32_t*>(w.heap);  // parent << 1 | right; the heap is done with
+        for (int v = threadIdx.x; v < nn; v += blockDim.x) w.size[v] = 0u;
+        for (int k = threadIdx.x; k < nn - nused; k += blockDim.x) {
+            parent[w.lchild[k]] = (uint32_t)(nused + k) << 1;
+            parent[w.rchild[k]] = ((uint32_t)(nused + k) << 1) | 1u;
+        }
+        __syncthreads();
+        for (int v = threadIdx.x; v < nn; v += blockDim.x) {
+            for (int u = v;; u = (int)(parent[u] >> 1)) {
+                atomicAdd(&w.size[u], 1u);
+                if (u == root) break;
+            }
+        }
+        __syncthreads();
+        uint32_t longest = 0;
+        for (int v = threadIdx.x; v < nn; v += blockDim.x) {
+            uint32_t pre = 0, depth = 0;
+            unsigned long long code = 0;
+            for (int u = v; u != root;) {
+                const uint32_t p = parent[u];
+                pre += 1u;
+                if (p & 1u) {
+                    pre += w.size[w.lchild[(p >> 1) - nused]];
+                    if (depth < 64) code |= 1ull << depth;
+                }
+                depth++;
+                u = (int)(p >> 1);
+            }
+            w.pre[v]   = pre;
+            w.depth[v] = depth;
+            w.code[v]  = code;
+            longest    = max(longest, depth);
+        }
+        longest = __reduce_max_sync(0xffffffffu, longest);
+        if ((threadIdx.x & 31) == 0) atomicMax(&s_info[2], longest);
     }
     __syncthreads();
     if (s_fail) {
