@@ -660,8 +660,9 @@ __global__ void __launch_bounds__(128, 6) k_dq_decompress_b8s(DqDecArgs a) {
 // elements per lane instead of 512; the predictor is the reference's, in its FP32 order, so the
 // values are the same bits.  A warp holds 4 blocks along x.
 // ------------------------------------------------------------------------------------------
+// Units u = first, first + stride, ... < end of one field (one warp each).
 template <bool VEC>
-__global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
+__device__ __forceinline__ void dq_w8_units(const DqDecArgs& a, uint32_t first, uint32_t end, uint32_t stride) {
     const Consts c = *a.consts;
     if (c.status != VSZ_OK || *a.status != VSZ_OK) return;
     const int R           = a.R;
@@ -670,12 +671,9 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
     const unsigned lane   = lane_id();
     const int y           = (int)(lane & 7u);  // row of the block
     const uint32_t nxq    = (a.nbx8 + 3) / 4;  // groups of 4 blocks along x
-    const unsigned long long wtot = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-    for (unsigned long long u = (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-         u < a.nunits; u += wtot) {
-        const uint32_t xq = (uint32_t)(u % nxq);
-        const unsigned long long r = u / nxq;
-        const uint32_t yb = (uint32_t)(r % a.nyb), zb = (uint32_t)(r / a.nyb);
+    for (uint32_t u = first; u < end; u += stride) {  // at most kW8MaxN / 256 units
+        const uint32_t xq = u % nxq, r = u / nxq;
+        const uint32_t yb = r % a.nyb, zb = r / a.nyb;
         const uint32_t bx = xq * 4 + (lane >> 3);
         const uint32_t x0 = bx * 8, z0 = zb * 8, yr = yb * 8 + (uint32_t)y;
         const int nz        = (int)min(8u, a.d2 - z0);  // the same for the whole warp
@@ -755,6 +753,14 @@ __global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
         }
     }
 }
+
+template <bool VEC>
+__global__ void __launch_bounds__(128, 4) k_dq_decompress_w8(DqDecArgs a) {
+    dq_w8_units<VEC>(a, blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), (uint32_t)a.nunits,
+                     gridDim.x * (blockDim.x >> 5));
+}
+
+void dq_w8_geometry(DqDecArgs& a) { a.nunits = (unsigned long long)((a.nbx8 + 3) / 4) * a.nyb * ((a.d2 + 7) / 8); }
 
 bool dq_w8_applies(const DqDecArgs& a, int ndim) {
     if (ndim != 3 || a.pad.vals || a.n > kW8MaxN) return false;
@@ -947,8 +953,8 @@ bool dq_b8_separable(const DqDecArgs& a, int ndim) {
 }
 
 // ---- many fields (block size 8, no padding): tasks of (field, unit range), taken one at a time
-// by whichever warp is free (`next`: the class's task counter, zero at launch), so that warps do
-// not idle behind uneven tasks.  Per field the result is k_dq_decompress_b8 / _b8s's.
+// by whichever warp is free (`next`: the launch's task counter, zero at launch), so that warps do
+// not idle behind uneven tasks.  Per field the result is the single-field kernels'.
 __device__ __forceinline__ uint32_t dq_next_task(uint32_t* next) {
     uint32_t t = 0;
     if (lane_id() == 0) t = atomicAdd(next, 1u);
@@ -979,6 +985,28 @@ __global__ void __launch_bounds__(128, 6)
     }
 }
 
+// Small batches: every class in one launch, the task naming its class (tk.pad, kDqDec*).  A launch per
+// class runs them one after another, each too small to fill the GPU, and 3D fields take the wavefront
+// pass here (60 mixed fields, 20 M elements of them 3D: 594 -> 343 us).  In large batches (see
+// vsz_dbatch_create) the block kernels keep their own launches: one kernel of them all spills (632).
+__global__ void __launch_bounds__(128, 5)
+    k_dq_decompress_small_batch(const DqDecArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks,
+                                uint32_t* __restrict__ next) {
+    for (uint32_t t = dq_next_task(next); t < ntasks; t = dq_next_task(next)) {
+        const BatchTask tk = tasks[t];  // the field's arguments are read in place (a copy spills)
+        const DqDecArgs& a = args[tk.field];
+        const uint32_t u0 = (uint32_t)tk.u0, u1 = (uint32_t)tk.u1;
+        switch (tk.pad) {
+            case kDqDec1D: dq_b8_units<1, false, false, false>(a, u0, u1, 1u, nullptr, 0); break;
+            case kDqDec1D + kDqDecVec: dq_b8_units<1, true, false, false>(a, u0, u1, 1u, nullptr, 0); break;
+            case kDqDec2D: dq_b8_units<2, false, false, false>(a, u0, u1, 1u, nullptr, 0); break;
+            case kDqDec2D + kDqDecVec: dq_b8_units<2, true, false, false>(a, u0, u1, 1u, nullptr, 0); break;
+            case kDqDec3D: dq_w8_units<false>(a, u0, u1, 1u); break;
+            default: dq_w8_units<true>(a, u0, u1, 1u); break;
+        }
+    }
+}
+
 // The units the separable pass listed, one CTA per field (tasks carry only the field).
 __global__ void __launch_bounds__(128, 6)
     k_dq_decompress_redo_batch(const DqDecArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks) {
@@ -988,6 +1016,15 @@ __global__ void __launch_bounds__(128, 6)
         const DqDecArgs& a = args[tasks[t].field];  // read in place: fewer registers than a copy
         dq_b8_units<3, true, false, true>(a, wib, a.redo[0], 4u, reinterpret_cast<DqPlane*>(s_dq_dyn), wib);
     }
+}
+
+int launch_dq_decompress_small_batch(const DqDecArgs* args, const BatchTask* tasks, uint32_t ntasks, uint32_t* next,
+                                     cudaStream_t st, int num_sms) {
+    if (ntasks == 0) return VSZ_OK;
+    const uint32_t want = (ntasks + 3) / 4, cap = (uint32_t)num_sms * 5;  // resident CTAs of 4 warps
+    k_dq_decompress_small_batch<<<want < cap ? want : cap, 128, 0, st>>>(args, tasks, ntasks, next);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }
 
 int launch_dq_decompress_batch(const DqDecArgs* args, const BatchTask* tasks, uint32_t ntasks, int ndim, bool vec,
@@ -1031,7 +1068,7 @@ int launch_dq_decompress(DqDecArgs a, int ndim, int bs, bool force_general, cuda
         dq_b8_geometry(a, ndim);
         const bool vec = dq_b8_vec(a);
         if (dq_w8_applies(a, ndim)) {  // small 3D field: the wavefront pass
-            a.nunits = (unsigned long long)((a.nbx8 + 3) / 4) * a.nyb * ((a.d2 + 7) / 8);
+            dq_w8_geometry(a);
             const long long want = (long long)((a.nunits + 3) / 4), cap = (long long)num_sms * 16;
             const int grid = (int)(want < cap ? want : cap);
             if (vec) k_dq_decompress_w8<true><<<grid, 128, 0, st>>>(a);

@@ -409,6 +409,9 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
         B->copy_units.push_back(g.nseg);
     }
     for (auto& kv : classes) {
+        // kernel class by kernel class, so that blocks on the GPU together run the same code
+        std::stable_sort(kv.second.begin(), kv.second.end(),
+                         [&](uint32_t a, uint32_t b) { return B->dq_class[a] > B->dq_class[b]; });
         DqGroup grp{};
         grp.bs = kv.first;
         for (uint32_t f : kv.second) {

@@ -42,8 +42,12 @@ constexpr uint64_t kSplitTaskChunks = 64;     // (split decoder) its warps take 
 constexpr uint64_t kCopyTaskBytes = 1 << 12;  // index copies: a few KB a CTA, so that they spread
 constexpr uint64_t kOutTaskChunks = 64;       // outlier placement
 constexpr uint64_t kDqTaskUnits   = 1;        // reverse-Lorenzo warp units per task (one warp's)
+constexpr uint64_t kDqTaskUnits1D = 8;        // ... in a small batch's 1D fields (2048 elements)
 constexpr size_t kDqNextOff       = 64;       // after the batch status in the control tail: one
-constexpr size_t kDqMaxClasses    = 16;       // task counter per reverse-Lorenzo class
+constexpr size_t kDqMaxClasses    = 16;       // task counter per reverse-Lorenzo launch
+// 3D fields of a batch take the wavefront pass, and all its fields one launch, while they hold at most
+// this many elements together: 8 times the units of the block kernels, at twice the instructions.
+constexpr uint64_t kDbatchW8MaxN  = uint64_t(1) << 25;
 
 // A byte range copied into an aligned buffer (the archive's index).
 struct DCopy {
@@ -70,7 +74,7 @@ struct DField {
     double ebf;
     size_t nch;
     size_t units;  // block-8 warp units
-    bool sep, vec, konst;
+    bool sep, vec, konst, w8;
 };
 
 struct DqClass {
@@ -118,12 +122,13 @@ __global__ void k_dbatch_status(const DCheck* __restrict__ c, uint32_t nfields) 
     *k.out_status  = k.consts->status != VSZ_OK ? k.consts->status : *k.status;
 }
 
-void add_tasks(std::vector<BatchTask>& t, uint32_t field, uint64_t units, uint64_t per) {
+void add_tasks(std::vector<BatchTask>& t, uint32_t field, uint64_t units, uint64_t per, uint32_t cls = 0) {
     for (uint64_t u = 0; u < units; u += per) {
         BatchTask k{};
         k.u0    = u;
         k.u1    = std::min(units, u + per);
         k.field = field;
+        k.pad   = cls;
         t.push_back(k);
     }
 }
@@ -202,9 +207,18 @@ DLayout layout_dbatch(const std::vector<DField>& fs, uint8_t* base, size_t cap) 
     return L;
 }
 
-int dfields(const vsz_dbatch_field* fields, int nfields, std::vector<DField>& out) {
+// planes: 3D fields by the block kernels, not the wavefront pass
+int dfields(const vsz_dbatch_field* fields, int nfields, std::vector<DField>& out, bool* planes = nullptr) {
     if (!fields || nfields <= 0) return VSZ_ERR_INVALID;
     out.clear();
+    uint64_t n3 = 0;
+    for (int i = 0; i < nfields; i++) {
+        const vsz_archive_desc& d = fields[i].desc;  // checked below; a larger product only means more
+        if (d.ndim == 3) n3 += std::min<uint64_t>(d.dims[0], 1u << 31) * std::min<uint64_t>(d.dims[1] * d.dims[2], 1u << 31);
+        if (n3 > kDbatchW8MaxN) break;
+    }
+    const bool w8 = n3 <= kDbatchW8MaxN;
+    if (planes) *planes = !w8;
     for (int i = 0; i < nfields; i++) {
         DField f{};
         VSZ_TRY(field_of(fields[i], f));
@@ -217,14 +231,16 @@ int dfields(const vsz_dbatch_field* fields, int nfields, std::vector<DField>& ou
         a.n_outliers = fields[i].desc.n_outlier;
         a.redo       = reinterpret_cast<uint32_t*>(1);
         f.vec        = dq_b8_vec(a);
-        f.sep        = dq_b8_separable(a, f.g.ndim);
+        f.w8         = w8 && f.g.ndim == 3;
+        f.sep        = !f.w8 && dq_b8_separable(a, f.g.ndim);
         if (!f.sep) {  // the reference-order kernel groups narrow rows: its own unit count
             DqDecArgs t{};
             t.d0 = f.g.d0;
             t.d1 = f.g.d1;
             t.d2 = f.g.d2;
             dq_b8_geometry(t, f.g.ndim);
-            dq_b8_narrow(t, f.g.ndim);
+            if (f.w8) dq_w8_geometry(t);
+            else dq_b8_narrow(t, f.g.ndim);
             f.units = t.nunits;
         }
         out.push_back(f);
@@ -248,7 +264,8 @@ struct vsz_dbatch {
     const BatchTask* tasks = nullptr;
     uint32_t idx_off = 0, idx_n = 0, dec_off = 0, dec_n = 0, const_off = 0, const_n = 0, out_off = 0, out_n = 0;
     uint32_t redo_off = 0, redo_n = 0;
-    std::vector<DqClass> classes;
+    std::vector<DqClass> classes;       // a launch each, or
+    uint32_t small_off = 0, small_n = 0;  // one for all
     uint8_t* ctl = nullptr;
     size_t ctl_bytes = 0;
     uint16_t* all_bits = nullptr;
@@ -274,7 +291,8 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     if (!out || !d_ws || !d_status) return VSZ_ERR_INVALID;
     *out = nullptr;
     std::vector<DField> fs;
-    VSZ_TRY(dfields(fields, nfields, fs));
+    bool planes = true;
+    VSZ_TRY(dfields(fields, nfields, fs, &planes));
     DLayout L = layout_dbatch(fs, reinterpret_cast<uint8_t*>(d_ws), ws_bytes);
     if (L.bytes > ws_bytes) return VSZ_ERR_CAPACITY;
     const uint32_t nf = (uint32_t)nfields;
@@ -355,7 +373,8 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         q.xtail       = (G.g.ndim == 3 && (G.g.d0 % 8) != 0) ? (G.g.d0 & ~7u) : G.g.d0;
         q.redo        = L.redo[f];
         dq_b8_geometry(q, G.g.ndim);
-        if (!G.sep) dq_b8_narrow(q, G.g.ndim);
+        if (G.w8) dq_w8_geometry(q);
+        else if (!G.sep) dq_b8_narrow(q, G.g.ndim);
 
         ci[f] = DCopy{F.d_archive + d.index_offset, reinterpret_cast<uint8_t*>(L.all_bits + base), status};
         OutlierArgs& o = oa[f];
@@ -391,6 +410,17 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     B->out_n = (uint32_t)tasks.size() - B->out_off;
     std::map<std::tuple<int, bool, bool>, std::vector<uint32_t>> classes;
     for (uint32_t f = 0; f < nf; f++) classes[std::make_tuple(fs[f].g.ndim, fs[f].vec, fs[f].sep)].push_back(f);
+    B->small_off = (uint32_t)tasks.size();
+    if (!planes) {
+        // class by class, so that warps on the GPU together run the same code
+        for (auto kv = classes.rbegin(); kv != classes.rend(); ++kv) {
+            const int nd       = std::get<0>(kv->first);
+            const uint32_t cls = (nd == 1 ? kDqDec1D : nd == 2 ? kDqDec2D : kDqDec3D) + (std::get<1>(kv->first) ? kDqDecVec : 0u);
+            for (uint32_t f : kv->second) add_tasks(tasks, f, fs[f].units, nd == 1 ? kDqTaskUnits1D : kDqTaskUnits, cls);
+        }
+        classes.clear();
+    }
+    B->small_n = (uint32_t)tasks.size() - B->small_off;
     static_assert(kDqNextOff + 4 * kDqMaxClasses <= 256, "the counters fit the control tail");
     if (classes.size() > kDqMaxClasses) {  // 3 dimensionalities x aligned or not x separable or not
         delete B;
@@ -508,6 +538,7 @@ vsz_status vsz_dbatch_decompress(vsz_dbatch* B, void* stream) {
     {
         StageTimer t(kStLorenzoDecompress, st);
         uint32_t* next = reinterpret_cast<uint32_t*>(B->ctl + B->nfields * kDCtlBytes + kDqNextOff);
+        VSZ_TRY(launch_dq_decompress_small_batch(B->dq, B->tasks + B->small_off, B->small_n, next, st, sms));
         for (size_t i = 0; i < B->classes.size(); i++) {
             const DqClass& c = B->classes[i];
             VSZ_TRY(launch_dq_decompress_batch(B->dq, B->tasks + c.task_off, c.ntasks, c.ndim, c.vec, c.sep, next + i,

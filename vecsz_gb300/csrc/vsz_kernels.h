@@ -72,7 +72,7 @@ __device__ __forceinline__ Halo halo_of(const PadView& p, int ndim, uint32_t bx,
 struct BatchTask {
     unsigned long long u0, u1;
     uint32_t field;
-    uint32_t pad;  // dual-quant tasks: the field's kernel class
+    uint32_t pad;  // dual-quant and reverse Lorenzo tasks: the field's kernel class
 };
 
 struct MinmaxField {
@@ -201,9 +201,15 @@ bool dq_b8_separable(const DqDecArgs& a, int ndim);
 // The wavefront pass applies: 3D, no padding, at most kW8MaxN elements (kW8MaxSeparableN for a
 // field the separable pass takes), VSZ_DQ_NO_WAVEFRONT unset.
 bool dq_w8_applies(const DqDecArgs& a, int ndim);
-// Many fields of one class (ndim, vec, separable), block size 8, no padding: tasks of (field,
-// unit range), one warp each, handed out through the counter `next` (zero on entry; the class's
-// own word).  A separable class is followed by launch_dq_redo_batch over its fields.
+void dq_w8_geometry(DqDecArgs& a);  // its units (after dq_b8_geometry)
+// Many fields, block size 8, no padding: tasks of (field, unit range), one warp each, handed out
+// through the counter `next` (zero on entry; each launch's own word).  Small batches: fields of
+// every class, 3D ones by the wavefront pass; a task's pad word is its field's class (kDqDec*).
+// Others: the fields of one class (ndim, vec, separable); a separable class is followed by
+// launch_dq_redo_batch over its fields.
+constexpr uint32_t kDqDec1D = 0, kDqDec2D = 2, kDqDec3D = 4, kDqDecVec = 1;  // + kDqDecVec: 16-byte rows
+int launch_dq_decompress_small_batch(const DqDecArgs* args, const BatchTask* tasks, uint32_t ntasks, uint32_t* next,
+                                     cudaStream_t st, int num_sms);
 int launch_dq_decompress_batch(const DqDecArgs* args, const BatchTask* tasks, uint32_t ntasks, int ndim, bool vec,
                                bool sep, uint32_t* next, cudaStream_t st, int num_sms);
 int launch_dq_redo_batch(const DqDecArgs* args, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st,
