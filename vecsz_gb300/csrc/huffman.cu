@@ -1067,19 +1067,25 @@ constexpr int kWinRound     = 8;
 constexpr int kWinRing      = 8;    // blocks of 16 bytes per lane
 constexpr int kWinWait      = 4;    // copy groups left in flight at a round's start
 constexpr int kWinLaneWords = kWinRing * 4 + 4;  // a lane's ring, padded: lanes 8 apart share banks
-constexpr int kWinThreads   = 256;  // one primary table per CTA, shared by its warps
-constexpr int kWinMinBlocks = 4;
+constexpr int kWinThreads   = 512;  // one copy of the tables per CTA, shared by its warps
+constexpr int kWinMinBlocks = 2;
+constexpr int kWinBatchThreads = 256, kWinBatchBlocks = 3;
+// Secondary entries in shared memory (a 1024-symbol tree has 2.5-4.3 K; those past it are read from
+// L2).  In L2 they stalled a warp whenever one lane left the primary table, on 59 % of the steps at 6.5
+// bits a code.
+constexpr uint32_t kWinTable2 = 4096;
 // Blocks wn / 4 .. wn / 4 + kWinRing - 2 are requested and all but the newest kWinWait have landed
 // at a round's start: at least 4 (kWinRing - 1 - kWinWait) - 3 words from wn, and a round of
 // kWinRound codewords of <= 32 bits moves the window by at most kWinRound words.
 static_assert(4 * (kWinRing - 1 - kWinWait) - 3 >= kWinRound, "a round may read words still in flight");
 static_assert((kWinRing & (kWinRing - 1)) == 0 && (kWinRound == 8 || kWinRound == 4), "ring and round shapes");
-constexpr size_t kWinSmem   = (sizeof(uint32_t) << kDecBits) + (size_t)kWinThreads * kWinLaneWords * 4;
+constexpr size_t kWinTables = (sizeof(uint32_t) << kDecBits) + sizeof(uint32_t) * kWinTable2;
+constexpr size_t win_smem(int threads) { return kWinTables + (size_t)threads * kWinLaneWords * 4; }
 typedef uint32_t WinRing[32][kWinLaneWords];  // one warp's rings, [lane][word]
 
-// Lane j of the calling warp decodes chunk j (the table is in s_table; no block barrier inside).
+// Lane j of the calling warp decodes chunk j (the tables are in shared memory; no block barrier inside).
 __device__ __forceinline__ void decode_win_lane(const HuffDecodeArgs& a, size_t j, const uint32_t* s_table,
-                                                WinRing* s_ring) {
+                                                const uint32_t* s_table2, WinRing* s_ring) {
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (j - lane >= a.nchunks) return;
     const unsigned long long out0 = (unsigned long long)j * kChunkSyms;
@@ -1161,8 +1167,8 @@ __device__ __forceinline__ void decode_win_lane(const HuffDecodeArgs& a, size_t 
                 uint32_t node = e >> 8, usedb = kDecBits;
                 if (e & 0x80u) {
                     const uint32_t w2b = (e >> 8) & 0xfu;
-                    const uint32_t e2 =
-                        __ldg(&a.table2[(e >> 12) + ((win >> (32 - kDecBits - w2b)) & ((1u << w2b) - 1u))]);
+                    const uint32_t i2  = (e >> 12) + ((win >> (32 - kDecBits - w2b)) & ((1u << w2b) - 1u));
+                    const uint32_t e2  = i2 < kWinTable2 ? s_table2[i2] : __ldg(&a.table2[i2]);
                     len   = e2 & 0xffu;
                     sy    = e2 >> 8;
                     node  = e2 >> 8;
@@ -1247,16 +1253,23 @@ __device__ __forceinline__ void decode_win_lane(const HuffDecodeArgs& a, size_t 
     if (j < a.nchunks && a.chunk_zero) a.chunk_zero[j] = zeros;
 }
 
+// Both tables of one field into shared memory, by the whole CTA.
+__device__ __forceinline__ void win_tables(const HuffDecodeArgs& a, uint32_t* s_table) {
+    for (uint32_t i = threadIdx.x; i < (1u << kDecBits); i += blockDim.x) s_table[i] = a.table[i];
+    const uint32_t n2 = min(a.tree_info[3], kWinTable2);
+    for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) s_table[(1 << kDecBits) + i] = a.table2[i];
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kWinThreads, kWinMinBlocks) k_huff_decode_win(HuffDecodeArgs a) {
     extern __shared__ __align__(16) uint8_t s_win_dyn[];
-    // [primary table: 1 << kDecBits words][rings: warp][lane][kWinLaneWords] (kWinSmem bytes)
+    // [primary table: 1 << kDecBits words][kWinTable2 words][rings: warp][lane][kWinLaneWords]
     uint32_t* s_table = reinterpret_cast<uint32_t*>(s_win_dyn);
-    WinRing* s_ring   = reinterpret_cast<WinRing*>(s_win_dyn + (sizeof(uint32_t) << kDecBits));
+    WinRing* s_ring   = reinterpret_cast<WinRing*>(s_win_dyn + kWinTables);
     if (!a.tree_info || a.tree_info[2] > (uint32_t)kWinMaxLen) return;  // uniform: k_huff_decode_idx's trees
-    for (int i = threadIdx.x; i < (1 << kDecBits); i += blockDim.x) s_table[i] = a.table[i];
-    __syncthreads();
+    win_tables(a, s_table);
     if (*a.status != VSZ_OK) return;  // no block barrier below
-    decode_win_lane(a, blockIdx.x * (size_t)blockDim.x + threadIdx.x, s_table, s_ring);
+    decode_win_lane(a, blockIdx.x * (size_t)blockDim.x + threadIdx.x, s_table, s_table + (1 << kDecBits), s_ring);
 }
 
 constexpr int kDecRound = 16;                 // codes per lane staged before the coalesced store
@@ -1466,18 +1479,17 @@ __global__ void __launch_bounds__(256) k_huff_decode_idx(HuffDecodeArgs a) {
 // ---- many fields: tasks of (field, chunk range [256 k, 256 k + 256) of its index), one CTA
 // each; lane t of the CTA decodes chunk u0 + t.  A kernel takes the tasks of the fields whose trees
 // are of its kind (read from k_huff_table's results, so uniform over the CTA) and skips the rest.
-__global__ void __launch_bounds__(kWinThreads, kWinMinBlocks)
+__global__ void __launch_bounds__(kWinBatchThreads, kWinBatchBlocks)
     k_huff_decode_win_batch(const HuffDecodeArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks) {
     extern __shared__ __align__(16) uint8_t s_win_dyn[];
     uint32_t* s_table = reinterpret_cast<uint32_t*>(s_win_dyn);
-    WinRing* s_ring = reinterpret_cast<WinRing*>(s_win_dyn + (sizeof(uint32_t) << kDecBits));
+    WinRing* s_ring = reinterpret_cast<WinRing*>(s_win_dyn + kWinTables);
     for (uint32_t t = blockIdx.x; t < ntasks; t += gridDim.x) {
         const BatchTask tk     = tasks[t];
         const HuffDecodeArgs a = args[tk.field];
         if (a.tree_info[2] > (uint32_t)kWinMaxLen) continue;
-        for (int i = threadIdx.x; i < (1 << kDecBits); i += blockDim.x) s_table[i] = a.table[i];
-        __syncthreads();
-        if (*a.status == VSZ_OK) decode_win_lane(a, tk.u0 + threadIdx.x, s_table, s_ring);
+        win_tables(a, s_table);
+        if (*a.status == VSZ_OK) decode_win_lane(a, tk.u0 + threadIdx.x, s_table, s_table + (1 << kDecBits), s_ring);
         __syncthreads();
     }
 }
@@ -1769,11 +1781,11 @@ int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks,
                                              split_smem<kSplitS>(kSplitThreads), st>>>(args, tasks, ntasks);
         count_launch();
     } else if (ntasks) {
-        const uint32_t cap  = (uint32_t)num_sms * kWinMinBlocks;
+        const uint32_t cap  = (uint32_t)num_sms * kWinBatchBlocks;
         const uint32_t grid = ntasks < cap ? ntasks : cap;
         static std::atomic<unsigned long long> attr{0};
-        smem_limit_once(k_huff_decode_win_batch, (int)kWinSmem, attr);
-        k_huff_decode_win_batch<<<grid, kWinThreads, kWinSmem, st>>>(args, tasks, ntasks);
+        smem_limit_once(k_huff_decode_win_batch, (int)win_smem(kWinBatchThreads), attr);
+        k_huff_decode_win_batch<<<grid, kWinBatchThreads, win_smem(kWinBatchThreads), st>>>(args, tasks, ntasks);
         count_launch();
         k_huff_decode_idx_batch<<<grid, 256, 0, st>>>(args, tasks, ntasks);
         count_launch();
@@ -2044,8 +2056,11 @@ int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms) {
     } else if (indexed) {
         if (a.tree_info) {
             static std::atomic<unsigned long long> attr_win{0};
-            smem_limit_once(k_huff_decode_win, (int)kWinSmem, attr_win);
-            k_huff_decode_win<<<(unsigned)((a.nchunks + kWinThreads - 1) / kWinThreads), kWinThreads, kWinSmem, st>>>(a);
+            smem_limit_once(k_huff_decode_win, (int)win_smem(kWinThreads), attr_win);
+            // whole warps over as many SMs as there are, at most kWinThreads to a copy of the tables
+            const size_t per  = (a.nchunks + (size_t)num_sms * kWinMinBlocks - 1) / ((size_t)num_sms * kWinMinBlocks);
+            const int threads = 32 * (int)min((size_t)kWinThreads / 32, max((size_t)2, (per + 31) / 32));
+            k_huff_decode_win<<<(unsigned)((a.nchunks + threads - 1) / threads), threads, win_smem(threads), st>>>(a);
             count_launch();
         }
         if (a.walk_smem) {
