@@ -28,10 +28,57 @@
 namespace vsz {
 
 // ------------------------------------------------------------------------------------------
-// K0: min / max of the field for r2r (GetDatumValueRange, src/types.cc:28-35)
+// K0: min / max of the field for r2r (GetDatumValueRange, src/types.cc:28-35) and the constants
 // ------------------------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(256) k_minmax(const float* __restrict__ x, size_t n, uint32_t* __restrict__ mm) {
+// Error-bound constants (one thread).  For r2r: range = (double)((float)max - (float)min), with
+// std::max_element's rule that a NaN first element wins; a zero range is VSZ_ERR_RANGE, as the
+// reference exits there (src/types.cc:49-56).
+__device__ __forceinline__ void consts_of(int mode, double eb, const uint32_t* __restrict__ mm,
+                                          const float* __restrict__ x, Consts* __restrict__ c, int* status_word) {
+    double ebf   = eb;
+    double range = 0.0;
+    int status   = VSZ_OK;
+    if (mode == VSZ_MODE_R2R) {
+        float x0 = x[0];
+        float mx, mn;
+        if (x0 != x0) {
+            mx = x0;
+            mn = x0;
+        } else {
+            mx = key2f(mm[0]);
+            mn = key2f(mm[1]);
+        }
+        float r = __fsub_rn(mx, mn);
+        range   = (double)r;
+        if (range == 0.0) status = VSZ_ERR_RANGE;
+        ebf = __dmul_rn(ebf, range);
+    }
+    c->eb_final = ebf;
+    c->r_d      = 1.0 / __dmul_rn(2.0, ebf);  // src/types.cc:91
+    c->c_d      = __dmul_rn(2.0, ebf);        // src/types.cc:90
+    c->range    = range;
+    c->r_f      = __double2float_rn(c->r_d);
+    float ch    = __double2float_rn(c->c_d);
+    float cl    = __double2float_rn(__dsub_rn(c->c_d, (double)ch));
+    c->c_hi     = ch;
+    c->c_lo     = cl;
+    auto normal = [](float f) {
+        uint32_t e = __float_as_uint(f) & 0x7f800000u;
+        return e != 0u && e != 0x7f800000u;
+    };
+    c->dq_fast  = normal(ch) && (cl == 0.0f || normal(cl));
+    c->status   = status;
+    c->dq_mul   = 0;  // until k_dq_mul_verify has checked the two-operation dequantization
+    c->dq_exc   = 0.f;
+    c->dq_exc_y = 0.f;
+    if (status != VSZ_OK && status_word) set_status(status_word, status);
+}
+
+// mm: {max key, min key, finished blocks}, {0, 0xffffffff, 0} on entry; the last block computes the
+// constants.
+__global__ void __launch_bounds__(256) k_minmax(const float* __restrict__ x, size_t n, uint32_t* __restrict__ mm,
+                                                double eb, Consts* __restrict__ c, int* status_word) {
     uint32_t kmax = 0u, kmin = 0xffffffffu;
     size_t tid    = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -77,51 +124,35 @@ __global__ void __launch_bounds__(256) k_minmax(const float* __restrict__ x, siz
         }
         atomicMax(&mm[0], kmax);
         atomicMin(&mm[1], kmin);
+        __threadfence();
+        if (atomicAdd(&mm[2], 1u) == gridDim.x - 1) {  // the last block: the extremes are final
+            __threadfence();
+            const uint32_t all[2] = {atomicMax(&mm[0], 0u), atomicMin(&mm[1], 0xffffffffu)};
+            consts_of(VSZ_MODE_R2R, eb, all, x, c, status_word);
+        }
     }
 }
 
-// Error-bound constants (one thread).  For r2r: range = (double)((float)max - (float)min), with
-// std::max_element's rule that a NaN first element wins; a zero range is VSZ_ERR_RANGE, as the
-// reference exits there (src/types.cc:49-56).
-__device__ __forceinline__ void consts_of(int mode, double eb, const uint32_t* __restrict__ mm,
-                                          const float* __restrict__ x, Consts* __restrict__ c, int* status_word) {
-    double ebf   = eb;
-    double range = 0.0;
-    int status   = VSZ_OK;
-    if (mode == VSZ_MODE_R2R) {
-        float x0 = x[0];
-        float mx, mn;
-        if (x0 != x0) {
-            mx = x0;
-            mn = x0;
-        } else {
-            mx = key2f(mm[0]);
-            mn = key2f(mm[1]);
-        }
-        float r = __fsub_rn(mx, mn);
-        range   = (double)r;
-        if (range == 0.0) status = VSZ_ERR_RANGE;
-        ebf = __dmul_rn(ebf, range);
+// What a call needs cleared, and the constants of an absolute bound (mode abs), in one launch: a
+// stream's small memsets cost 2 us each, and a compress had eleven of them, a decompress six (64^3: 95
+// -> 74 and 88 -> 67 us).
+__global__ void __launch_bounds__(256) k_init(InitArgs i) {
+    const size_t t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    for (size_t k = t0; k < i.words; k += step) i.zero[k] = 0u;
+    if (t0 < 4 && i.zero4) i.zero4[t0] = 0u;
+    if (t0 != 0) return;
+    if (i.mode == VSZ_MODE_ABS) consts_of(i.mode, i.eb, nullptr, nullptr, i.consts, nullptr);
+    if (i.mm) {
+        i.mm[0] = i.mm[2] = 0u;
+        i.mm[1] = 0xffffffffu;
     }
-    c->eb_final = ebf;
-    c->r_d      = 1.0 / __dmul_rn(2.0, ebf);  // src/types.cc:91
-    c->c_d      = __dmul_rn(2.0, ebf);        // src/types.cc:90
-    c->range    = range;
-    c->r_f      = __double2float_rn(c->r_d);
-    float ch    = __double2float_rn(c->c_d);
-    float cl    = __double2float_rn(__dsub_rn(c->c_d, (double)ch));
-    c->c_hi     = ch;
-    c->c_lo     = cl;
-    auto normal = [](float f) {
-        uint32_t e = __float_as_uint(f) & 0x7f800000u;
-        return e != 0u && e != 0x7f800000u;
-    };
-    c->dq_fast  = normal(ch) && (cl == 0.0f || normal(cl));
-    c->status   = status;
-    c->dq_mul   = 0;  // until k_dq_mul_verify has checked the two-operation dequantization
-    c->dq_exc   = 0.f;
-    c->dq_exc_y = 0.f;
-    if (status != VSZ_OK && status_word) set_status(status_word, status);
+}
+
+int launch_init(const InitArgs& i, cudaStream_t st) {
+    const size_t want = (i.words + 1023) / 1024;
+    k_init<<<(unsigned)(want < 1 ? 1 : want < 128 ? want : 128), 256, 0, st>>>(i);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }
 
 __global__ void k_consts(int mode, double eb, const uint32_t* __restrict__ mm, const float* __restrict__ x,
@@ -908,17 +939,23 @@ __global__ void k_consts_batch(const ConstsField* __restrict__ f, uint32_t nfiel
 // Host-side launchers
 // ------------------------------------------------------------------------------------------
 
+int launch_range(double eb, const float* d_in, size_t n, Consts* d_consts, uint32_t* d_mm, cudaStream_t st,
+                 int* status_word) {
+    const size_t nb  = (n + 1023) / 1024;
+    const int blocks = (int)(nb < 1 ? 1 : nb < (size_t)(152 * 8) ? nb : (size_t)(152 * 8));
+    k_minmax<<<blocks, 256, 0, st>>>(d_in, n, d_mm, eb, d_consts, status_word);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
+}
+
 int launch_eb_setup(int mode, double eb, const float* d_in, size_t n, Consts* d_consts, uint32_t* d_mm,
                     cudaStream_t st, int* status_word) {
     if (mode == VSZ_MODE_R2R) {
-        // {0, 0xffffffff} by memsets: a copy from a host array would, under stream capture, bake
+        // {0, 0xffffffff, 0} by memsets: a copy from a host array would, under stream capture, bake
         // that host address into the graph
-        if (cudaMemsetAsync(d_mm, 0, 4, st) != cudaSuccess || cudaMemsetAsync(d_mm + 1, 0xff, 4, st) != cudaSuccess)
+        if (cudaMemsetAsync(d_mm, 0, 12, st) != cudaSuccess || cudaMemsetAsync(d_mm + 1, 0xff, 4, st) != cudaSuccess)
             return VSZ_ERR_CUDA;
-        size_t nb = (n + 1023) / 1024; int blocks = (int)(nb < (size_t)(152 * 8) ? nb : (size_t)(152 * 8));
-        if (blocks < 1) blocks = 1;
-        k_minmax<<<blocks, 256, 0, st>>>(d_in, n, d_mm);
-        count_launch();
+        return launch_range(eb, d_in, n, d_consts, d_mm, st, status_word);
     }
     k_consts<<<1, 32, 0, st>>>(mode, eb, d_mm, d_in, d_consts, status_word);
     count_launch();
@@ -1015,13 +1052,14 @@ int launch_dq_compress(DqArgs a, int ndim, int bs, cudaStream_t st, int num_sms)
     return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }
 
-int launch_outlier_gather(GatherArgs g, cudaStream_t st, int num_sms) {
+int launch_outlier_gather(GatherArgs g, cudaStream_t st, int num_sms, bool cleared) {
     g.ntiles = (uint32_t)((g.nseg + kGatherTile - 1) / kGatherTile);
     if (g.ntiles == 0) {
         return cudaMemsetAsync(g.total, 0, sizeof(unsigned long long), st) == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
     }
-    if (cudaMemsetAsync(g.tile_status, 0, sizeof(unsigned long long) * g.ntiles, st) != cudaSuccess) return VSZ_ERR_CUDA;
-    if (cudaMemsetAsync(g.tile_counter, 0, sizeof(uint32_t), st) != cudaSuccess) return VSZ_ERR_CUDA;
+    if (!cleared && (cudaMemsetAsync(g.tile_status, 0, sizeof(unsigned long long) * g.ntiles, st) != cudaSuccess ||
+                     cudaMemsetAsync(g.tile_counter, 0, sizeof(uint32_t), st) != cudaSuccess))
+        return VSZ_ERR_CUDA;
     k_outlier_gather<<<g.ntiles, kGatherThreads, 0, st>>>(g);
     count_launch();
     if (g.seg_off) {

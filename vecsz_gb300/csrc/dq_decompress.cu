@@ -1098,7 +1098,7 @@ int launch_dq_decompress(DqDecArgs a, int ndim, int bs, bool force_general, cuda
             // separable pass, then the reference-order kernel over the units it listed.  A large
             // field first checks the cheaper dequantization (a few microseconds, all SMs).
             const bool verify = a.consts_rw && a.n >= kDqVerifyMin;
-            if (cudaMemsetAsync(a.redo, 0, (verify ? 3 : 1) * sizeof(uint32_t), st) != cudaSuccess)
+            if (!a.redo_cleared && cudaMemsetAsync(a.redo, 0, (verify ? 3 : 1) * sizeof(uint32_t), st) != cudaSuccess)
                 return VSZ_ERR_CUDA;
             if (verify) {
                 k_dq_mul_verify<<<(unsigned)num_sms * 4, 256, 0, st>>>(a.consts_rw, a.redo, a.dq_cache);

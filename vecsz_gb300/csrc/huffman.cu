@@ -320,9 +320,6 @@ __global__ void __launch_bounds__(256) k_huff_build_batch(const HuffBuildArgs* _
     }
 }
 
-int launch_scan_u32(const uint32_t* in, unsigned long long* out, size_t n, unsigned long long* tile_status,
-                    uint32_t* tile_counter, unsigned long long* total, int* status, cudaStream_t st);
-
 // ------------------------------------------------------------------------------------------
 // K3: encoder, two passes over the codes with no cross-warp waiting.  The unit is a chunk of 512
 // codes -- one warp, 16 codes per lane -- the same chunk the decode index records:
@@ -1883,18 +1880,20 @@ __global__ void __launch_bounds__(256) k_huff_sync_round(HuffSyncArgs a, const u
 // Generic exclusive scan (decoupled look-back) of u16/u32 values into u64 offsets.
 // ------------------------------------------------------------------------------------------
 
-template <typename TIn>
-__global__ void __launch_bounds__(256) k_scan_excl(const TIn* __restrict__ in, unsigned long long* __restrict__ out,
-                                                   size_t n, unsigned long long* tile_status, uint32_t* tile_counter,
-                                                   unsigned long long* total, int* status) {
-    constexpr int PER = 16;
+// One tile of kScanTile values (the next ticket), by a CTA of THREADS.
+constexpr int kScanTile = 4096;
+template <typename TIn, int THREADS>
+__device__ __forceinline__ void scan_tile(const TIn* __restrict__ in, unsigned long long* __restrict__ out, size_t n,
+                                          unsigned long long* tile_status, uint32_t* tile_counter,
+                                          unsigned long long* total, int* status) {
+    constexpr int PER = kScanTile / THREADS;
     __shared__ unsigned long long s_scan[33];
     __shared__ unsigned long long s_base;
     __shared__ uint32_t s_tile;
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
-    const size_t i0     = (size_t)tile * 256 * PER + (size_t)threadIdx.x * PER;
+    const size_t i0     = (size_t)tile * kScanTile + (size_t)threadIdx.x * PER;
     unsigned long long v[PER], sum = 0;
 #pragma unroll
     for (int k = 0; k < PER; k++) {
@@ -1907,7 +1906,7 @@ __global__ void __launch_bounds__(256) k_scan_excl(const TIn* __restrict__ in, u
         const unsigned long long b = lookback_publish_warp(tile_status, tile, tot, status);
         if (threadIdx.x == 0) {
             s_base = b;
-            if ((size_t)(tile + 1) * 256 * PER >= n && total) *total = b + tot;
+            if ((size_t)(tile + 1) * kScanTile >= n && total) *total = b + tot;
         }
     }
     __syncthreads();
@@ -1917,6 +1916,22 @@ __global__ void __launch_bounds__(256) k_scan_excl(const TIn* __restrict__ in, u
         if (i0 + k < n) out[i0 + k] = run;
         run += v[k];
     }
+}
+
+template <typename TIn>
+__global__ void __launch_bounds__(256) k_scan_excl(const TIn* __restrict__ in, unsigned long long* __restrict__ out,
+                                                   size_t n, unsigned long long* tile_status, uint32_t* tile_counter,
+                                                   unsigned long long* total, int* status) {
+    scan_tile<TIn, 256>(in, out, n, tile_status, tile_counter, total, status);
+}
+
+// The decode tables (block 0) and, beside them, the scan of the decode index (a tile per other block):
+// neither needs the other.
+__global__ void __launch_bounds__(1024) k_huff_table_scan(HuffTableArgs a, const uint16_t* __restrict__ bits,
+                                                          unsigned long long* __restrict__ start, size_t n,
+                                                          unsigned long long* tile_status, uint32_t* tile_counter) {
+    if (blockIdx.x == 0) huff_table_run(a);
+    else scan_tile<uint16_t, 1024>(bits, start, n, tile_status, tile_counter, nullptr, a.status);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2017,7 +2032,7 @@ int launch_huff_encode(HuffEncodeArgs a, cudaStream_t st, int num_sms) {
         k_huff_count<<<grid, kEncThreads, a.cb_in_smem ? (size_t)a.dict : 0, st>>>(a);
         count_launch();
         int rc = launch_scan_u16(a.chunk_bits, a.chunk_off, a.nchunks, a.scan_status, a.scan_counter, a.total_bits,
-                                 a.status, st);
+                                 a.status, st, a.scan_cleared);
         if (rc) return rc;
     }
     {
@@ -2033,6 +2048,14 @@ int launch_huff_encode(HuffEncodeArgs a, cudaStream_t st, int num_sms) {
 
 int launch_huff_table(HuffTableArgs a, cudaStream_t st) {
     k_huff_table<<<1, 1024, 0, st>>>(a);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
+}
+
+int launch_huff_table_scan(HuffTableArgs a, const uint16_t* bits, unsigned long long* start, size_t n,
+                           unsigned long long* tile_status, uint32_t* tile_counter, cudaStream_t st) {
+    k_huff_table_scan<<<(unsigned)(1 + (n + kScanTile - 1) / kScanTile), 1024, 0, st>>>(a, bits, start, n, tile_status,
+                                                                                       tile_counter);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }
@@ -2104,26 +2127,27 @@ int launch_huff_sync_round(HuffSyncArgs a, const unsigned long long* exit_in, un
 
 template <typename TIn>
 int launch_scan_excl_t(const TIn* in, unsigned long long* out, size_t n, unsigned long long* tile_status,
-                       uint32_t* tile_counter, unsigned long long* total, int* status, cudaStream_t st) {
+                       uint32_t* tile_counter, unsigned long long* total, int* status, cudaStream_t st, bool cleared) {
     size_t ntiles = (n + 4095) / 4096;
     if (ntiles == 0) {
         if (total) return cudaMemsetAsync(total, 0, 8, st) == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
         return VSZ_OK;
     }
-    if (cudaMemsetAsync(tile_status, 0, 8 * ntiles, st) != cudaSuccess) return VSZ_ERR_CUDA;
-    if (cudaMemsetAsync(tile_counter, 0, 4, st) != cudaSuccess) return VSZ_ERR_CUDA;
+    if (!cleared && (cudaMemsetAsync(tile_status, 0, 8 * ntiles, st) != cudaSuccess ||
+                     cudaMemsetAsync(tile_counter, 0, 4, st) != cudaSuccess))
+        return VSZ_ERR_CUDA;
     k_scan_excl<TIn><<<(unsigned)ntiles, 256, 0, st>>>(in, out, n, tile_status, tile_counter, total, status);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? VSZ_OK : VSZ_ERR_CUDA;
 }
 
 int launch_scan_u16(const uint16_t* in, unsigned long long* out, size_t n, unsigned long long* ts, uint32_t* tc,
-                    unsigned long long* total, int* status, cudaStream_t st) {
-    return launch_scan_excl_t<uint16_t>(in, out, n, ts, tc, total, status, st);
+                    unsigned long long* total, int* status, cudaStream_t st, bool cleared) {
+    return launch_scan_excl_t<uint16_t>(in, out, n, ts, tc, total, status, st, cleared);
 }
 int launch_scan_u32(const uint32_t* in, unsigned long long* out, size_t n, unsigned long long* ts, uint32_t* tc,
-                    unsigned long long* total, int* status, cudaStream_t st) {
-    return launch_scan_excl_t<uint32_t>(in, out, n, ts, tc, total, status, st);
+                    unsigned long long* total, int* status, cudaStream_t st, bool cleared) {
+    return launch_scan_excl_t<uint32_t>(in, out, n, ts, tc, total, status, st, cleared);
 }
 
 size_t scan_tmp_tiles(size_t n) { return (n + 4095) / 4096; }

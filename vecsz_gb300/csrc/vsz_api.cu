@@ -93,19 +93,24 @@ struct CompressWs {
 CompressWs layout_compress(const Geometry& g, int dict, uint8_t* base, size_t cap) {
     Bump b{base, cap};
     CompressWs w{};
+    w.n_chunks  = (g.n + kChunkSyms - 1) / kChunkSyms;
+    size_t gt   = (g.nseg + 4095) / 4096 + 1;
     w.consts    = b.take<Consts>(1);
     w.mm        = b.take<uint32_t>(4);
+    // what a call clears, in one piece
     w.status    = b.take<int>(4);
     w.hist      = b.take<unsigned long long>(dict);
+    w.g_tile_status = b.take<unsigned long long>(gt);
+    w.g_counter = b.take<uint32_t>(4);
+    w.e_scan_status = b.take<unsigned long long>(scan_tmp_tiles(w.n_chunks) + 1);
+    w.e_counter  = b.take<uint32_t>(4);
+    w.total_bits = b.take<unsigned long long>(1);
+    w.n_out     = b.take<unsigned long long>(1);
     w.code      = b.take<uint16_t>(g.n + 8);
     w.seg_count = b.take<uint8_t>(g.nseg + 16);
     w.scratch   = b.take<float>(g.nseg * kSegX);
-    size_t gt   = (g.nseg + 4095) / 4096 + 1;
-    w.g_tile_status = b.take<unsigned long long>(gt);
-    w.g_counter = b.take<uint32_t>(4);
     w.g_seg_off = b.take<uint32_t>(g.nseg + 16);
     w.g_tile_base = b.take<unsigned long long>(gt);
-    w.n_out     = b.take<unsigned long long>(1);
     w.build_scratch = b.take<uint8_t>(huff_build_scratch_bytes(dict));
     // codebook block [cb_word dict x u64][info 4 x u32][cb_len dict x u8]: one copy from the host
     // tree builder's staging fills it
@@ -114,13 +119,9 @@ CompressWs layout_compress(const Geometry& g, int dict, uint8_t* base, size_t ca
     w.cb_word    = reinterpret_cast<unsigned long long*>(cb);
     w.build_info = cb ? reinterpret_cast<uint32_t*>(cb + 8 * (size_t)dict) : nullptr;
     w.cb_len     = cb ? cb + 8 * (size_t)dict + 16 : nullptr;
-    w.n_chunks   = (g.n + kChunkSyms - 1) / kChunkSyms;
     w.e_chunk_off   = b.take<unsigned long long>(w.n_chunks + 1);
-    w.e_scan_status = b.take<unsigned long long>(scan_tmp_tiles(w.n_chunks) + 1);
     w.e_edge_idx  = b.take<unsigned long long>(2 * w.n_chunks + 2);
     w.e_edge_bits = b.take<uint32_t>(2 * w.n_chunks + 2);
-    w.e_counter  = b.take<uint32_t>(4);
-    w.total_bits = b.take<unsigned long long>(1);
     w.chunk_bits = b.take<uint16_t>(w.n_chunks + 8);
     w.pad_ws     = b.take<uint8_t>(pad_ws_bytes());
     w.halo_g     = b.take<float>(4);
@@ -149,6 +150,8 @@ struct DecompressWs {
     unsigned long long* scan_status;
     uint32_t* scan_counter;
     unsigned long long* scan_total;
+    unsigned long long* idx_status;   // the index's scan
+    uint32_t* idx_counter;
     unsigned long long* chunk_start;  // index path
     unsigned long long* s_start;      // sync path
     unsigned long long* s_exit_a;
@@ -169,7 +172,17 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
     w.consts   = b.take<Consts>(1);
     w.dq_cache = b.take<unsigned long long>(4);  // offset 256 whatever the field: kept across calls
     w.mm       = b.take<uint32_t>(4);
+    const uint32_t nxs = (g.d0 + 255) / 256;
+    const size_t nsegd = f64 ? g.nrows * nxs : 0, nch = (g.n + kChunkSyms - 1) / kChunkSyms;
+    const size_t nsync = (payload_bytes * 8 + kSyncBits - 1) / kSyncBits + 1;
+    const size_t scan_n = std::max(std::max(nsegd, nch), nsync);
+    // what a call clears, in one piece
     w.status   = b.take<int>(4);
+    w.scan_counter = b.take<uint32_t>(4);
+    w.scan_total   = b.take<unsigned long long>(1);
+    w.scan_status  = b.take<unsigned long long>(scan_tmp_tiles(scan_n) + 1);
+    w.idx_counter  = b.take<uint32_t>(4);
+    w.idx_status   = b.take<unsigned long long>(scan_tmp_tiles(n_index_chunks) + 1);
     w.table    = b.take<uint32_t>(1u << kDecBits);
     w.table2   = b.take<uint32_t>(table2_capacity(maxn));
     w.child    = b.take<uint32_t>(2 * (size_t)maxn);
@@ -179,17 +192,10 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
     w.tinfo    = b.take<uint32_t>(4);
     w.win      = b.take<uint32_t>(n_index_chunks && n_index_chunks <= kSplitMaxChunks ? kWinImageWords : 4);
     w.code     = b.take<uint16_t>(g.n + 8);
-    uint32_t nxs = (g.d0 + 255) / 256;
-    const size_t nsegd = f64 ? g.nrows * nxs : 0, nch = (g.n + kChunkSyms - 1) / kChunkSyms;
     w.seg_zero = b.take<uint32_t>(nsegd + 1);
     w.seg_off  = b.take<unsigned long long>(nsegd + 1);
     w.chunk_zero = b.take<uint32_t>(nch + 1);
     w.chunk_off  = b.take<unsigned long long>(nch + 1);
-    size_t nsync = (payload_bytes * 8 + kSyncBits - 1) / kSyncBits + 1;
-    const size_t scan_n = std::max(std::max(nsegd, nch), nsync);
-    w.scan_status  = b.take<unsigned long long>(scan_tmp_tiles(scan_n) + 1);
-    w.scan_counter = b.take<uint32_t>(4);
-    w.scan_total   = b.take<unsigned long long>(1);
     w.chunk_start  = b.take<unsigned long long>(n_index_chunks + 1);
     w.s_start      = b.take<unsigned long long>(nsync);
     w.s_exit_a     = b.take<unsigned long long>(nsync);
@@ -199,7 +205,7 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
     w.s_changed    = b.take<int>(4);
     {
         const size_t units8 = (size_t)nxs * ((g.d1 + 7) / 8) * ((g.d2 + 7) / 8);  // block-8 warp units
-        w.redo = b.take<uint32_t>(units8 + 2);
+        w.redo = b.take<uint32_t>(units8 + 4);
     }
     w.bytes        = b.off + 256;
     return w;
@@ -208,7 +214,7 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
 // Decode n codes from a Huffman section at d_huff.  Index path when chunk_bits != null.
 int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, size_t tree_bytes, size_t n, int dict,
                  const uint16_t* chunk_bits, size_t n_index_chunks, uint32_t chunk_syms, const DecompressWs& w,
-                 cudaStream_t st) {
+                 bool cleared, cudaStream_t st) {
     const uint8_t* payload   = d_huff + 8 + tree_bytes;
     size_t payload_bytes     = huff_bytes - 8 - tree_bytes;
     unsigned long long pbits = (unsigned long long)payload_bytes * 8ull;
@@ -228,9 +234,12 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     const bool split = chunk_bits && huff_split_applies(n_index_chunks, pbits) && (reinterpret_cast<uintptr_t>(w.win) & 15u) == 0;
     ta.win = split ? w.win : nullptr;
     ta.status = w.status;
+    const bool with_scan = chunk_bits && cleared && node_count > 1;  // tables and index scan in one launch
     {
         StageTimer t(kStDecTable, st);
-        VSZ_TRY(launch_huff_table(ta, st));
+        if (with_scan) VSZ_TRY(launch_huff_table_scan(ta, chunk_bits, w.chunk_start, n_index_chunks, w.idx_status,
+                                                      w.idx_counter, st));
+        else VSZ_TRY(launch_huff_table(ta, st));
     }
     if (node_count == 1) {
         // one-symbol tree: constant output (src/huffman.hh:348-352)
@@ -255,9 +264,9 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     da.tree_info = getenv("VSZ_DECODE_NO_WINDOW") ? nullptr : w.tinfo;
     da.status = w.status;
     if (chunk_bits) {
-        {
+        if (!with_scan) {
             StageTimer t(kStDecScanIndex, st);
-            VSZ_TRY(launch_scan_u16(chunk_bits, w.chunk_start, n_index_chunks, w.scan_status, w.scan_counter, nullptr,
+            VSZ_TRY(launch_scan_u16(chunk_bits, w.chunk_start, n_index_chunks, w.idx_status, w.idx_counter, nullptr,
                                     w.status, st));
         }
         da.start_bit = w.chunk_start;
@@ -860,7 +869,7 @@ vsz_status vsz_huffman_decode(const uint8_t* d_huff, size_t huff_bytes, size_t n
     if (nc == 0 || nc > (uint32_t)(2 * dict_size - 1) || 8 + tree_bytes_size(nc) > huff_bytes) return VSZ_ERR_CORRUPT;
     VSZ_CUDA(cudaMemsetAsync(w.status, 0, sizeof(int), S(stream)));
     // decode into w.code, then copy to the caller (w.code is sized for n)
-    int rc = decode_codes(d_huff, huff_bytes, nc, tree_bytes_size(nc), n, dict_size, nullptr, 0, 0, w, S(stream));
+    int rc = decode_codes(d_huff, huff_bytes, nc, tree_bytes_size(nc), n, dict_size, nullptr, 0, 0, w, false, S(stream));
     if (rc) return rc;
     VSZ_CUDA(cudaMemcpyAsync(d_code, w.code, n * sizeof(uint16_t), cudaMemcpyDeviceToDevice, S(stream)));
     int st = 0;
@@ -954,15 +963,19 @@ vsz_status vsz_compress(const vsz_params* p, int ndim, const size_t dims[3], con
     cudaStream_t st = S(stream);
     const size_t hdr = hdr_bytes(ndim);
     const size_t huff_off = hdr + 4 * npad;  // the Huffman section follows the pad values
-    VSZ_CUDA(cudaMemsetAsync(w.status, 0, sizeof(int), st));
-    VSZ_CUDA(cudaMemsetAsync(w.hist, 0, sizeof(unsigned long long) * nsym, st));
-    VSZ_CUDA(cudaMemsetAsync(w.build_info, 0, 4 * sizeof(uint32_t), st));
-    VSZ_CUDA(cudaMemsetAsync(w.total_bits, 0, sizeof(unsigned long long), st));
-    VSZ_CUDA(cudaMemsetAsync(w.n_out, 0, sizeof(unsigned long long), st));
-    // 1. error-bound family (+ value range for r2r)
+    // 1. cleared words, error-bound family (+ value range for r2r)
     {
         StageTimer t(kStEbSetup, st);
-        VSZ_TRY(launch_eb_setup(p->mode, p->eb, d_in, g.n, w.consts, w.mm, st, w.status));
+        InitArgs in{};
+        in.zero    = reinterpret_cast<uint32_t*>(w.status);
+        in.words   = (size_t)(reinterpret_cast<uint32_t*>(w.n_out) + 2 - in.zero);
+        in.zero4   = w.build_info;
+        in.mode    = p->mode;
+        in.eb      = p->eb;
+        in.consts  = w.consts;
+        in.mm      = w.mm;
+        VSZ_TRY(launch_init(in, st));
+        if (p->mode == VSZ_MODE_R2R) VSZ_TRY(launch_range(p->eb, d_in, g.n, w.consts, w.mm, st, w.status));
     }
     // 1b. padding (-p): pad values into the archive's pad section (and the global halo value)
     DqArgs a = make_dq_args(g, p->block_size, dict, d_in, w.consts, w.code, w.scratch, w.seg_count, w.hist);
@@ -1036,6 +1049,7 @@ vsz_status vsz_compress(const vsz_params* p, int ndim, const size_t dims[3], con
     he.edge_bits = w.e_edge_bits;
     he.status = w.status;
     he.build_info = w.build_info;
+    he.scan_cleared = 1;
     VSZ_TRY(launch_huff_encode(he, st, num_sms()));  // stages huff_count, huff_pack
     // 5. outliers after the bitstream, in row-major order
     GatherArgs ga{};
@@ -1052,7 +1066,7 @@ vsz_status vsz_compress(const vsz_params* p, int ndim, const size_t dims[3], con
     ga.tile_base = w.g_tile_base;
     {
         StageTimer t(kStOutlierGather, st);
-        VSZ_TRY(launch_outlier_gather(ga, st, num_sms()));
+        VSZ_TRY(launch_outlier_gather(ga, st, num_sms(), true));
     }
     // 6. header, result record, trailer with the decode index
     FinalizeArgs f{};
@@ -1263,11 +1277,19 @@ vsz_status vsz_decompress(const vsz_archive_desc* d, const vsz_decompress_opts* 
                                        reinterpret_cast<uint8_t*>(d_ws), ws_bytes);
     if (w.bytes > ws_bytes) return VSZ_ERR_CAPACITY;
     cudaStream_t st = S(stream);
-    VSZ_CUDA(cudaMemsetAsync(w.status, 0, sizeof(int), st));
-    VSZ_TRY(launch_eb_setup(VSZ_MODE_ABS, ebf, nullptr, 0, w.consts, w.mm, st, w.status));
+    {
+        InitArgs in{};
+        in.zero   = reinterpret_cast<uint32_t*>(w.status);
+        in.words  = (size_t)(reinterpret_cast<uint32_t*>(w.table) - in.zero);
+        in.zero4  = w.redo;
+        in.mode   = VSZ_MODE_ABS;
+        in.eb     = ebf;
+        in.consts = w.consts;
+        VSZ_TRY(launch_init(in, st));
+    }
     const uint16_t* idx = d->has_trailer ? reinterpret_cast<const uint16_t*>(d_archive + d->index_offset) : nullptr;
     VSZ_TRY(decode_codes(d_archive + d->huff_offset, d->huff_bytes, d->node_count, d->tree_bytes, g.n, nsym, idx,
-                         d->has_trailer ? d->n_chunks : 0, d->chunk_syms, w, st));
+                         d->has_trailer ? d->n_chunks : 0, d->chunk_syms, w, true, st));
     // the outliers to their elements of the output: the indexed decoders count the zero codes of each
     // chunk, other codes are counted here
     OutlierArgs oa{};
@@ -1286,7 +1308,7 @@ vsz_status vsz_decompress(const vsz_archive_desc* d, const vsz_decompress_opts* 
         StageTimer t(kStZeroScan, st);
         if (!indexed_counts(d)) VSZ_TRY(launch_count_zeros_chunk(w.code, g.n, w.chunk_zero, st, num_sms()));
         VSZ_TRY(launch_scan_u32(w.chunk_zero, w.chunk_off, oa.nchunks, w.scan_status, w.scan_counter, w.scan_total,
-                                w.status, st));
+                                w.status, st, idx != nullptr));  // the sync path's scan has used the words
     }
     {
         StageTimer t(kStOutlierCopy, st);
@@ -1301,6 +1323,7 @@ vsz_status vsz_decompress(const vsz_archive_desc* d, const vsz_decompress_opts* 
     a.n_outliers = d->n_outlier;
     a.status = w.status;
     a.chunk_off = w.chunk_off;
+    a.redo_cleared = 1;
     a.consts = w.consts;
     a.out = d_out;
     a.d0 = g.d0;
@@ -1585,7 +1608,7 @@ vsz_status vsz_decompress_f64(const vsz_archive_desc* d, const uint8_t* d_archiv
                                 reinterpret_cast<unsigned long long*>(w.mm), w.status, st, num_sms()));
     const uint16_t* idx = reinterpret_cast<const uint16_t*>(d_archive + d->index_offset);
     VSZ_TRY(decode_codes(d_archive + d->huff_offset, d->huff_bytes, d->node_count, d->tree_bytes, g.n, dict, idx,
-                         d->n_chunks, d->chunk_syms, w, st));
+                         d->n_chunks, d->chunk_syms, w, false, st));
     {
         StageTimer t(kStZeroScan, st);
         VSZ_TRY(launch_count_zeros(w.code, g.d0, g.nrows, w.seg_zero, st, num_sms()));

@@ -77,6 +77,7 @@ struct HuffEncodeArgs {
     unsigned long long* chunk_off;    // nchunks: first bit of each chunk
     unsigned long long* scan_status;  // scan scratch: scan_tmp_tiles(nchunks) + 1
     uint32_t* scan_counter;
+    int scan_cleared;                 // scan_status and scan_counter are zero already
     unsigned long long* edge_idx;     // 2 nchunks: word index of a chunk's partial first / last word
     uint32_t* edge_bits;              // 2 nchunks: its bits (stored byte order)
     int* status;
@@ -175,10 +176,16 @@ int launch_huff_const(uint16_t* codes, size_t n, const uint32_t* info, const int
 int launch_huff_sync_init(HuffSyncArgs a, cudaStream_t st);
 int launch_huff_sync_round(HuffSyncArgs a, const unsigned long long* exit_in, unsigned long long* exit_out,
                            int* changed, cudaStream_t st);
+// cleared: tile_status and tile_counter are zero already.
 int launch_scan_u16(const uint16_t* in, unsigned long long* out, size_t n, unsigned long long* tile_status,
-                    uint32_t* tile_counter, unsigned long long* total, int* status, cudaStream_t st);
+                    uint32_t* tile_counter, unsigned long long* total, int* status, cudaStream_t st,
+                    bool cleared = false);
 int launch_scan_u32(const uint32_t* in, unsigned long long* out, size_t n, unsigned long long* tile_status,
-                    uint32_t* tile_counter, unsigned long long* total, int* status, cudaStream_t st);
+                    uint32_t* tile_counter, unsigned long long* total, int* status, cudaStream_t st,
+                    bool cleared = false);
+// The decode tables and the exclusive scan of the decode index (tile_status, tile_counter zero).
+int launch_huff_table_scan(HuffTableArgs a, const uint16_t* bits, unsigned long long* start, size_t n,
+                           unsigned long long* tile_status, uint32_t* tile_counter, cudaStream_t st);
 size_t scan_tmp_tiles(size_t n);
 // Test hooks (vsz_debug_*): this unit's look-back spin limit; a scan whose first tile never runs.
 int set_spin_limit_huffman(long long polls);

@@ -169,6 +169,7 @@ struct DqDecArgs {
     int strict;                          // strict archive: outliers are input values (re-prequantized)
     uint32_t xtail;                      // 3D: first scalar-prequant column (d0 & ~7 when d0 % 8), else d0
     PadView pad;                         // padded archive: the halo of each block (vals = pad section)
+    int redo_cleared;                    // redo[0..2] are zero already
     uint32_t* redo;                      // 3D block 8, separable pass: [0] count, then units whose
                                          // values left the exact range (null: reference order only)
     Consts* consts_rw;                   // the same constants when writable: the separable pass of a
@@ -248,6 +249,21 @@ inline void dq_set_narrow(DqArgs& a, int ndim, int bs) {
     a.nyg    = ((a.d1 + 7) / 8 + a.grp - 1) / a.grp;
     a.nunits = (unsigned long long)a.nxt * a.nyg * a.nzb;
 }
+// Clears `words` words at zero and the 4 at zero4 (or null), sets mm (or null) to {0, 0xffffffff, 0} for
+// launch_range (all disjoint) and, in mode abs, computes the constants.
+struct InitArgs {
+    uint32_t* zero;
+    size_t words;
+    uint32_t* zero4;
+    uint32_t* mm;
+    int mode;
+    double eb;
+    Consts* consts;
+};
+int launch_init(const InitArgs& i, cudaStream_t st);
+// r2r: the field's range and the constants; d_mm {0, 0xffffffff, 0} on entry (launch_eb_setup sets it).
+int launch_range(double eb, const float* d_in, size_t n, Consts* d_consts, uint32_t* d_mm, cudaStream_t st,
+                 int* status_word);
 // Planes per 3D unit: block_size halved `halvings` times (and nzb, nunits for it).  dq_zlen_halvings:
 // for a launch whose units number `units` at whole blocks.
 inline void dq_set_zlen(DqArgs& a, int bs, int halvings) {
@@ -259,7 +275,8 @@ int dq_zlen_halvings(unsigned long long units, int bs, int num_sms);
 int launch_eb_setup(int mode, double eb, const float* d_in, size_t n, Consts* d_consts, uint32_t* d_mm,
                     cudaStream_t st, int* status_word = nullptr);
 int launch_dq_compress(DqArgs a, int ndim, int bs, cudaStream_t st, int num_sms);
-int launch_outlier_gather(GatherArgs g, cudaStream_t st, int num_sms = 0);
+// cleared: tile_status and tile_counter are zero already.
+int launch_outlier_gather(GatherArgs g, cudaStream_t st, int num_sms = 0, bool cleared = false);
 
 // Pad values of a field (-p).  Writes the archive's pad section (`arch`, any alignment) and, in
 // global mode, the value the compressor's 2D/3D blocks predict from (`halo_g`).  ws: pad_ws_bytes.
