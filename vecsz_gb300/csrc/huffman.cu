@@ -726,11 +726,183 @@ __device__ __forceinline__ uint32_t win_primary(const uint32_t* table, const uin
 // The decode tables of one field, by the whole CTA (1024 threads; returns are block-uniform).
 constexpr int kTableSmemNodes = 4096;
 
+constexpr uint32_t kNodeLeaf = 0x80000000u;
+static_assert(kTableSmemNodes <= 4096 && kDec2Max <= 8, "16-bit parents, a byte of widths per prefix");
+
+// ... of a tree of up to kTableSmemNodes nodes (dictionaries up to 2048 symbols), with the tree and the
+// primary table in shared memory.  Every primary entry finds its own codeword by walking down the
+// tree (at most 12 steps; filling from the leaves, one thread wrote the up to 2048 entries of a short
+// codeword); depths and codes come from one walk up from each node.  One CTA of a few phases, so what
+// counts is the latency of each: global memory is read once and written at the end (1024 symbols:
+// 25 -> 11 us).
+__device__ __forceinline__ void huff_table_smem(const HuffTableArgs& a, uint32_t nc, int w, const uint8_t* pL,
+                                                const uint8_t* pR, const uint8_t* pC, const uint8_t* pT,
+                                                uint32_t* s_tab, uint32_t* s_node, uint32_t* s_scan, int* s_bad) {
+    constexpr int kPerThread = kTableSmemNodes / 1024, kEntries = (1 << kDecBits) / 1024;
+    __shared__ uint16_t s_parent[kTableSmemNodes];       // parent << 1 | side; 0xffff: none
+    __shared__ uint32_t s_widths[(1 << kDecBits) / 4];   // a byte per prefix: bit r - 1 for a leaf r bits down
+    __shared__ uint32_t s_longest;
+    const uint32_t tid = threadIdx.x;
+    for (uint32_t i = tid; i < nc; i += 1024u) s_parent[i] = 0xffffu;
+    s_widths[tid] = 0u;
+    if (tid == 0) s_longest = 0u;
+    __syncthreads();
+    for (uint32_t i = tid; i < nc; i += 1024u) {
+        const bool leaf  = i != 0 && pT[i] != 0;
+        const uint32_t c = (uint32_t)pC[4 * (size_t)i] | ((uint32_t)pC[4 * (size_t)i + 1] << 8) |
+                           ((uint32_t)pC[4 * (size_t)i + 2] << 16) | ((uint32_t)pC[4 * (size_t)i + 3] << 24);
+        uint32_t l = rd_index(pL + (size_t)i * w, w), r = rd_index(pR + (size_t)i * w, w);
+        if (leaf) {
+            if (c >= (uint32_t)a.dict) *s_bad = 1;
+            l = r = 0;
+        } else if (l == 0 || r == 0 || l >= nc || r >= nc) {
+            // an internal node needs both children (the reference would dereference null)
+            *s_bad = 1;
+            l = r = 0;
+        } else {
+            s_parent[l] = (uint16_t)(i << 1);
+            s_parent[r] = (uint16_t)((i << 1) | 1u);
+        }
+        s_node[i]                  = leaf ? kNodeLeaf | (c & 0xffffu) : l | (r << 16);
+        a.node_sym[i]              = leaf ? 0x80000000u | (c & 0xffffu) : 0u;
+        a.child[2 * (size_t)i]     = l;
+        a.child[2 * (size_t)i + 1] = r;
+    }
+    __syncthreads();
+    if (*s_bad) {
+        if (tid == 0) set_status(a.status, VSZ_ERR_CORRUPT);
+        return;
+    }
+    // primary entries: down the tree
+    uint32_t node[kEntries], val[kEntries], dep[kEntries];
+#pragma unroll
+    for (int k = 0; k < kEntries; k++) {
+        node[k] = 0;
+        dep[k]  = 0;
+        val[k]  = s_node[0];
+    }
+    for (int d = 0; d < kDecBits; d++) {
+#pragma unroll
+        for (int k = 0; k < kEntries; k++) {
+            if (val[k] & kNodeLeaf) continue;
+            const uint32_t bit = ((uint32_t)(k * 1024 + tid) >> (kDecBits - 1 - d)) & 1u;
+            node[k]            = (val[k] >> (16 * bit)) & 0xffffu;
+            val[k]             = s_node[node[k]];
+            dep[k]++;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kEntries; k++)
+        s_tab[k * 1024 + tid] = (val[k] & kNodeLeaf) ? ((val[k] & 0xffffu) << 8) | dep[k] : node[k] << 8;
+    // every node's depth and code: up the tree (depth bounded by 64; 255: unreachable or deeper)
+    uint32_t depth[kPerThread], longest = 0;
+    unsigned long long code[kPerThread];
+#pragma unroll
+    for (int q = 0; q < kPerThread; q++) {
+        const uint32_t i = q * 1024u + tid;
+        depth[q]         = 255u;
+        code[q]          = 0;
+        if (i >= nc) continue;
+        uint32_t cur = i, d = 0;
+        while (cur != 0) {
+            const uint32_t p = s_parent[cur];
+            if (p == 0xffffu || d >= 64) break;
+            code[q] |= (unsigned long long)(p & 1u) << d;
+            d++;
+            cur = p >> 1;
+        }
+        if (cur == 0) depth[q] = d;
+        if (!(s_node[i] & kNodeLeaf)) continue;
+        longest = max(longest, depth[q]);
+        if (depth[q] > (uint32_t)kDecBits && depth[q] <= 64u) {
+            const uint32_t r = depth[q] - kDecBits, pfx = (uint32_t)(code[q] >> r);
+            atomicOr(&s_widths[pfx >> 2], 1u << (8 * (pfx & 3u) + min(r, (uint32_t)kDec2Max) - 1u));
+        }
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if ((tid & 31u) == 0) atomicMax(&s_longest, longest);
+    if (a.walk && a.dict <= 16384) {  // both children of an internal node, for the shared-memory walk
+        auto enc = [&](uint32_t c) -> uint32_t {
+            const uint32_t v = s_node[c];
+            return (v & kNodeLeaf) ? (0x8000u | (v & 0x7fffu)) : c;
+        };
+        for (uint32_t i = tid; i < nc; i += 1024u) {
+            const uint32_t v = s_node[i];
+            a.walk[i] = (v & kNodeLeaf) ? 0u : enc(v & 0xffffu) | (enc(v >> 16) << 16);
+        }
+    }
+    __syncthreads();
+    // offsets of the secondary tables (exclusive scan of 2^w2, kDecBits-bit prefixes in order)
+    static_assert(kEntries == 4, "a thread's prefixes are the bytes of a word of s_widths");
+    const uint32_t wm = s_widths[tid];
+    uint32_t w2[kEntries], mine = 0;
+#pragma unroll
+    for (int k = 0; k < kEntries; k++) {
+        w2[k] = 32u - __clz((wm >> (8 * k)) & 0xffu);
+        mine += w2[k] ? 1u << w2[k] : 0u;
+    }
+    uint32_t total;
+    uint32_t off    = block_exclusive_scan<uint32_t>(mine, s_scan, &total);
+    const bool fits = total <= table2_capacity(a.max_nodes);  // always, by the capacity's construction
+    if (fits) {
+#pragma unroll
+        for (int k = 0; k < kEntries; k++) {
+            if (!w2[k]) continue;
+            s_tab[tid * kEntries + k] = (off << 12) | (w2[k] << 8) | 0x80u;
+            off += 1u << w2[k];
+        }
+        for (uint32_t i = tid; i < total; i += 1024u) a.table2[i] = 0u;  // not a codeword
+    }
+    __syncthreads();
+    // secondary entries -- leaves within w2 bits of their prefix, and walk entries for the internal
+    // nodes w2 bits down (codewords longer than kDecBits + kDec2Max)
+    if (fits) {
+#pragma unroll
+        for (int q = 0; q < kPerThread; q++) {
+            const uint32_t i = q * 1024u + tid;
+            if (i >= nc || depth[q] <= (uint32_t)kDecBits || depth[q] > 64u) continue;
+            const uint32_t r = depth[q] - kDecBits, e = s_tab[(uint32_t)(code[q] >> r)];
+            if (!(e & 0x80u)) continue;
+            const uint32_t wd = (e >> 8) & 0xfu, base = e >> 12;
+            if (r > wd) continue;
+            const uint32_t rel = (uint32_t)(code[q] & ((1ull << r) - 1ull)), v = s_node[i];
+            if (v & kNodeLeaf) {
+                const uint32_t lo = base + (rel << (wd - r)), hi = lo + (1u << (wd - r));
+                for (uint32_t t = lo; t < hi; t++) a.table2[t] = ((v & 0xffffu) << 8) | depth[q];
+            } else if (r == wd) {
+                a.table2[base + rel] = i << 8;
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kEntries; k++) a.table[k * 1024 + tid] = s_tab[k * 1024 + tid];
+    __syncthreads();
+    const uint32_t n2 = fits ? total : 0u;
+    if (a.win) {
+#pragma unroll
+        for (uint32_t k = 0; k < (1u << kWinBits) / 1024u; k++) {
+            const uint32_t i = k * 1024u + tid;
+            a.win[i]         = win_primary(s_tab, a.table2, i);
+        }
+        for (uint32_t i = tid; i < min(n2, (uint32_t)kDec2Smem); i += 1024u) {
+            const uint32_t e = a.table2[i];
+            a.win[(1u << kWinBits) + i] = (e & 0xffu) ? win_entry(e) : 0u;
+        }
+    }
+    if (tid == 0) {
+        a.info[0] = 0;
+        a.info[1] = 0;
+        a.info[2] = s_longest;
+        a.info[3] = n2;
+    }
+}
+
 __device__ __forceinline__ void huff_table_run(const HuffTableArgs& a) {
     const uint8_t* h = a.huff;
     __shared__ uint32_t s_nc;
     __shared__ int s_bad;
-    __shared__ uint32_t s_w2[1 << kDecBits];  // secondary table width per primary prefix
+    __shared__ uint32_t s_tab[1 << kDecBits];  // the primary table; large trees: secondary widths by prefix
+    __shared__ uint32_t s_node[kTableSmemNodes];  // children (left | right << 16) or kNodeLeaf | symbol
     __shared__ uint32_t s_scan[33];
     __shared__ uint32_t s_maxlen;             // longest codeword (255: some leaf deeper than 64)
     if (threadIdx.x == 0) {
@@ -749,17 +921,19 @@ __device__ __forceinline__ void huff_table_run(const HuffTableArgs& a) {
     const uint8_t* pR = pL + (size_t)w * nc;
     const uint8_t* pC = pR + (size_t)w * nc;
     const uint8_t* pT = pC + 4 * (size_t)nc;
-    // nc entries: parent << 1 | side; 0xffffffff = none.  In shared memory for trees of up to
-    // kTableSmemNodes nodes (dictionaries up to 2048 symbols): every node's depth and code come
-    // from a walk up to the root, one dependent read per level, twice.
-    __shared__ uint32_t s_parent[kTableSmemNodes];
-    uint32_t* parent  = nc <= (uint32_t)kTableSmemNodes ? s_parent : a.parent;
-    for (uint32_t i = threadIdx.x; i < nc; i += blockDim.x) parent[i] = 0xffffffffu;
-    for (uint32_t i = threadIdx.x; i < (1u << kDecBits); i += blockDim.x) a.table[i] = 0u;
-    __syncthreads();
     // The reference rebuilds the root as an internal node when nodeCount > 256 and from
     // (C[0], t[0]) otherwise (src/huffman.hh:577,602,627).
     const bool root_leaf = (nc <= 256) && pT[0];
+    if (nc <= (uint32_t)kTableSmemNodes && !root_leaf) {
+        huff_table_smem(a, nc, w, pL, pR, pC, pT, s_tab, s_node, s_scan, &s_bad);
+        return;
+    }
+    uint32_t* s_w2   = s_tab;
+    // nc entries: parent << 1 | side; 0xffffffff = none
+    uint32_t* parent = a.parent;
+    for (uint32_t i = threadIdx.x; i < nc; i += blockDim.x) parent[i] = 0xffffffffu;
+    for (uint32_t i = threadIdx.x; i < (1u << kDecBits); i += blockDim.x) a.table[i] = 0u;
+    __syncthreads();
     for (uint32_t i = threadIdx.x; i < nc; i += blockDim.x) {
         bool leaf = (i == 0) ? root_leaf : (pT[i] != 0);
         uint32_t c = (uint32_t)pC[4 * (size_t)i] | ((uint32_t)pC[4 * (size_t)i + 1] << 8) |
