@@ -1,5 +1,5 @@
 """The device heap replay (k_huff_build) against the host's, on histograms with ties, gaps and long
-chains (totals below 2^44, in 32 bits and beyond), at the heap sizes where its three-level steps end."""
+chains (totals below 2^44, in 32 bits and beyond), at the heap sizes where its levels fill."""
 import ctypes as C
 
 import numpy as np

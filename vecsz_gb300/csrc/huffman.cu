@@ -85,70 +85,207 @@ struct HeapKey {
     }
 };
 
-// The reference's heap, operation for operation (src/huffman.hh:169-192, 248-262), by one thread.
-// Returns the number of nodes created.  Each operation depends on the one before: 20 levels a merge at
-// 65 cycles each.  Slower for 1024 symbols (0.63 ms): three levels a step with their 14 frequencies
-// loaded together (0.74), a warp taking five levels a step by ballots (0.98), two lanes running the two
-// removals of a merge two levels apart (1.39) -- branches and votes cost more than the loads they save.
-template <bool K32>
-__device__ __forceinline__ int heap_replay(BuildWs& w, int nused) {
-    using K  = HeapKey<K32>;
-    int qend = 1;
-    for (int i = 0; i < nused; i++) {  // leaves: qinsert(new_node(freq, i)) in symbol order
-        const unsigned long long key = K::make(w.code[i], (uint32_t)i);
-        const unsigned long long fk  = K::fq(key);
-        int ii = qend++, j;
-        while ((j = ii >> 1)) {
-            const unsigned long long pj = w.heap[j];
-            if (K::fq(pj) <= fk) break;
-            w.heap[ii] = pj;
-            ii         = j;
-        }
-        w.heap[ii] = key;
+// The heap array by address: entry i is at base + 8 i, its children's pair at 2 (base + 8 i) - base.
+// In shared memory the addresses are 32 bits.
+template <bool IN_SMEM>
+struct HeapMem {
+    using Addr = uintptr_t;
+    static __device__ __forceinline__ Addr addr(unsigned long long* p) { return reinterpret_cast<Addr>(p); }
+    static __device__ __forceinline__ unsigned long long load(Addr a) { return *reinterpret_cast<unsigned long long*>(a); }
+    static __device__ __forceinline__ ulonglong2 load2(Addr a) { return *reinterpret_cast<ulonglong2*>(a); }
+    static __device__ __forceinline__ void store(Addr a, unsigned long long v) {
+        *reinterpret_cast<unsigned long long*>(a) = v;
     }
-    int nnodes = nused;
-    // merges: new_node(.., qremove(), qremove()) -- the first removal is the RIGHT child
-    while (qend > 2) {
-        unsigned long long rem[2];
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-            // qremove: the hole sinks along the smaller child (ties: left) to the bottom, then takes
-            // the last element, without sifting it up.  Children of both candidates are loaded one
-            // level ahead.
-            const unsigned long long top = w.heap[1];
-            qend--;
-            const unsigned long long last = w.heap[qend];
-            int i = 1, l = 2;
-            ulonglong2 pr = *reinterpret_cast<const ulonglong2*>(&w.heap[2]);
-            while (l < qend) {
-                const ulonglong2 ga = *reinterpret_cast<const ulonglong2*>(&w.heap[2 * l]);
-                const ulonglong2 gb = *reinterpret_cast<const ulonglong2*>(&w.heap[2 * l + 2]);
-                const bool right    = (l + 1 < qend) && (K::fq(pr.y) < K::fq(pr.x));
-                w.heap[i] = right ? pr.y : pr.x;
-                i         = right ? l + 1 : l;
-                l         = 2 * i;
-                pr        = right ? gb : ga;
-            }
-            w.heap[i] = last;
-            rem[r]    = top;
-        }
-        const int k = nnodes - nused;
-        nnodes++;
-        w.rchild[k] = (int32_t)K::node(rem[0]);
-        w.lchild[k] = (int32_t)K::node(rem[1]);
-        const unsigned long long key = K::make(K::fq(rem[0]) + K::fq(rem[1]), (uint32_t)(nused + k));
-        const unsigned long long fk  = K::fq(key);
-        int ii = qend++, j;
-        while ((j = ii >> 1)) {
-            const unsigned long long pj = w.heap[j];
-            if (K::fq(pj) <= fk) break;
-            w.heap[ii] = pj;
-            ii         = j;
-        }
-        w.heap[ii] = key;
+};
+template <>
+struct HeapMem<true> {
+    using Addr = uint32_t;
+    static __device__ __forceinline__ Addr addr(unsigned long long* p) {
+        return static_cast<uint32_t>(__cvta_generic_to_shared(p));
     }
-    return nnodes;
+    static __device__ __forceinline__ unsigned long long load(Addr a) {
+        unsigned long long v;
+        asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+        return v;
+    }
+    static __device__ __forceinline__ ulonglong2 load2(Addr a) {
+        ulonglong2 v;
+        asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(a) : "memory");
+        return v;
+    }
+    static __device__ __forceinline__ void store(Addr a, unsigned long long v) {
+        asm volatile("st.shared.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+    }
+};
+
+// A removal's hole: its address and its children's pair's.
+template <bool IN_SMEM>
+struct Hole {
+    typename HeapMem<IN_SMEM>::Addr a, kids;
+};
+
+// The hole takes the smaller of its children c (ties: the left) and moves there.
+template <bool K32, bool IN_SMEM>
+__device__ __forceinline__ void heap_sink(Hole<IN_SMEM>& h, typename HeapMem<IN_SMEM>::Addr base, const ulonglong2 c) {
+    using K           = HeapKey<K32>;
+    const auto grands = 2 * h.kids - base;  // the left child's children
+    if constexpr (K32 && IN_SMEM) {
+        const uint32_t fx = (uint32_t)(c.x >> 32), fy = (uint32_t)(c.y >> 32);
+        const uint32_t to = h.a;
+        h.a               = h.kids;
+        h.kids            = grands;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.lt.u32 p, %3, %4;\n\t"
+            "@p add.u32 %1, %1, 16;\n\t"
+            "@p add.u32 %0, %0, 8;\n\t"
+            "@p st.shared.u64 [%2], %5;\n\t"
+            "@!p st.shared.u64 [%2], %6;\n\t}"
+            : "+r"(h.a), "+r"(h.kids)
+            : "r"(to), "r"(fy), "r"(fx), "l"(c.y), "l"(c.x)
+            : "memory");
+    } else {
+        const bool right = K::fq(c.y) < K::fq(c.x);
+        HeapMem<IN_SMEM>::store(h.a, right ? c.y : c.x);
+        h.a    = h.kids + (right ? 8 : 0);
+        h.kids = grands + (right ? 16 : 0);
+    }
 }
+
+// The last step: the hole takes a child if it has one (`end` is the address after the last element's),
+// then it takes `last`.  Returns where that went.
+template <bool K32, bool IN_SMEM>
+__device__ __forceinline__ typename HeapMem<IN_SMEM>::Addr heap_settle(const Hole<IN_SMEM>& h,
+                                                                       typename HeapMem<IN_SMEM>::Addr end,
+                                                                       const ulonglong2 c, unsigned long long last) {
+    using K          = HeapKey<K32>;
+    const bool has   = h.kids < end;
+    const bool right = (h.kids + 8 < end) & (K::fq(c.y) < K::fq(c.x));
+    const auto to    = has ? h.kids + (right ? 8 : 0) : h.a;
+    HeapMem<IN_SMEM>::store(h.a, has ? (right ? c.y : c.x) : last);
+    HeapMem<IN_SMEM>::store(to, last);
+    return to;
+}
+
+// qinsert (src/huffman.hh:169-180) of `key` at the end `ii`.  Entry 0 = 0 stops it at the root.
+template <bool K32, bool IN_SMEM>
+__device__ __forceinline__ void heap_insert(typename HeapMem<IN_SMEM>::Addr base, uint32_t ii, unsigned long long key) {
+    using K                     = HeapKey<K32>;
+    using M                     = HeapMem<IN_SMEM>;
+    const unsigned long long fk = K::fq(key);
+    auto pos                    = base + 8 * ii;
+    for (;;) {
+        const auto up              = base + 8 * (ii >>= 1);
+        const unsigned long long v = M::load(up);
+        if (K::fq(v) <= fk) break;
+        M::store(pos, v);
+        pos = up;
+    }
+    M::store(pos, key);
+}
+
+// The reference's heap, operation for operation (src/huffman.hh:169-192, 248-262), by one thread.
+// qremove: the hole sinks along the smaller child (ties: left) to the bottom, then takes the last
+// element, without sifting it up; so its way down doesn't depend on that element, and the two
+// removals of a merge go down together, the second two levels behind the first (it reads a level when
+// that has its final values).  The time is that of one thread's dependent instructions, about 800
+// cycles a merge: levels unrolled, addresses and not indexes carried along, no branch for the last
+// level.  60 fields of up to 1024 symbols, slowest tree: 0.45 ms; slower were one removal after the
+// other with loads a level ahead (0.64), three levels a step with their 14 frequencies loaded together
+// (0.74), a warp taking five levels a step by ballots (0.98), two lanes with a removal each (1.39).
+template <bool K32, bool IN_SMEM>
+struct HeapReplay {
+    using K    = HeapKey<K32>;
+    using M    = HeapMem<IN_SMEM>;
+    using Addr = typename M::Addr;
+    Addr base;
+    uint32_t q1;  // the last element
+    int nnodes;
+    int32_t *rc, *lc;
+
+    // new_node(.., qremove(), qremove()) -- the first removal is the RIGHT child -- and its qinsert
+    __device__ __forceinline__ void join(unsigned long long top1, unsigned long long top2) {
+        *rc++ = (int32_t)K::node(top1);
+        *lc++ = (int32_t)K::node(top2);
+        heap_insert<K32, IN_SMEM>(base, q1 - 1u, K::make(K::fq(top1) + K::fq(top2), (uint32_t)nnodes));
+        nnodes++;
+        q1--;
+    }
+
+    // Merges while a hole of the second removal has two children on `full` levels from the root
+    // (q1 - 1 >= 2 << full), full >= 2; a constant for LEVELS > 0.
+    template <int LEVELS>
+    __device__ __forceinline__ void merges(int levels) {
+        const int full       = LEVELS > 0 ? LEVELS : levels;
+        const uint32_t least = 2u << full;  // of q1 - 1
+        while (q1 > least) {
+            const Addr aq1 = base + 8 * q1, aq2 = aq1 - 8;
+            Hole<IN_SMEM> h1{base + 8, base + 16}, h2 = h1;
+            const unsigned long long top1 = M::load(base + 8), last1 = M::load(aq1), old2 = M::load(aq2);
+            // levels 0 .. full - 1 have both children below q1 - 1, the next has some, then there are none
+            const ulonglong2 c23 = M::load2(base + 16), c45 = M::load2(base + 32), c67 = M::load2(base + 48);
+            const bool right     = K::fq(c23.y) < K::fq(c23.x);
+            const unsigned long long top2 = right ? c23.y : c23.x;
+            heap_sink<K32, IN_SMEM>(h1, base, c23);
+            heap_sink<K32, IN_SMEM>(h1, base, right ? c67 : c45);
+#pragma unroll
+            for (int s = 2; s < full; s++) {
+                const ulonglong2 c1 = M::load2(h1.kids), c2 = M::load2(h2.kids);
+                heap_sink<K32, IN_SMEM>(h1, base, c1);
+                heap_sink<K32, IN_SMEM>(h2, base, c2);
+            }
+            const ulonglong2 c1 = M::load2(h1.kids), c2 = M::load2(h2.kids);
+            const Addr to1 = heap_settle<K32, IN_SMEM>(h1, aq1, c1, last1);
+            heap_sink<K32, IN_SMEM>(h2, base, c2);
+            heap_sink<K32, IN_SMEM>(h2, base, M::load2(h2.kids));
+            heap_settle<K32, IN_SMEM>(h2, aq2, M::load2(h2.kids), to1 == aq2 ? last1 : old2);
+            join(top1, top2);
+        }
+    }
+
+    __device__ __forceinline__ unsigned long long remove(uint32_t q) {  // q: the last element
+        const unsigned long long top = M::load(base + 8), last = M::load(base + 8 * q);
+        uint32_t i = 1;
+        for (uint32_t l = 2; l < q; l = 2 * i) {
+            const unsigned long long x = M::load(base + 8 * l), y = M::load(base + 8 * l + 8);
+            const bool right = l + 1 < q && K::fq(y) < K::fq(x);
+            M::store(base + 8 * i, right ? y : x);
+            i = l + (right ? 1u : 0u);
+        }
+        M::store(base + 8 * i, last);
+        return top;
+    }
+
+    // Returns the number of nodes created.
+    __device__ __forceinline__ int run(const BuildWs& w, int nused) {
+        base   = M::addr(w.heap);
+        rc     = w.rchild;
+        lc     = w.lchild;
+        nnodes = nused;
+        q1     = (uint32_t)nused;
+        // leaves: qinsert(new_node(freq, i)) in symbol order
+        unsigned long long f = w.code[0];
+        for (int i = 0; i < nused; i++) {
+            const unsigned long long key = K::make(f, (uint32_t)i);
+            f                            = w.code[i + 1];  // w.code has twice the entries
+            heap_insert<K32, IN_SMEM>(base, (uint32_t)i + 1u, key);
+        }
+        for (int full = 30 - __clz(nused); full > 9; full--) merges<0>(full);
+        merges<9>(0);
+        merges<8>(0);
+        merges<7>(0);
+        merges<6>(0);
+        merges<5>(0);
+        merges<4>(0);
+        merges<3>(0);
+        merges<2>(0);
+        while (q1 > 1u) {
+            const unsigned long long top1 = remove(q1), top2 = remove(q1 - 1u);
+            join(top1, top2);
+        }
+        return nnodes;
+    }
+};
 
 template <bool IN_SMEM>
 __device__ __forceinline__ void build_field(const HuffBuildArgs& a, uint8_t* s_build_dyn) {
@@ -202,8 +339,8 @@ __device__ __forceinline__ void build_field(const HuffBuildArgs& a, uint8_t* s_b
         int nnodes = nused, fail = 0;
         if (nused == 0) fail = VSZ_ERR_INVALID;
         else if (total >= (1ull << (64 - kKeyShift))) fail = VSZ_ERR_UNSUPPORTED;
-        else if (total < (1ull << 32)) nnodes = heap_replay<true>(w, nused);
-        else nnodes = heap_replay<false>(w, nused);
+        else if (total < (1ull << 32)) nnodes = HeapReplay<true, IN_SMEM>{}.run(w, nused);
+        else nnodes = HeapReplay<false, IN_SMEM>{}.run(w, nused);
         const uint32_t node_count = fail ? 0u : (uint32_t)nnodes;
         s_fail    = fail;
         s_info[0] = node_count;
