@@ -1775,12 +1775,12 @@ template <bool WALK_SMEM>
 __global__ void __launch_bounds__(256) k_huff_decode_idx(HuffDecodeArgs a) {
     __shared__ IdxSmem sm;
     extern __shared__ uint32_t s_walk[];  // WALK_SMEM: a.nodes entries
+    if (a.tree_info && a.tree_info[2] <= (uint32_t)kWinMaxLen) return;  // k_huff_decode_win's trees
     for (int i = threadIdx.x; i < (1 << kDecBits); i += blockDim.x) sm.table[i] = a.table[i];
     if (WALK_SMEM)
         for (uint32_t i = threadIdx.x; i < a.nodes; i += blockDim.x) s_walk[i] = a.walk[i];
     __syncthreads();
     if (*a.status != VSZ_OK) return;
-    if (a.tree_info && a.tree_info[2] <= (uint32_t)kWinMaxLen) return;  // k_huff_decode_win's trees
     decode_idx_lane<WALK_SMEM>(a, blockIdx.x * (size_t)blockDim.x + threadIdx.x, sm, s_walk);
 }
 
