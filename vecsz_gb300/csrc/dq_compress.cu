@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "api_common.cuh"
+#include "huff_build.cuh"
 #include "scan.cuh"
 #include "vsz_device.cuh"
 #include "vsz_kernels.h"
@@ -634,18 +635,26 @@ __global__ void __launch_bounds__(256) k_dq_compress_1d(DqArgs a) {
     hist_flush_block(a, s_hist, h);
 }
 
+// A call of its own, so that its registers don't add to the dual-quant's.
+__device__ __noinline__ void build_field_call(const HuffBuildArgs* b, uint8_t* s_dyn) { build_field<true>(*b, s_dyn); }
+
 // Many fields in one launch: block-wide tasks (one field, a range of its warp units), each taken
 // by the next free block (`next`: the launch's task counter, zero at launch), so that blocks do
 // not idle behind uneven tasks.  Fields of every dimensionality and alignment share the launch (the
 // task names its class): a launch per class ran one after another, most of them too small to fill
 // the GPU (60 mixed fields: 8 launches, 1.37 ms).  hist_words = shared-memory histogram words
 // reserved before the planes.
+//
+// The CTA that finishes a field's last unit builds the field's tree (a.build), one thread's work for up
+// to 0.45 ms that runs beside the other CTAs' dual-quant: 60 mixed fields 600 us for both, in a launch
+// after this one 270 + 438.
 template <int BS>
 __global__ void __launch_bounds__(256, 3)
     k_dq_compress_batch(const DqArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks,
                         uint32_t hist_words, uint32_t* __restrict__ next) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
     __shared__ uint32_t s_task;
+    __shared__ bool s_last;
     PrevRows* s_prev = reinterpret_cast<PrevRows*>(s_dyn + hist_words);
     for (uint32_t t = dq_block_next_task(next, &s_task); t < ntasks; t = dq_block_next_task(next, &s_task)) {
         const BatchTask tk = tasks[t];
@@ -686,6 +695,17 @@ __global__ void __launch_bounds__(256, 3)
         }
         hist_flush_block(a, s_hist, h);
         __syncthreads();  // the next task reuses shared memory
+        if (a.build) {
+            if (threadIdx.x == 0) {
+                const uint32_t units = (uint32_t)(tk.u1 - tk.u0);
+                __threadfence();
+                s_last = atomicAdd(a.done, units) + units == (uint32_t)a.nunits;
+                __threadfence();
+            }
+            __syncthreads();
+            if (s_last) build_field_call(a.build, reinterpret_cast<uint8_t*>(s_dyn));
+            __syncthreads();
+        }
     }
 }
 
@@ -1086,14 +1106,15 @@ int launch_consts_batch(const ConstsField* f, uint32_t nfields, cudaStream_t st)
 }
 
 int launch_dq_compress_batch(const DqArgs* args, const BatchTask* tasks, uint32_t ntasks, int bs, bool any3d,
-                             uint32_t hist_words, uint32_t* next, cudaStream_t st, int num_sms) {
+                             uint32_t hist_words, size_t build_ws, uint32_t* next, cudaStream_t st, int num_sms) {
     if (ntasks == 0) return VSZ_OK;
-    const size_t smem   = (size_t)hist_words * sizeof(uint32_t) + (any3d ? sizeof(PrevRows) * 8 : 0);
+    const size_t dq     = (size_t)hist_words * sizeof(uint32_t) + (any3d ? sizeof(PrevRows) * 8 : 0);
+    const size_t smem   = dq > build_ws ? dq : build_ws;
     const uint32_t cap  = (uint32_t)num_sms * 3u;
     const uint32_t grid = ntasks < cap ? ntasks : cap;
     static std::atomic<unsigned long long> attr[4];
     auto go = [&](auto kern, std::atomic<unsigned long long>& at) {
-        smem_limit_once(kern, kDqSmemMax, at);
+        smem_limit_once(kern, kDqSmemMax > (int)kDqBuildWs ? kDqSmemMax : (int)kDqBuildWs, at);
         kern<<<grid, 256, smem, st>>>(args, tasks, ntasks, hist_words, next);
     };
     switch (bs) {

@@ -33,8 +33,16 @@ constexpr size_t kCtlInfo    = 80;   // u32[4] tree info
 constexpr size_t kCtlBits    = 96;   // u64 payload bits
 constexpr size_t kCtlNOut    = 104;  // u64 outliers
 constexpr size_t kCtlTicket  = 112;  // u32 gather look-back ticket
+constexpr size_t kCtlDqDone  = 116;  // u32 finished dual-quant units
 // after the per-field records: the batch status, then one dual-quant task counter per block size
 constexpr size_t kDqNextOff  = 64;
+// The trees of a batch are built while its dual-quant still runs, so the fields with the longest ones
+// (tight bounds) come first, in four parts by bound, within a part by kernel class.  60 mixed fields,
+// dual-quant and trees: one part 624 us, two or four 600, 14 632, 60 643.
+constexpr size_t kDqEbGroups = 4;
+// Tasks per CTA the dual-quant stage holds (at least one unit per warp each): small ones, so that a
+// field is complete soon after it was begun (4: 800 us, 6: 698, 8: 600, more: the same).
+constexpr uint64_t kDqTasks = 8;
 
 // Work per task (vsz_batch_autotune searches the first two): dual-quant warp units and encoder chunks
 // (at most these many by default, fewer where the batch would not fill the GPU), min/max elements.
@@ -48,6 +56,7 @@ struct DqGroup {  // the fields of one block size
     bool any3d;
     uint32_t hist_words;
     uint32_t task_off, ntasks;
+    size_t build_ws;  // shared memory of the largest tree built within the launch
 };
 
 }  // namespace
@@ -68,7 +77,8 @@ struct vsz_batch {
     // launch plan
     uint32_t minmax_off = 0, minmax_n = 0;
     std::vector<DqGroup> dq_groups;
-    uint32_t build_smem_n = 0;  // fields [0, build_smem_n) of `build` use the shared-memory builder
+    // `build`: the trees built within the dual-quant launch, by the shared-memory builder, the others
+    uint32_t build_dq_n = 0, build_smem_n = 0;
     int build_dict_max = 0;
     uint32_t enc_off = 0, enc_n = 0;
     int cb_dict_max = 0;
@@ -216,10 +226,10 @@ int upload_tasks(vsz_batch* B) {
         if (B->minmax_units[f]) add_tasks(tasks, f, B->minmax_units[f], kMinmaxPerTask);
     B->minmax_n = (uint32_t)tasks.size();
     B->dq_groups.clear();
-    // default task sizes: a few tasks for each CTA the stage can hold, so that the last ones to finish
+    // default task sizes: some tasks for each CTA the stage can hold, so that the last ones to finish
     // leave little idle (8 units: one for each warp of the block)
-    auto per_task = [&](uint64_t set, uint64_t units, uint64_t ctas, uint64_t most) {
-        return set ? set : std::max<uint64_t>(8, std::min<uint64_t>(most, units / (4 * ctas) / 8 * 8));
+    auto per_task = [&](uint64_t set, uint64_t units, uint64_t tasks, uint64_t most) {
+        return set ? set : std::max<uint64_t>(8, std::min<uint64_t>(most, units / tasks / 8 * 8));
     };
     const uint64_t sms = (uint64_t)num_sms();
     for (auto& kv : B->classes) {
@@ -227,13 +237,13 @@ int upload_tasks(vsz_batch* B) {
         grp.task_off = (uint32_t)tasks.size();
         uint64_t units = 0;
         for (uint32_t f : kv.second) units += B->dq_units[f];
-        const uint64_t per = per_task(B->dq_per, units, 3 * sms, kDqUnitsPerTask);
+        const uint64_t per = per_task(B->dq_per, units, kDqTasks * 3 * sms, kDqUnitsPerTask);
         for (uint32_t f : kv.second) add_tasks(tasks, f, B->dq_units[f], per, B->dq_class[f]);
         grp.ntasks = (uint32_t)tasks.size() - grp.task_off;
         B->dq_groups.push_back(grp);
     }
     B->enc_off = (uint32_t)tasks.size();
-    const uint64_t enc_per = per_task(B->enc_per, B->total_chunks, 4 * sms, kEncChunksPerTask);
+    const uint64_t enc_per = per_task(B->enc_per, B->total_chunks, 4 * 4 * sms, kEncChunksPerTask);
     for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, B->enc_units[f], enc_per);
     B->enc_n      = (uint32_t)tasks.size() - B->enc_off;
     B->gather_off = (uint32_t)tasks.size();
@@ -286,7 +296,8 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
     std::vector<HuffEncodeArgs> enc(nf);
     std::vector<GatherArgs> ga(nf);
     std::vector<FinalizeArgs> fin(nf);
-    std::vector<HuffBuildArgs> build_smem, build_glob;
+    std::vector<HuffBuildArgs> build_dq, build_smem, build_glob;
+    std::vector<uint32_t> build_dq_field;
     vsz_batch* B = new vsz_batch();
     B->nfields   = nfields;
     cudaGetDevice(&B->device);
@@ -323,7 +334,12 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
         hb.info    = info;
         hb.scratch = L.build_scratch[f];
         hb.status  = status;
-        if (huff_build_in_smem(dict)) {
+        if (huff_build_scratch_bytes(dict) <= kDqBuildWs) {
+            hb.ws_in_smem = 1;
+            build_dq.push_back(hb);
+            build_dq_field.push_back(f);
+            dq[f].done = reinterpret_cast<uint32_t*>(ctl + kCtlDqDone);
+        } else if (huff_build_in_smem(dict)) {
             hb.ws_in_smem = 1;
             build_smem.push_back(hb);
             B->build_dict_max = std::max(B->build_dict_max, dict);
@@ -409,21 +425,32 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
         B->copy_units.push_back(g.nseg);
     }
     for (auto& kv : classes) {
-        // kernel class by kernel class, so that blocks on the GPU together run the same code
-        std::stable_sort(kv.second.begin(), kv.second.end(),
-                         [&](uint32_t a, uint32_t b) { return B->dq_class[a] > B->dq_class[b]; });
+        // by parts of tighter bounds first, then kernel class by kernel class, so that blocks on the GPU
+        // together run the same code
+        std::vector<uint32_t> by = kv.second;
+        auto eb = [&](uint32_t f) { return fg[f].r2r ? fg[f].p.eb : 0.0; };
+        std::stable_sort(by.begin(), by.end(), [&](uint32_t a, uint32_t b) { return eb(a) < eb(b); });
+        const size_t per = (by.size() + kDqEbGroups - 1) / kDqEbGroups;
+        std::vector<size_t> part(nf);
+        for (size_t i = 0; i < by.size(); i++) part[by[i]] = i / per;
+        std::stable_sort(kv.second.begin(), kv.second.end(), [&](uint32_t a, uint32_t b) {
+            return part[a] != part[b] ? part[a] < part[b] : B->dq_class[a] > B->dq_class[b];
+        });
         DqGroup grp{};
         grp.bs = kv.first;
         for (uint32_t f : kv.second) {
             if (dq[f].smem_hist) grp.hist_words = std::max(grp.hist_words, (uint32_t)((dq[f].dict + 3) & ~3));
             grp.any3d = grp.any3d || fg[f].g.ndim == 3;
+            if (dq[f].done) grp.build_ws = std::max(grp.build_ws, huff_build_scratch_bytes(dq[f].dict));
         }
         B->classes.emplace_back(grp, kv.second);
     }
     B->total_chunks = L.chunk_base.empty() ? 0 : L.chunk_base.back() + fg.back().nch;
     // ---- upload
-    std::vector<HuffBuildArgs> build = build_smem;
+    std::vector<HuffBuildArgs> build = build_dq;
+    build.insert(build.end(), build_smem.begin(), build_smem.end());
     build.insert(build.end(), build_glob.begin(), build_glob.end());
+    B->build_dq_n   = (uint32_t)build_dq.size();
     B->build_smem_n = (uint32_t)build_smem.size();
     size_t off = 0;
     auto place = [&](size_t bytes) {
@@ -440,7 +467,6 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
     std::vector<uint8_t> h(table_bytes, 0);
     memcpy(h.data() + o_mm, mm.data(), sizeof(MinmaxField) * nf);
     memcpy(h.data() + o_cs, cs.data(), sizeof(ConstsField) * nf);
-    memcpy(h.data() + o_dq, dq.data(), sizeof(DqArgs) * nf);
     memcpy(h.data() + o_bd, build.data(), sizeof(HuffBuildArgs) * nf);
     memcpy(h.data() + o_en, enc.data(), sizeof(HuffEncodeArgs) * nf);
     memcpy(h.data() + o_ga, ga.data(), sizeof(GatherArgs) * nf);
@@ -449,6 +475,9 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
         delete B;
         return VSZ_ERR_NOMEM;
     }
+    for (size_t i = 0; i < build_dq.size(); i++)
+        dq[build_dq_field[i]].build = reinterpret_cast<const HuffBuildArgs*>(B->d_tables + o_bd) + i;
+    memcpy(h.data() + o_dq, dq.data(), sizeof(DqArgs) * nf);
     if (cudaMemcpy(B->d_tables, h.data(), table_bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaFree(B->d_tables);
         delete B;
@@ -559,14 +588,15 @@ vsz_status vsz_batch_compress(vsz_batch* B, void* stream) {
         for (size_t i = 0; i < B->dq_groups.size(); i++) {
             const DqGroup& g = B->dq_groups[i];
             VSZ_TRY(launch_dq_compress_batch(B->dq, B->tasks + g.task_off, g.ntasks, g.bs, g.any3d, g.hist_words,
-                                             next + i, st, sms));
+                                             g.build_ws, next + i, st, sms));
         }
     }
     {
         StageTimer t(kStHuffBuild, st);
         huff_build_prepare();
-        VSZ_TRY(launch_huff_build_batch(B->build, B->build_smem_n, true, B->build_dict_max, st, sms));
-        VSZ_TRY(launch_huff_build_batch(B->build + B->build_smem_n, nf - B->build_smem_n, false, 0, st, sms));
+        const HuffBuildArgs* rest = B->build + B->build_dq_n;
+        VSZ_TRY(launch_huff_build_batch(rest, B->build_smem_n, true, B->build_dict_max, st, sms));
+        VSZ_TRY(launch_huff_build_batch(rest + B->build_smem_n, nf - B->build_dq_n - B->build_smem_n, false, 0, st, sms));
     }
     VSZ_TRY(launch_huff_encode_batch(B->enc, nf, B->tasks + B->enc_off, B->enc_n, B->cb_dict_max, B->all_bits,
                                      B->all_off, B->total_chunks, B->scan_status, B->scan_counter, B->batch_status,

@@ -160,7 +160,7 @@ int launch_huff_encode_batch(const HuffEncodeArgs* args, uint32_t nfields, const
                              cudaStream_t st, int num_sms);
 void huff_encode_prepare(HuffEncodeArgs& a);
 void huff_build_prepare();  // one-time kernel attributes of launch_huff_build (call outside capture)
-size_t huff_build_scratch_bytes(int dict);
+size_t huff_build_scratch_bytes(int dict);  // also the shared memory of a build there
 int launch_huff_encode(HuffEncodeArgs a, cudaStream_t st, int num_sms);
 int launch_huff_table(HuffTableArgs a, cudaStream_t st);
 // Many fields: decode tables one CTA per field; decoding over tasks of (field, 256-chunk range

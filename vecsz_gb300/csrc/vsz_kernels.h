@@ -9,6 +9,8 @@
 
 namespace vsz {
 
+struct HuffBuildArgs;
+
 struct Consts;
 
 // A byte offset known only on the device once earlier kernels ran (tree size, payload size):
@@ -110,6 +112,9 @@ struct DqArgs {
     unsigned long long nunits;   // warp work units
     int strict;                  // strict error-bound mode (outliers carry input values)
     PadView pad;                 // padding (-p): the halo each block predicts from
+    const HuffBuildArgs* build;  // batch: the field's tree, built by the CTA that finishes its last unit
+                                 // (null: by a launch of its own), and its count of finished units
+    uint32_t* done;
 };
 
 struct GatherArgs {
@@ -304,8 +309,11 @@ inline uint32_t dq_class_of(int ndim, bool vec, bool tail, bool narrow) {
 }
 int launch_minmax_batch(const MinmaxField* f, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st, int num_sms);
 int launch_consts_batch(const ConstsField* f, uint32_t nfields, cudaStream_t st);
+// Working sets of tree builds up to this size (dictionaries up to 1024) fit into shared memory beside
+// the dual-quant's three CTAs per SM.
+constexpr size_t kDqBuildWs = 72 * 1024;
 int launch_dq_compress_batch(const DqArgs* args, const BatchTask* tasks, uint32_t ntasks, int bs, bool any3d,
-                             uint32_t hist_words, uint32_t* next, cudaStream_t st, int num_sms);
+                             uint32_t hist_words, size_t build_ws, uint32_t* next, cudaStream_t st, int num_sms);
 int launch_outlier_gather_batch(const GatherArgs* args, const BatchTask* tasks, uint32_t ntasks, cudaStream_t st,
                                 int num_sms);
 // ... then the values, by tasks of (field, segment range) (kCopySegs segments a CTA).
