@@ -135,8 +135,8 @@ __global__ void __launch_bounds__(256) k_minmax(const float* __restrict__ x, siz
 }
 
 // What a call needs cleared, and the constants of an absolute bound (mode abs), in one launch: a
-// stream's small memsets cost 2 us each, and a compress had eleven of them, a decompress six (64^3: 95
-// -> 74 and 88 -> 67 us).
+// stream's small memsets cost 2 us each, and a compress had eleven of them, a decompress six (64^3: 93
+// -> 80 and 88 -> 75 us).
 __global__ void __launch_bounds__(256) k_init(InitArgs i) {
     const size_t t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
     for (size_t k = t0; k < i.words; k += step) i.zero[k] = 0u;

@@ -792,8 +792,8 @@ void dq_w8_geometry(DqDecArgs& a) { a.nunits = (unsigned long long)((a.nbx8 + 3)
 bool dq_w8_applies(const DqDecArgs& a, int ndim) {
     if (ndim != 3 || a.pad.vals || a.n > kW8MaxN) return false;
     if (getenv("VSZ_DQ_NO_WAVEFRONT") != nullptr) return false;
-    // the separable pass catches up with the wavefront between 160^3 and 256^3 (measured: 0.123
-    // vs 0.060 ms at 160^3, 0.099 vs 0.127 ms at 256^3, zero scans included)
+    // the separable pass catches up with the wavefront between 256x256x128 (82 us against 45) and 256^3
+    // (59 against 65); the reference-order pass over aligned rows at 384x384x256 (163 against 171)
     return a.n <= kW8MaxSeparableN || !dq_b8_separable(a, ndim);
 }
 

@@ -456,8 +456,8 @@ static_assert(kTableSmemNodes <= 4096 && kDec2Max <= 8, "16-bit parents, a byte 
 // primary table in shared memory.  Every primary entry finds its own codeword by walking down the
 // tree (at most 12 steps; filling from the leaves, one thread wrote the up to 2048 entries of a short
 // codeword); depths and codes come from one walk up from each node.  One CTA of a few phases, so what
-// counts is the latency of each: global memory is read once and written at the end (1024 symbols:
-// 25 -> 11 us).
+// counts is the latency of each: global memory is read once and written at the end (with the index
+// scan beside it, 1024 symbols: 25 -> 19 us, 295: 16.5 -> 12).
 __device__ __forceinline__ void huff_table_smem(const HuffTableArgs& a, uint32_t nc, int w, const uint8_t* pL,
                                                 const uint8_t* pR, const uint8_t* pC, const uint8_t* pT,
                                                 uint32_t* s_tab, uint32_t* s_node, uint32_t* s_scan, int* s_bad) {
@@ -1889,7 +1889,7 @@ int launch_huff_encode_batch(const HuffEncodeArgs* args, uint32_t nfields, const
         k_huff_count_batch<<<grid, kEncThreads, (size_t)cb_dict_max, st>>>(args, tasks, ntasks);
         count_launch();
         int rc = launch_scan_u16(all_bits, all_off, total_chunks, scan_status, scan_counter, all_off + total_chunks,
-                                 batch_status, st);
+                                 batch_status, st, true);
         if (rc) return rc;
         k_field_bits<<<(nfields + 127) / 128, 128, 0, st>>>(args, nfields, batch_status);
         count_launch();

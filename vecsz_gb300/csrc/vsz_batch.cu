@@ -91,13 +91,9 @@ struct vsz_batch {
     std::vector<uint64_t> minmax_units, dq_units, enc_units, gather_units, copy_units;  // per field
     std::vector<uint32_t> dq_class;
     std::vector<std::pair<DqGroup, std::vector<uint32_t>>> classes;
-    // workspace regions zeroed per call
+    // workspace region cleared per call: control words, histograms, look-back status
     uint8_t* ctl = nullptr;
-    size_t ctl_bytes = 0;
-    unsigned long long* hist = nullptr;
-    size_t hist_bytes = 0;
-    unsigned long long* gstatus = nullptr;
-    size_t gstatus_bytes = 0;
+    size_t cleared = 0;
     uint16_t* all_bits = nullptr;
     unsigned long long* all_off = nullptr;
     unsigned long long* scan_status = nullptr;
@@ -113,6 +109,14 @@ struct FieldGeom {
     size_t nch, ntiles;
     bool r2r;
 };
+
+// The region cleared per call, in one launch (six small memsets took 2 us each); the {max, min} keys of
+// a field's range start at {0, 0xffffffff}.
+__global__ void __launch_bounds__(256) k_batch_init(unsigned long long* ctl, size_t words, uint32_t nfields) {
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < words; i += step)
+        ctl[i] = i < (size_t)nfields * (kCtlBytes / 8) && i % (kCtlBytes / 8) == kCtlMm / 8 ? 0xffffffff00000000ull : 0ull;
+}
 
 // The workspace layout, measured (base == nullptr) or carved.
 struct BatchLayout {
@@ -134,6 +138,7 @@ struct BatchLayout {
     std::vector<uint32_t*> seg_off;               // gather: offsets of the segments in their tiles
     std::vector<unsigned long long*> tile_base;   // and the tiles' first outliers
     std::vector<size_t> hist_off, gstat_off, chunk_base;
+    size_t cleared;
     size_t bytes;
 };
 
@@ -154,10 +159,11 @@ BatchLayout layout_batch(const std::vector<FieldGeom>& fg, uint8_t* base, size_t
     }
     L.hist         = b.take<unsigned long long>(hwords);
     L.gstatus      = b.take<unsigned long long>(gwords);
-    L.all_bits     = b.take<uint16_t>(chunks + 8);
-    L.all_off      = b.take<unsigned long long>(chunks + 1);
     L.scan_status  = b.take<unsigned long long>(scan_tmp_tiles(chunks) + 1);
     L.scan_counter = b.take<uint32_t>(4);
+    L.cleared      = b.off;  // ctl to here is cleared per call
+    L.all_bits     = b.take<uint16_t>(chunks + 8);
+    L.all_off      = b.take<unsigned long long>(chunks + 1);
     for (const auto& f : fg) {
         L.code.push_back(b.take<uint16_t>(f.g.n + 8));
         L.seg_count.push_back(b.take<uint8_t>(f.g.nseg + 16));
@@ -491,14 +497,8 @@ vsz_status vsz_batch_create(const vsz_batch_field* fields, int nfields, void* d_
     B->gather = reinterpret_cast<const GatherArgs*>(B->d_tables + o_ga);
     B->fin    = reinterpret_cast<const FinalizeArgs*>(B->d_tables + o_fi);
     B->ctl           = L.ctl;
-    B->ctl_bytes     = (size_t)nf * kCtlBytes + 256;
-    B->batch_status  = L.batch_status;
-    B->hist          = L.hist;
-    B->hist_bytes    = 0;
-    for (uint32_t f = 0; f < nf; f++) B->hist_bytes += 8 * (size_t)fg[f].p.dict_size;
-    B->gstatus       = L.gstatus;
-    B->gstatus_bytes = 0;
-    for (uint32_t f = 0; f < nf; f++) B->gstatus_bytes += 8 * (fg[f].ntiles + 1);
+    B->cleared      = L.cleared;
+    B->batch_status = L.batch_status;
     B->all_bits     = L.all_bits;
     B->all_off      = L.all_off;
     B->scan_status  = L.scan_status;
@@ -573,10 +573,10 @@ vsz_status vsz_batch_compress(vsz_batch* B, void* stream) {
     const uint32_t nf = (uint32_t)B->nfields;
     // control words (status, tree info, sizes, tickets, the batch status) to zero, the min key
     // of every field to 0xffffffff; histograms and look-back status to zero
-    VSZ_CUDA(cudaMemsetAsync(B->ctl, 0, B->ctl_bytes, st));
-    VSZ_CUDA(cudaMemset2DAsync(B->ctl + kCtlMm + 4, kCtlBytes, 0xff, 4, nf, st));
-    VSZ_CUDA(cudaMemsetAsync(B->hist, 0, B->hist_bytes, st));
-    VSZ_CUDA(cudaMemsetAsync(B->gstatus, 0, B->gstatus_bytes, st));
+    const size_t words = B->cleared / 8;
+    k_batch_init<<<(unsigned)std::min<size_t>((words + 1023) / 1024, (size_t)sms * 8), 256, 0, st>>>(
+        reinterpret_cast<unsigned long long*>(B->ctl), words, nf);
+    count_launch();
     {
         StageTimer t(kStEbSetup, st);
         VSZ_TRY(launch_minmax_batch(B->minmax, B->tasks + B->minmax_off, B->minmax_n, st, sms));

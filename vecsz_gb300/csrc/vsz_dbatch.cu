@@ -165,8 +165,9 @@ struct DLayout {
     uint16_t* all_bits;
     unsigned long long *all_start, *all_zoff;
     uint32_t* all_zero;
-    unsigned long long* scan_status;
-    uint32_t* scan_counter;
+    unsigned long long* scan_status[2];  // index scan, zero scan
+    uint32_t* scan_counter[2];
+    size_t cleared;
     std::vector<uint32_t*> table, table2, win, child, node_sym, parent, walk, redo;
     std::vector<uint16_t*> code;
     std::vector<size_t> chunk_base;
@@ -184,12 +185,15 @@ DLayout layout_dbatch(const std::vector<DField>& fs, uint8_t* base, size_t cap) 
         L.chunk_base.push_back(T);
         T += f.nch;
     }
+    for (int k = 0; k < 2; k++) {
+        L.scan_status[k]  = b.take<unsigned long long>(scan_tmp_tiles(T) + 1);
+        L.scan_counter[k] = b.take<uint32_t>(4);
+    }
+    L.cleared      = b.off;  // ctl to here is cleared per call
     L.all_bits     = b.take<uint16_t>(T + 8);
     L.all_start    = b.take<unsigned long long>(T + 1);
     L.all_zero     = b.take<uint32_t>(T + 1);
     L.all_zoff     = b.take<unsigned long long>(T + 1);
-    L.scan_status  = b.take<unsigned long long>(scan_tmp_tiles(T) + 1);
-    L.scan_counter = b.take<uint32_t>(4);
     for (size_t i = 0; i < nf; i++) {
         const DField& f     = fs[i];
         const uint32_t maxn = (uint32_t)(2 * f.nsym);
@@ -267,13 +271,13 @@ struct vsz_dbatch {
     std::vector<DqClass> classes;       // a launch each, or
     uint32_t small_off = 0, small_n = 0;  // one for all
     uint8_t* ctl = nullptr;
-    size_t ctl_bytes = 0;
+    size_t cleared = 0;
     uint16_t* all_bits = nullptr;
     unsigned long long *all_start = nullptr, *all_zoff = nullptr;
     uint32_t* all_zero = nullptr;
     size_t total_chunks = 0;
-    unsigned long long* scan_status = nullptr;
-    uint32_t* scan_counter = nullptr;
+    unsigned long long* scan_status[2] = {};
+    uint32_t* scan_counter[2] = {};
     int* batch_status = nullptr;
 };
 
@@ -477,15 +481,17 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     B->check        = reinterpret_cast<const DCheck*>(B->d_tables + o_ck);
     B->tasks        = reinterpret_cast<const BatchTask*>(B->d_tables + o_tk);
     B->ctl          = L.ctl;
-    B->ctl_bytes    = (size_t)nf * kDCtlBytes + 256;
+    B->cleared      = L.cleared;
     B->batch_status = L.batch_status;
     B->all_bits     = L.all_bits;
     B->all_start    = L.all_start;
     B->all_zero     = L.all_zero;
     B->all_zoff     = L.all_zoff;
-    B->scan_status  = L.scan_status;
-    B->scan_counter = L.scan_counter;
-    *out            = B;
+    for (int k = 0; k < 2; k++) {
+        B->scan_status[k]  = L.scan_status[k];
+        B->scan_counter[k] = L.scan_counter[k];
+    }
+    *out = B;
     return VSZ_OK;
 }
 
@@ -497,8 +503,9 @@ vsz_status vsz_dbatch_decompress(vsz_dbatch* B, void* stream) {
     const int sms     = num_sms();
     const uint32_t nf = (uint32_t)B->nfields;
     const uint32_t fb = (nf + 127) / 128;
-    // control words (constants, status, tree info, the batch status) to zero, redo counts to zero
-    VSZ_CUDA(cudaMemsetAsync(B->ctl, 0, B->ctl_bytes, st));
+    // control words (constants, status, tree info, the batch status) and both scans' look-back to zero,
+    // redo counts to zero
+    VSZ_CUDA(cudaMemsetAsync(B->ctl, 0, B->cleared, st));
     k_dbatch_init<<<fb, 128, 0, st>>>(B->check, nf);
     count_launch();
     {
@@ -516,8 +523,8 @@ vsz_status vsz_dbatch_decompress(vsz_dbatch* B, void* stream) {
                                                                                           B->tasks + B->idx_off, B->idx_n);
             count_launch();
         }
-        VSZ_TRY(launch_scan_u16(B->all_bits, B->all_start, B->total_chunks, B->scan_status, B->scan_counter, nullptr,
-                                B->batch_status, st));
+        VSZ_TRY(launch_scan_u16(B->all_bits, B->all_start, B->total_chunks, B->scan_status[0], B->scan_counter[0],
+                                nullptr, B->batch_status, st, true));
     }
     {
         StageTimer t(kStHuffDecode, st);
@@ -526,8 +533,8 @@ vsz_status vsz_dbatch_decompress(vsz_dbatch* B, void* stream) {
     }
     {
         StageTimer t(kStZeroScan, st);
-        VSZ_TRY(launch_scan_u32(B->all_zero, B->all_zoff, B->total_chunks, B->scan_status, B->scan_counter,
-                                B->all_zoff + B->total_chunks, B->batch_status, st));
+        VSZ_TRY(launch_scan_u32(B->all_zero, B->all_zoff, B->total_chunks, B->scan_status[1], B->scan_counter[1],
+                                B->all_zoff + B->total_chunks, B->batch_status, st, true));
         k_dbatch_check<<<fb, 128, 0, st>>>(B->check, nf, B->batch_status);
         count_launch();
     }
