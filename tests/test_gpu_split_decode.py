@@ -51,6 +51,16 @@ def test_roundtrip(cuda, kind, dict_size, n):
     np.testing.assert_array_equal(out, x)
 
 
+# 2^12 chunks: a warp for each; more: half a warp
+@pytest.mark.parametrize("kind,dict_size", [("smooth", 1024), ("runs", 1024), ("wide", 65536), ("long", 256)])
+@pytest.mark.parametrize("n", [(1 << 21) - 3, 1 << 21, (1 << 21) + 1, (1 << 21) + 513])
+def test_where_the_lanes_per_chunk_change(cuda, kind, dict_size, n):
+    x = field(kind, n, n)
+    status, out = roundtrip(cuda, x, dict_size)
+    assert status == 0
+    np.testing.assert_array_equal(out, x)
+
+
 @pytest.mark.parametrize("kind,n", [("smooth", 1 << 24), ("smooth", (1 << 24) + 1), ("runs", 1 << 22), ("runs", (1 << 22) + 1)])
 def test_last_field_that_takes_it(cuda, kind, n):
     x = field(kind, n, 3)

@@ -1412,13 +1412,15 @@ __global__ void __launch_bounds__(256)
 // round settles one more lane; one or two in practice).  The codeword counts give every lane's place
 // in the chunk, and a last pass decodes into shared memory, from where the codes are stored whole.
 // About three times the decoding work, S times less of it in a row: 64^3 at 4.4 bits a code 92 -> 27
-// us with S = 16 (8: 37, 32: 21, but 32 is slower from 10 K chunks on).
+// us with S = 16 (8: 37, 32: 21).  S = 32 up to kSplitWideChunks (4096 chunks at 1e-4: 43 -> 31 us, 8000:
+// 35 -> 39).
 //
 // A warp's chunks are consecutive in the stream: their words are loaded once, in bit order, into
 // shared memory (read from global memory where they average more than kSpanBits bits a codeword).
 // Both levels of the tables are in shared memory (win_primary), so the chain never waits for L2.
 // ------------------------------------------------------------------------------------------
 constexpr int kSplitS       = 16;   // lanes per chunk
+constexpr size_t kSplitWideChunks = size_t(1) << 12;  // up to this many chunks: a warp per chunk
 constexpr int kSplitThreads = 512;
 constexpr int kSplitBlocks  = 2;    // CTAs per SM
 constexpr int kSpanBits     = 10;
@@ -1964,14 +1966,19 @@ int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms) {
                          (reinterpret_cast<uintptr_t>(a.codes) & 15u) == 0 && a.chunk_len;
     if (indexed && a.tree_info && a.win) {
         // whole warps over as many SMs as there are, at most kSplitThreads to a copy of the tables
-        constexpr int kPer = 32 / kSplitS;  // chunks per warp
-        const size_t warps = (a.nchunks + kPer - 1) / kPer;
-        const size_t want  = (warps + (size_t)num_sms * kSplitBlocks - 1) / ((size_t)num_sms * kSplitBlocks);
-        const int threads  = 32 * (int)min((size_t)kSplitThreads / 32, max((size_t)4, want));
-        static std::atomic<unsigned long long> attr{0};
-        smem_limit_once(k_huff_decode_split<kSplitS>, (int)split_smem<kSplitS>(kSplitThreads), attr);
-        k_huff_decode_split<kSplitS><<<(unsigned)((warps * 32 + threads - 1) / threads), threads,
-                                       split_smem<kSplitS>(threads), st>>>(a);
+        static std::atomic<unsigned long long> attr{0}, attr_wide{0};
+        auto go = [&](auto s_c, std::atomic<unsigned long long>& at) {
+            constexpr int S    = decltype(s_c)::value;
+            constexpr int kPer = 32 / S;  // chunks per warp
+            const size_t warps = (a.nchunks + kPer - 1) / kPer;
+            const size_t want  = (warps + (size_t)num_sms * kSplitBlocks - 1) / ((size_t)num_sms * kSplitBlocks);
+            const int threads  = 32 * (int)min((size_t)kSplitThreads / 32, max((size_t)4, want));
+            smem_limit_once(k_huff_decode_split<S>, (int)split_smem<S>(kSplitThreads), at);
+            k_huff_decode_split<S><<<(unsigned)((warps * 32 + threads - 1) / threads), threads, split_smem<S>(threads),
+                                     st>>>(a);
+        };
+        if (a.nchunks <= kSplitWideChunks) go(std::integral_constant<int, 32>{}, attr_wide);
+        else go(std::integral_constant<int, kSplitS>{}, attr);
         count_launch();
     } else if (indexed) {
         if (a.tree_info) {
