@@ -647,6 +647,12 @@ __device__ __forceinline__ void huff_table_run(const HuffTableArgs& a) {
     // The reference rebuilds the root as an internal node when nodeCount > 256 and from
     // (C[0], t[0]) otherwise (src/huffman.hh:577,602,627).
     const bool root_leaf = (nc <= 256) && pT[0];
+    // A leaf as the root of several nodes, or of the one node where the caller's header had more, leaves
+    // nothing to decode by: a decoder given this tree must not run on tables that were never written.
+    if (root_leaf && (nc != 1 || a.win)) {
+        if (threadIdx.x == 0) set_status(a.status, VSZ_ERR_CORRUPT);
+        return;
+    }
     if (nc <= (uint32_t)kTableSmemNodes && !root_leaf) {
         huff_table_smem(a, nc, w, pL, pR, pC, pT, s_tab, s_node, s_scan, &s_bad);
         return;

@@ -334,7 +334,7 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
         t.parent         = L.parent[f];
         t.walk           = L.walk[f];
         t.table2         = L.table2[f];
-        t.win            = L.win[f];
+        t.win            = G.konst ? nullptr : L.win[f];
         t.info           = info;
         t.status         = status;
 

@@ -99,7 +99,8 @@ struct HuffTableArgs {
     uint32_t* walk;       // max_nodes: both children of an internal node, 16 bits each:
                           // 0x8000 | symbol for a leaf, else the node index (dict <= 16384)
     uint32_t* table2;     // table2_capacity(max_nodes) secondary entries
-    uint32_t* win;        // kWinImageWords, 16-byte aligned: the split decoder's tables, or null
+    uint32_t* win;        // kWinImageWords, 16-byte aligned: the split decoder's tables, or null (always for
+                          // one-node trees)
     uint32_t* info;       // [0] single-symbol tree flag [1] its symbol [2] longest codeword (255: > 64)
                           // [3] entries of table2
     int* status;
