@@ -918,6 +918,8 @@ __device__ __forceinline__ uint32_t decode_one(BitReader& br, const uint32_t* ta
     return 0xffffffffu;
 }
 
+// The general decoder: streams cut at bit positions (out_begin, nsym) and indexed ones whose codes are not
+// 16-byte aligned.  Zero codes are added to their 512-code chunk's count (cleared before the launch).
 __global__ void __launch_bounds__(256) k_huff_decode(HuffDecodeArgs a) {
     __shared__ uint32_t s_table[1 << kDecBits];
     for (int i = threadIdx.x; i < (1 << kDecBits); i += blockDim.x) s_table[i] = a.table[i];
@@ -933,7 +935,12 @@ __global__ void __launch_bounds__(256) k_huff_decode(HuffDecodeArgs a) {
     const uint32_t* gw   = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(a.payload) & ~(uintptr_t)3);
     BitReader br;
     br.init(gw, base0 + a.start_bit[j], base0 + a.payload_bits);
-    uint16_t* out = a.codes + out0;
+    uint16_t* out  = a.codes + out0;
+    uint32_t zeros = 0;  // since the last chunk boundary
+    auto flush = [&](unsigned long long at) {
+        if (zeros && a.chunk_zero) atomicAdd(&a.chunk_zero[at / kChunkSyms], zeros);
+        zeros = 0;
+    };
     for (unsigned long long k = 0; k < cnt; k++) {
         uint32_t s = decode_one(br, s_table, a.table2, a.child, a.node_sym, a.max_nodes);
         if (s == 0xffffffffu) {
@@ -941,6 +948,8 @@ __global__ void __launch_bounds__(256) k_huff_decode(HuffDecodeArgs a) {
             return;
         }
         out[k] = (uint16_t)s;
+        zeros += (s == 0);
+        if (((uint32_t)(out0 + k + 1) & (kChunkSyms - 1)) == 0 || k + 1 == cnt) flush(out0 + k);
     }
 }
 
@@ -2007,6 +2016,8 @@ int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms) {
             count_launch();
         }
     } else {
+        if (a.chunk_zero && cudaMemsetAsync(a.chunk_zero, 0, 4 * ((a.n + kChunkSyms - 1) / kChunkSyms), st) != cudaSuccess)
+            return VSZ_ERR_CUDA;
         k_huff_decode<<<grid, 256, 0, st>>>(a);
         count_launch();
     }

@@ -1245,7 +1245,7 @@ static PadView pad_view_of(const vsz_archive_desc* d, int bs, const uint8_t* d_a
     return v;
 }
 
-// Whether the decoder of this archive counts the zero codes of each chunk: the indexed ones do.
+// Whether the decoder of this archive counts the zero codes of each chunk: all that read the index do.
 static bool indexed_counts(const vsz_archive_desc* d) {
     return d->has_trailer && d->node_count > 1;
 }
