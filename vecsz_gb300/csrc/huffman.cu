@@ -1683,8 +1683,8 @@ int launch_huff_table_batch(const HuffTableArgs* args, uint32_t nfields, cudaStr
 }
 
 int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks, uint32_t ntasks,
-                             const BatchTask* const_tasks, uint32_t nconst, size_t total_chunks, cudaStream_t st, int num_sms) {
-    if (ntasks && total_chunks <= kSplitChunks) {
+                             const BatchTask* const_tasks, uint32_t nconst, bool split, cudaStream_t st, int num_sms) {
+    if (ntasks && split) {
         const uint32_t cap  = (uint32_t)num_sms * kSplitBlocks;
         static std::atomic<unsigned long long> attr{0};
         smem_limit_once(k_huff_decode_split_batch<kSplitS>, (int)split_smem<kSplitS>(kSplitThreads), attr);

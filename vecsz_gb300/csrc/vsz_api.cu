@@ -231,7 +231,7 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     ta.table2 = w.table2;
     ta.info = w.tinfo;
     // the split decoder's tables, for fields that take it (it copies them 16 bytes at a time)
-    const bool split = chunk_bits && node_count > 1 && huff_split_applies(n_index_chunks, pbits) &&
+    const bool split = chunk_bits && node_count > 1 && huff_split_applies(n_index_chunks, pbits, node_count) &&
                        (reinterpret_cast<uintptr_t>(w.win) & 15u) == 0;
     ta.win = split ? w.win : nullptr;
     ta.status = w.status;

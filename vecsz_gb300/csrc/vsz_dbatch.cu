@@ -74,6 +74,7 @@ struct DField {
     double ebf;
     size_t nch;
     size_t units;  // block-8 warp units
+    uint32_t nodes;
     bool sep, vec, konst, w8;
 };
 
@@ -149,6 +150,7 @@ int field_of(const vsz_dbatch_field& F, DField& out) {
     out.ebf   = d.eb_final;
     out.nch   = (out.g.n + kChunkSyms - 1) / kChunkSyms;
     if (d.n_chunks != out.nch) return VSZ_ERR_CORRUPT;
+    out.nodes = d.node_count;
     out.konst = d.node_count == 1;
     DqDecArgs a{};
     a.d0 = out.g.d0;
@@ -168,6 +170,7 @@ struct DLayout {
     unsigned long long* scan_status[2];  // index scan, zero scan
     uint32_t* scan_counter[2];
     size_t cleared;
+    bool split;  // fields are decoded by the split decoder
     std::vector<uint32_t*> table, table2, win, child, node_sym, parent, walk, redo;
     std::vector<uint16_t*> code;
     std::vector<size_t> chunk_base;
@@ -181,10 +184,13 @@ DLayout layout_dbatch(const std::vector<DField>& fs, uint8_t* base, size_t cap) 
     L.ctl          = b.take<uint8_t>(nf * kDCtlBytes + 256);
     L.batch_status = reinterpret_cast<int*>(L.ctl ? L.ctl + nf * kDCtlBytes : nullptr);
     size_t T = 0;
+    uint32_t nodes = 0;
     for (const auto& f : fs) {
         L.chunk_base.push_back(T);
         T += f.nch;
+        nodes = std::max(nodes, f.nodes);
     }
+    L.split = huff_split_batch(T, nodes);
     for (int k = 0; k < 2; k++) {
         L.scan_status[k]  = b.take<unsigned long long>(scan_tmp_tiles(T) + 1);
         L.scan_counter[k] = b.take<uint32_t>(4);
@@ -198,7 +204,7 @@ DLayout layout_dbatch(const std::vector<DField>& fs, uint8_t* base, size_t cap) 
         const DField& f     = fs[i];
         const uint32_t maxn = (uint32_t)(2 * f.nsym);
         L.table.push_back(b.take<uint32_t>(1u << kDecBits));
-        L.win.push_back(T <= kSplitChunks ? b.take<uint32_t>(kWinImageWords) : nullptr);
+        L.win.push_back(L.split ? b.take<uint32_t>(kWinImageWords) : nullptr);
         L.table2.push_back(b.take<uint32_t>(table2_capacity(maxn - 1)));
         L.child.push_back(b.take<uint32_t>(2 * (size_t)maxn));
         L.node_sym.push_back(b.take<uint32_t>(maxn));
@@ -268,6 +274,7 @@ struct vsz_dbatch {
     const BatchTask* tasks = nullptr;
     uint32_t idx_off = 0, idx_n = 0, dec_off = 0, dec_n = 0, const_off = 0, const_n = 0, out_off = 0, out_n = 0;
     uint32_t redo_off = 0, redo_n = 0;
+    bool split = false;
     std::vector<DqClass> classes;       // a launch each, or
     uint32_t small_off = 0, small_n = 0;  // one for all
     uint8_t* ctl = nullptr;
@@ -396,7 +403,8 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     }
     // ---- task lists
     B->total_chunks       = L.chunk_base.empty() ? 0 : L.chunk_base.back() + fs.back().nch;
-    const uint64_t dec_per = B->total_chunks <= kSplitChunks ? kSplitTaskChunks : kDecTaskChunks;
+    B->split               = L.split;
+    const uint64_t dec_per = L.split ? kSplitTaskChunks : kDecTaskChunks;
     B->idx_off = (uint32_t)tasks.size();
     for (uint32_t f = 0; f < nf; f++) add_tasks(tasks, f, 2 * fs[f].nch, kCopyTaskBytes);
     B->idx_n   = (uint32_t)tasks.size() - B->idx_off;
@@ -529,7 +537,7 @@ vsz_status vsz_dbatch_decompress(vsz_dbatch* B, void* stream) {
     {
         StageTimer t(kStHuffDecode, st);
         VSZ_TRY(launch_huff_decode_batch(B->dec, B->tasks + B->dec_off, B->dec_n, B->tasks + B->const_off,
-                                         B->const_n, B->total_chunks, st, sms));
+                                         B->const_n, B->split, st, sms));
     }
     {
         StageTimer t(kStZeroScan, st);

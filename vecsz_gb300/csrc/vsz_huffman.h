@@ -1,6 +1,7 @@
 // Internal interface of the Huffman kernels (huffman.cu).
 #pragma once
 
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -32,13 +33,33 @@ __host__ __device__ inline size_t table2_capacity(uint32_t max_nodes) {
 constexpr int kWinBits     = 13;
 constexpr int kDec2Smem    = 3072;
 constexpr size_t kWinImageWords = ((size_t)1 << kWinBits) + kDec2Smem;
-// Whether a stream takes the split decoder (k_huff_decode_split).  It costs about 4 us per 1024
-// chunks over a floor of 20; a lane per chunk costs one lane's chain, 75 us at 1-2 bits a code and
-// 160 at 7 (its secondary table is in L2): 64^3 (512 chunks) 92 -> 27 us, 333x241x187 (29 K chunks, 7 bits)
-// 161 -> 125, but 3600x1800 (12.7 K chunks, 1.5 bits) 75 -> 78.
-constexpr size_t kSplitChunks = size_t(1) << 13, kSplitMaxChunks = size_t(1) << 15;
-inline bool huff_split_applies(size_t nchunks, unsigned long long payload_bits) {
-    return nchunks <= kSplitChunks || (nchunks <= kSplitMaxChunks && payload_bits / 4 >= nchunks * 512);
+// Whether a stream takes the split decoder (k_huff_decode_split) or a lane per chunk (k_huff_decode_win).
+// The window decoder's time is one lane's chain whatever the number of chunks: 60 us where every codeword
+// has at most kDecBits bits, 80-160 at 6-9 bits a code, 150-400 with trees of 8K nodes and more.  The split
+// decoder runs in rounds of CTAs (9728 chunks of 16 lanes fill 152 SMs), each 25-45 us where its
+// tables hold the codewords and a warp's words fit its buffer (kSpanBits bits a code), 100-400 where not.
+// Decode of a field, window -> split, us:
+//   one round: 8000 chunks, 7 bits 98 -> 34; 13.7 bits, 118K nodes 325 -> 228; but 16 bits 190 -> 354 (512: 205 -> 160)
+//   two: 15.6 K chunks, 6.3 bits 132 -> 87, 8 bits, 7.8K nodes 229 -> 160; uniform residuals, 8 bits 76 -> 82; 12 bits
+//     100 -> 194; 12.7 K chunks, 1.5 bits 75 -> 78
+//   three: 29.3 K chunks, 6.3 bits 159 -> 138, 9 bits 108 -> 95; 5.4 bits 67 -> 72; 8 bits, 7.8K nodes (27 K) 203 -> 243
+//   32.8 K chunks: 6.5 bits 126 -> 147, 9 bits 92 -> 99
+// So: one round always, unless nearly no codeword is in the tables; two where codewords are of many lengths
+// (0.4 bits below the fixed length for as many leaves) and fit both tables and buffer; three at 6 bits or
+// more with trees whose long codewords are in the image.
+constexpr size_t kSplitChunks = size_t(1) << 13, kSplitTwoRounds = 19456, kSplitMaxChunks = 30000;
+inline bool huff_split_applies(size_t nchunks, unsigned long long payload_bits, uint32_t nodes) {
+    const double bits = (double)payload_bits / ((double)nchunks * 512.0);
+    if (nchunks <= kSplitChunks) return bits <= 14.0 || nchunks <= 1024;
+    if (bits < 4.0 || bits > 9.5 || nodes > 8192u || bits > std::log2((nodes + 1u) / 2.0) - 0.4) return false;
+    return nchunks <= kSplitTwoRounds || (nchunks <= kSplitMaxChunks && bits >= 6.0 && nodes <= 5000u);
+}
+// The same for a batch (k_huff_decode_split_batch), by its chunks and its largest tree.  A task is 64 chunks
+// of one field there, two rounds of one CTA, so one field past the image costs the batch what it costs a
+// large field: largest tree 2.2K nodes 90 -> 53 us, 3.8K 158 -> 164, 5.0K 187 -> 319, 8.1K 182 -> 330.
+constexpr uint32_t kSplitBatchNodes = 3072;
+inline bool huff_split_batch(size_t total_chunks, uint32_t most_nodes) {
+    return total_chunks <= kSplitChunks && most_nodes <= kSplitBatchNodes;
 }
 constexpr int kChunkSyms   = 512;  // codewords per entry of this library's decode index
 constexpr int kSyncBits    = 8192; // chunk size (bits) of the self-synchronising decoder
@@ -170,7 +191,7 @@ int launch_huff_table(HuffTableArgs a, cudaStream_t st);
 // constant fill.
 int launch_huff_table_batch(const HuffTableArgs* args, uint32_t nfields, cudaStream_t st, int num_sms);
 int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks, uint32_t ntasks,
-                             const BatchTask* const_tasks, uint32_t nconst, size_t total_chunks, cudaStream_t st,
+                             const BatchTask* const_tasks, uint32_t nconst, bool split, cudaStream_t st,
                              int num_sms);
 int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms);
 int launch_huff_const(uint16_t* codes, size_t n, const uint32_t* info, const int* status, cudaStream_t st, int num_sms);
