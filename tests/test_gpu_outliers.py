@@ -54,3 +54,16 @@ def test_redo_units_with_outliers(cuda, monkeypatch, dims):
     x[at] = rng.integers(1 << 21, 1 << 23, int(at.sum()))
     codec = check(cuda, x, dims, dict_size=1024)
     assert 0 < codec._desc.n_outlier * 64 < n
+
+
+@pytest.mark.parametrize("density", [0.0, 0.001, 0.3, 1.0])
+@pytest.mark.parametrize("dims", [(511,), (513,), (70001,), (300, 211), (40, 37, 24)])
+def test_without_the_index(cuda, dims, density):
+    """Archives as the reference writes them: the self-synchronising decoder's streams cut chunks of 512
+    codes anywhere, and it counts their zero codes."""
+    n = int(np.prod(dims))
+    rng = np.random.default_rng(n + 1)
+    x = np.where(rng.random(n) < density, rng.integers(1000, 100000, n), rng.integers(-4, 5, n)).astype(np.float32)
+    ref, _ = O.compress(x, dims, 8, 256, 0.5, False)
+    y = V.decompress(ref, len(ref), 0, 256, 8)
+    np.testing.assert_array_equal(y.view(np.uint32), O.decompress(ref, 8, 256, 0.0).view(np.uint32))

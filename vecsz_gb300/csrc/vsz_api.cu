@@ -211,10 +211,11 @@ DecompressWs layout_decompress(const Geometry& g, int dict, size_t payload_bytes
     return w;
 }
 
-// Decode n codes from a Huffman section at d_huff.  Index path when chunk_bits != null.
+// Decode n codes from a Huffman section at d_huff.  Index path when chunk_bits != null.  chunk_zero (or
+// null): zero codes per 512 codes; not written for one-node trees.
 int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, size_t tree_bytes, size_t n, int dict,
                  const uint16_t* chunk_bits, size_t n_index_chunks, uint32_t chunk_syms, const DecompressWs& w,
-                 bool cleared, cudaStream_t st) {
+                 uint32_t* chunk_zero, bool cleared, cudaStream_t st) {
     const uint8_t* payload   = d_huff + 8 + tree_bytes;
     size_t payload_bytes     = huff_bytes - 8 - tree_bytes;
     unsigned long long pbits = (unsigned long long)payload_bytes * 8ull;
@@ -263,6 +264,7 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
     // the window decoder takes trees whose codewords are at most 32 bits; VSZ_DECODE_NO_WINDOW
     // sends every tree to the general indexed decoder (tests of that path)
     da.tree_info = getenv("VSZ_DECODE_NO_WINDOW") ? nullptr : w.tinfo;
+    da.chunk_zero = chunk_zero;
     da.status = w.status;
     if (chunk_bits) {
         if (!with_scan) {
@@ -272,7 +274,6 @@ int decode_codes(const uint8_t* d_huff, size_t huff_bytes, uint32_t node_count, 
         }
         da.start_bit = w.chunk_start;
         da.chunk_len = chunk_bits;
-        da.chunk_zero = w.chunk_zero;
         da.out_begin = nullptr;
         da.nsym = nullptr;
         da.nchunks = n_index_chunks;
@@ -870,7 +871,8 @@ vsz_status vsz_huffman_decode(const uint8_t* d_huff, size_t huff_bytes, size_t n
     if (nc == 0 || nc > (uint32_t)(2 * dict_size - 1) || 8 + tree_bytes_size(nc) > huff_bytes) return VSZ_ERR_CORRUPT;
     VSZ_CUDA(cudaMemsetAsync(w.status, 0, sizeof(int), S(stream)));
     // decode into w.code, then copy to the caller (w.code is sized for n)
-    int rc = decode_codes(d_huff, huff_bytes, nc, tree_bytes_size(nc), n, dict_size, nullptr, 0, 0, w, false, S(stream));
+    int rc = decode_codes(d_huff, huff_bytes, nc, tree_bytes_size(nc), n, dict_size, nullptr, 0, 0, w, nullptr, false,
+                          S(stream));
     if (rc) return rc;
     VSZ_CUDA(cudaMemcpyAsync(d_code, w.code, n * sizeof(uint16_t), cudaMemcpyDeviceToDevice, S(stream)));
     int st = 0;
@@ -1245,11 +1247,6 @@ static PadView pad_view_of(const vsz_archive_desc* d, int bs, const uint8_t* d_a
     return v;
 }
 
-// Whether the decoder of this archive counts the zero codes of each chunk: all that read the index do.
-static bool indexed_counts(const vsz_archive_desc* d) {
-    return d->has_trailer && d->node_count > 1;
-}
-
 vsz_status vsz_decompress_bounds(const vsz_archive_desc* d, const vsz_decompress_opts* o, size_t* ws_bytes) {
     if (!d) return VSZ_ERR_INVALID;
     int dict, bs;
@@ -1290,9 +1287,9 @@ vsz_status vsz_decompress(const vsz_archive_desc* d, const vsz_decompress_opts* 
     }
     const uint16_t* idx = d->has_trailer ? reinterpret_cast<const uint16_t*>(d_archive + d->index_offset) : nullptr;
     VSZ_TRY(decode_codes(d_archive + d->huff_offset, d->huff_bytes, d->node_count, d->tree_bytes, g.n, nsym, idx,
-                         d->has_trailer ? d->n_chunks : 0, d->chunk_syms, w, true, st));
-    // the outliers to their elements of the output: the indexed decoders count the zero codes of each
-    // chunk, other codes are counted here
+                         d->has_trailer ? d->n_chunks : 0, d->chunk_syms, w, w.chunk_zero, true, st));
+    // the outliers to their elements of the output: the decoders count the zero codes of each chunk, a
+    // constant field's are counted here
     OutlierArgs oa{};
     oa.codes       = w.code;
     oa.n           = g.n;
@@ -1307,7 +1304,7 @@ vsz_status vsz_decompress(const vsz_archive_desc* d, const vsz_decompress_opts* 
     oa.status      = w.status;
     {
         StageTimer t(kStZeroScan, st);
-        if (!indexed_counts(d)) VSZ_TRY(launch_count_zeros_chunk(w.code, g.n, w.chunk_zero, st, num_sms()));
+        if (d->node_count == 1) VSZ_TRY(launch_count_zeros_chunk(w.code, g.n, w.chunk_zero, st, num_sms()));
         VSZ_TRY(launch_scan_u32(w.chunk_zero, w.chunk_off, oa.nchunks, w.scan_status, w.scan_counter, w.scan_total,
                                 w.status, st, idx != nullptr));  // the sync path's scan has used the words
     }
@@ -1609,7 +1606,7 @@ vsz_status vsz_decompress_f64(const vsz_archive_desc* d, const uint8_t* d_archiv
                                 reinterpret_cast<unsigned long long*>(w.mm), w.status, st, num_sms()));
     const uint16_t* idx = reinterpret_cast<const uint16_t*>(d_archive + d->index_offset);
     VSZ_TRY(decode_codes(d_archive + d->huff_offset, d->huff_bytes, d->node_count, d->tree_bytes, g.n, dict, idx,
-                         d->n_chunks, d->chunk_syms, w, false, st));
+                         d->n_chunks, d->chunk_syms, w, w.chunk_zero, false, st));
     {
         StageTimer t(kStZeroScan, st);
         VSZ_TRY(launch_count_zeros(w.code, g.d0, g.nrows, w.seg_zero, st, num_sms()));
