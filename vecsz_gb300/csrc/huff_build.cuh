@@ -280,7 +280,10 @@ __device__ __forceinline__ void build_field(const HuffBuildArgs& a, uint8_t* s_b
     __shared__ unsigned long long s_fsum[8];
     if (*a.status != VSZ_OK) return;  // an earlier stage failed (uniform: one CTA)
     const int dict = a.dict;
-    BuildWs w      = carve_build_ws(IN_SMEM ? s_build_dyn : reinterpret_cast<uint8_t*>(a.scratch), dict);
+    uint8_t* ws    = s_build_dyn;
+    // pairs of heap entries are 16 bytes; build_ws_bytes has 256 to spare
+    if (!IN_SMEM) ws = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(a.scratch) + 15u) & ~(uintptr_t)15);
+    BuildWs w      = carve_build_ws(ws, dict);
     if (threadIdx.x == 0) s_fail = 0;
     for (int i = threadIdx.x; i < 2 * dict + 8; i += blockDim.x) w.heap[i] = 0ull;
     for (int i = threadIdx.x; i < dict; i += blockDim.x) {

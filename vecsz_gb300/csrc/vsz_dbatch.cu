@@ -178,6 +178,9 @@ struct DLayout {
 };
 
 DLayout layout_dbatch(const std::vector<DField>& fs, uint8_t* base, size_t cap) {
+    // from the next 256-byte boundary (the last 256 bytes leave room for it): the decoders store 16 bytes
+    // at a time to the codes and copy the table images so
+    if (base) base += (256 - reinterpret_cast<uintptr_t>(base) % 256) % 256;
     Bump b{base, cap};
     DLayout L{};
     const size_t nf = fs.size();
