@@ -259,15 +259,16 @@ vsz_status vsz_compress(const vsz_params* p, int ndim, const size_t dims[3], con
 
 /* ---- many fields at once -------------------------------------------------------------------
  * A batch of fields of any shapes, dimensionalities, error bounds and dictionary sizes is
- * compressed in a handful of launches: each stage is one launch (one per kernel class for the
+ * compressed in a handful of launches: each stage is one launch (one per block size for the
  * dual-quant stage) over a device-side table of per-field arguments and a list of block-wide
- * tasks, and the Huffman trees are built on the device, one CTA per field.  Every field's archive
+ * tasks, and the Huffman trees are built on the device, one CTA per field (dictionaries up to 1024
+ * within the dual-quant launch).  Every field's archive
  * and result are byte-identical to vsz_compress of that field alone.  No counterpart in the
  * reference, which compresses one field per process.
  *
  * vsz_batch_create lays out the caller's workspace (vsz_batch_workspace_bytes), resolves every
  * pointer and uploads the tables once (synchronous; it allocates the tables).  vsz_batch_compress
- * then only enqueues device work on `stream` -- memsets and launches, no host synchronisation and no
+ * then only enqueues device work on `stream` -- launches, no host synchronisation and no
  * allocation -- so it may be captured in a CUDA graph and replayed; each replay recompresses the
  * current contents of the fields' input buffers.  d_results: 8 u64 (vsz_result) per field. */
 typedef struct vsz_batch_field {

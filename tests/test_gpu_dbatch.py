@@ -40,8 +40,8 @@ def _mixed_archives(seed, n):
 
 def test_dbatch_matches_single_field_decompress(cuda):
     items = _mixed_archives(5, 36)
-    # a constant field (one-symbol tree), dense outliers (the adversarial field) and a 3D field
-    # wide enough for the separable pass
+    # a constant field (one-symbol tree), dense outliers (the adversarial field) and a 3D field with
+    # rows of 256 (the wavefront pass, as every 3D field of a batch of this size)
     xc = np.full(70000, 3.25, np.float32)
     items.append((xc, (70000,), 1e-3, "abs", 1024, V.compress(xc, (70000,), 1e-3, "abs", 1024, 8)))
     xa = fields.adversarial_3d(24, 40, 64, seed=9).ravel()

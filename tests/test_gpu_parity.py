@@ -305,8 +305,8 @@ def test_long_codewords_general_decoder(cuda, monkeypatch):
 
 
 def test_long_codewords_dict4096_match_oracle(cuda):
-    """Dictionary 4096 and a last chunk of 265 codes: the window decoder's secondary table and its
-    tree walk, for codewords over 12 and 20 bits."""
+    """Dictionary 4096 and a last chunk of 265 codes: the secondary table and the tree walk, for codewords
+    over 12 and 20 bits."""
     rng = np.random.default_rng(78)
     n = (1 << 21) + 777
     k = np.minimum(rng.geometric(0.45, n) - 1, 30)

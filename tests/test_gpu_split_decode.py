@@ -1,5 +1,5 @@
-"""The split Huffman decoder (several lanes per 512-code chunk, fields of up to 2^15 chunks; up to 2^13
-at under 4 bits a code): streams that start out of step, at the edges of chunks, warps and of the range that takes it.  Fields hold
+"""The split Huffman decoder (several lanes per 512-code chunk, fields of up to 2^13 chunks; more where
+its rule says so): streams that start out of step, at the edges of chunks and warps and about the range that takes it.  Fields hold
 integers and the bound is 0.5, so the reconstruction is the field itself."""
 import numpy as np
 import pytest

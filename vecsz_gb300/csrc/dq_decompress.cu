@@ -651,7 +651,8 @@ __global__ void __launch_bounds__(128, 6) k_dq_decompress_b8s(DqDecArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Wavefront pass, 3D, block 8, no padding, fields of at most kW8MaxN elements.  The block-8
+// Wavefront pass, 3D, block 8, no padding: single fields of at most kW8MaxN elements, and the 3D fields of
+// batches that hold at most 2^25 elements of them (kDbatchW8MaxN).  The block-8
 // kernels give each lane a whole 8 x 8 x 8 block, 512 elements one after another; a field with
 // fewer warp units than the GPU holds then takes that chain's latency (0.1-0.3 ms) whatever its
 // size.  Here a block has 8 lanes, one per row y, and lane y runs one plane behind lane y - 1: at
@@ -678,7 +679,9 @@ __device__ __forceinline__ void dq_w8_units(const DqDecArgs& a, uint32_t first, 
     const unsigned lane   = lane_id();
     const int y           = (int)(lane & 7u);  // row of the block
     const uint32_t nxq    = (a.nbx8 + 3) / 4;  // groups of 4 blocks along x
-    for (uint32_t u = first; u < end; u += stride) {  // at most kW8MaxN / 256 units
+    // unit indices fit 32 bits: there are no more units than elements, 2^25 at most (a unit of four whole
+    // blocks holds 2048)
+    for (uint32_t u = first; u < end; u += stride) {
         const uint32_t xq = u % nxq, r = u / nxq;
         const uint32_t yb = r % a.nyb, zb = r / a.nyb;
         const uint32_t bx = xq * 4 + (lane >> 3);

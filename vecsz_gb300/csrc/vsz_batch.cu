@@ -2,11 +2,12 @@
 // launches, each over a device-side table of per-field arguments and a list of block-wide tasks
 // (one field, a range of its work units).  The plan is built once on the host, where every
 // field's geometry is known, and uploaded; vsz_batch_compress then only enqueues device work
-// (memsets and launches on the caller's stream), so it can be captured in a CUDA graph.
+// (launches on the caller's stream), so it can be captured in a CUDA graph.
 //
 // Per field the result is byte-identical to vsz_compress of that field: the same kernels' unit
 // bodies run, only the way units are handed out differs.  The Huffman trees are built on the
-// device, one CTA per field, all fields in one launch.
+// device, one CTA per field: for dictionaries up to 1024 within the dual-quant launch, by the CTA that
+// finishes the field's last unit, for larger ones in a launch after it.
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
@@ -24,7 +25,7 @@ using namespace vsz::api;
 
 namespace {
 
-// Per-field control words, one 256-byte record per field, zeroed by one memset.
+// Per-field control words, one 256-byte record per field, cleared by k_batch_init.
 constexpr size_t kCtlBytes   = 256;
 constexpr size_t kCtlConsts  = 0;    // Consts (<= 64 bytes)
 constexpr size_t kCtlMm      = 64;   // u32 {max key, min key}

@@ -41,7 +41,7 @@ constexpr size_t kWinImageWords = ((size_t)1 << kWinBits) + kDec2Smem;
 // Decode of a field, window -> split, us:
 //   one round: 8000 chunks, 7 bits 98 -> 34; 13.7 bits, 118K nodes 325 -> 228; but 16 bits 190 -> 354 (512: 205 -> 160)
 //   two: 15.6 K chunks, 6.3 bits 132 -> 87, 8 bits, 7.8K nodes 229 -> 160; uniform residuals, 8 bits 76 -> 82; 12 bits
-//     100 -> 194; 12.7 K chunks, 1.5 bits 75 -> 78
+//     100 -> 194; 12.7 K chunks, 2.6 bits 87 -> 93
 //   three: 29.3 K chunks, 6.3 bits 159 -> 138, 9 bits 108 -> 95; 5.4 bits 67 -> 72; 8 bits, 7.8K nodes (27 K) 203 -> 243
 //   32.8 K chunks: 6.5 bits 126 -> 147, 9 bits 92 -> 99
 // So: one round always, unless nearly no codeword is in the tables; two where codewords are of many lengths
@@ -185,10 +185,10 @@ void huff_build_prepare();  // one-time kernel attributes of launch_huff_build (
 size_t huff_build_scratch_bytes(int dict);  // also the shared memory of a build there
 int launch_huff_encode(HuffEncodeArgs a, cudaStream_t st, int num_sms);
 int launch_huff_table(HuffTableArgs a, cudaStream_t st);
-// Many fields: decode tables one CTA per field; decoding over tasks of (field, 256-chunk range
-// of the field's index), every field's tree by the decoder of its kind (the window decoder for
-// codewords up to 32 bits, the general one beyond), and const_tasks (one-symbol trees) by a
-// constant fill.
+// Many fields: decode tables one CTA per field; decoding over tasks of (field, range of the field's
+// index), split (huff_split_batch): all by the split decoder, else 256 chunks each, every field's tree by the
+// decoder of its kind (the window decoder for codewords up to 32 bits, the general one beyond); const_tasks
+// (one-symbol trees) by a constant fill.
 int launch_huff_table_batch(const HuffTableArgs* args, uint32_t nfields, cudaStream_t st, int num_sms);
 int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks, uint32_t ntasks,
                              const BatchTask* const_tasks, uint32_t nconst, bool split, cudaStream_t st,
