@@ -128,3 +128,18 @@ def test_where_the_batch_decoder_changes(cuda, width):
     assert b.statuses() == [0, 0, 0]
     for x, o in zip(xs, b.outputs):
         np.testing.assert_array_equal(o.cpu().numpy(), x)
+
+
+# more than 2^13 chunks, small trees: the window decoder with its secondary table in shared memory; at 152
+# SMs 456 tasks of 256 chunks are one round of that form, 608 of the other
+@pytest.mark.parametrize("tasks", [40, 500])
+def test_batch_of_small_trees(cuda, tasks):
+    rng = np.random.default_rng(tasks)
+    r = np.rint(rng.laplace(0, 40, tasks * 256 * 512 - 77)).clip(-500, 500).astype(np.int64)
+    xs = [from_residuals(r), from_residuals(rng.integers(-3, 4, 70_003)), np.full(600, 2.0, np.float32)]
+    b = V.BatchDecompressor([V.compress(x, (x.size,), 0.5, "abs", 1024, 8).data for x in xs])
+    assert sum(int(d.n_chunks) for d in b.descs) > 1 << 13 and max(int(d.node_count) for d in b.descs) < 3000
+    b.decompress()
+    assert b.statuses() == [0, 0, 0]
+    for x, o in zip(xs, b.outputs):
+        np.testing.assert_array_equal(o.cpu().numpy(), x)

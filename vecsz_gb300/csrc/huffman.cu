@@ -976,23 +976,31 @@ constexpr int kWinRound     = 8;
 constexpr int kWinRing      = 8;    // blocks of 16 bytes per lane
 constexpr int kWinWait      = 4;    // copy groups left in flight at a round's start
 constexpr int kWinLaneWords = kWinRing * 4 + 4;  // a lane's ring, padded: lanes 8 apart share banks
-constexpr int kWinThreads   = 512;  // one copy of the tables per CTA, shared by its warps
-constexpr int kWinMinBlocks = 2;
-constexpr int kWinBatchThreads = 256, kWinBatchBlocks = 3;
-// Secondary entries in shared memory (a 1024-symbol tree has 2.5-4.3 K; those past it are read from
-// L2).  In L2 they stalled a warp whenever one lane left the primary table, on 59 % of the steps at 6.5
-// bits a code.
+// Secondary entries in shared memory (a 1024-symbol tree has 2.5-4.3 K of them; those past it are read
+// from L2).  In L2 they stalled a warp whenever one lane left the primary table, on 59 % of the steps at
+// 6.5 bits a code.
 constexpr uint32_t kWinTable2 = 4096;
+// Trees of more nodes go without (SECOND = false): most of their long codewords would be past it, and its 16 KB a
+// CTA are missed elsewhere.  Decode of 512^3, with -> without: 5005 nodes 309 -> 290 us, 8191 391 -> 360, 131 K 961
+// -> 837, but 2047 (1e-5) 255 -> 274; of a batch of 200 fields up to 1 M values, 8 K nodes 279 -> 222.
+constexpr uint32_t kWinSecondNodes = 5000;
+template <bool SECOND>
+struct WinShape {
+    static constexpr int kThreads = SECOND ? 512 : 256;  // one copy of the tables per CTA, shared by its warps
+    static constexpr int kBlocks  = SECOND ? 2 : 4;
+    static constexpr int kBatchThreads = 256, kBatchBlocks = SECOND ? 3 : 4;
+    static constexpr size_t kTables = (sizeof(uint32_t) << kDecBits) + (SECOND ? sizeof(uint32_t) * kWinTable2 : 0);
+    static constexpr size_t smem(int threads) { return kTables + (size_t)threads * kWinLaneWords * 4; }
+};
 // Blocks wn / 4 .. wn / 4 + kWinRing - 2 are requested and all but the newest kWinWait have landed
 // at a round's start: at least 4 (kWinRing - 1 - kWinWait) - 3 words from wn, and a round of
 // kWinRound codewords of <= 32 bits moves the window by at most kWinRound words.
 static_assert(4 * (kWinRing - 1 - kWinWait) - 3 >= kWinRound, "a round may read words still in flight");
 static_assert((kWinRing & (kWinRing - 1)) == 0 && (kWinRound == 8 || kWinRound == 4), "ring and round shapes");
-constexpr size_t kWinTables = (sizeof(uint32_t) << kDecBits) + sizeof(uint32_t) * kWinTable2;
-constexpr size_t win_smem(int threads) { return kWinTables + (size_t)threads * kWinLaneWords * 4; }
 typedef uint32_t WinRing[32][kWinLaneWords];  // one warp's rings, [lane][word]
 
 // Lane j of the calling warp decodes chunk j (the tables are in shared memory; no block barrier inside).
+template <bool SECOND>
 __device__ __forceinline__ void decode_win_lane(const HuffDecodeArgs& a, size_t j, const uint32_t* s_table,
                                                 const uint32_t* s_table2, WinRing* s_ring) {
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -1077,7 +1085,7 @@ __device__ __forceinline__ void decode_win_lane(const HuffDecodeArgs& a, size_t 
                 if (e & 0x80u) {
                     const uint32_t w2b = (e >> 8) & 0xfu;
                     const uint32_t i2  = (e >> 12) + ((win >> (32 - kDecBits - w2b)) & ((1u << w2b) - 1u));
-                    const uint32_t e2  = i2 < kWinTable2 ? s_table2[i2] : __ldg(&a.table2[i2]);
+                    const uint32_t e2  = SECOND && i2 < kWinTable2 ? s_table2[i2] : __ldg(&a.table2[i2]);
                     len   = e2 & 0xffu;
                     sy    = e2 >> 8;
                     node  = e2 >> 8;
@@ -1162,23 +1170,26 @@ __device__ __forceinline__ void decode_win_lane(const HuffDecodeArgs& a, size_t 
     if (j < a.nchunks && a.chunk_zero) a.chunk_zero[j] = zeros;
 }
 
-// Both tables of one field into shared memory, by the whole CTA.
+// The tables of one field into shared memory, by the whole CTA.
+template <bool SECOND>
 __device__ __forceinline__ void win_tables(const HuffDecodeArgs& a, uint32_t* s_table) {
     for (uint32_t i = threadIdx.x; i < (1u << kDecBits); i += blockDim.x) s_table[i] = a.table[i];
-    const uint32_t n2 = min(a.tree_info[3], kWinTable2);
+    const uint32_t n2 = SECOND ? min(a.tree_info[3], kWinTable2) : 0u;
     for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) s_table[(1 << kDecBits) + i] = a.table2[i];
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kWinThreads, kWinMinBlocks) k_huff_decode_win(HuffDecodeArgs a) {
+template <bool SECOND>
+__global__ void __launch_bounds__(WinShape<SECOND>::kThreads, WinShape<SECOND>::kBlocks)
+    k_huff_decode_win(HuffDecodeArgs a) {
     extern __shared__ __align__(16) uint8_t s_win_dyn[];
-    // [primary table: 1 << kDecBits words][kWinTable2 words][rings: warp][lane][kWinLaneWords]
+    // [primary table: 1 << kDecBits words][SECOND: kWinTable2 words][rings: warp][lane][kWinLaneWords]
     uint32_t* s_table = reinterpret_cast<uint32_t*>(s_win_dyn);
-    WinRing* s_ring   = reinterpret_cast<WinRing*>(s_win_dyn + kWinTables);
+    WinRing* s_ring   = reinterpret_cast<WinRing*>(s_win_dyn + WinShape<SECOND>::kTables);
     if (!a.tree_info || a.tree_info[2] > (uint32_t)kWinMaxLen) return;  // uniform: k_huff_decode_idx's trees
-    win_tables(a, s_table);
+    win_tables<SECOND>(a, s_table);
     if (*a.status != VSZ_OK) return;  // no block barrier below
-    decode_win_lane(a, blockIdx.x * (size_t)blockDim.x + threadIdx.x, s_table, s_table + (1 << kDecBits), s_ring);
+    decode_win_lane<SECOND>(a, blockIdx.x * (size_t)blockDim.x + threadIdx.x, s_table, s_table + (1 << kDecBits), s_ring);
 }
 
 constexpr int kDecRound = 16;                 // codes per lane staged before the coalesced store
@@ -1388,17 +1399,19 @@ __global__ void __launch_bounds__(256) k_huff_decode_idx(HuffDecodeArgs a) {
 // ---- many fields: tasks of (field, chunk range [256 k, 256 k + 256) of its index), one CTA
 // each; lane t of the CTA decodes chunk u0 + t.  A kernel takes the tasks of the fields whose trees
 // are of its kind (read from k_huff_table's results, so uniform over the CTA) and skips the rest.
-__global__ void __launch_bounds__(kWinBatchThreads, kWinBatchBlocks)
+template <bool SECOND>
+__global__ void __launch_bounds__(WinShape<SECOND>::kBatchThreads, WinShape<SECOND>::kBatchBlocks)
     k_huff_decode_win_batch(const HuffDecodeArgs* __restrict__ args, const BatchTask* __restrict__ tasks, uint32_t ntasks) {
     extern __shared__ __align__(16) uint8_t s_win_dyn[];
     uint32_t* s_table = reinterpret_cast<uint32_t*>(s_win_dyn);
-    WinRing* s_ring = reinterpret_cast<WinRing*>(s_win_dyn + kWinTables);
+    WinRing* s_ring = reinterpret_cast<WinRing*>(s_win_dyn + WinShape<SECOND>::kTables);
     for (uint32_t t = blockIdx.x; t < ntasks; t += gridDim.x) {
         const BatchTask tk     = tasks[t];
         const HuffDecodeArgs a = args[tk.field];
         if (a.tree_info[2] > (uint32_t)kWinMaxLen) continue;
-        win_tables(a, s_table);
-        if (*a.status == VSZ_OK) decode_win_lane(a, tk.u0 + threadIdx.x, s_table, s_table + (1 << kDecBits), s_ring);
+        win_tables<SECOND>(a, s_table);
+        if (*a.status == VSZ_OK)
+            decode_win_lane<SECOND>(a, tk.u0 + threadIdx.x, s_table, s_table + (1 << kDecBits), s_ring);
         __syncthreads();
     }
 }
@@ -1683,7 +1696,8 @@ int launch_huff_table_batch(const HuffTableArgs* args, uint32_t nfields, cudaStr
 }
 
 int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks, uint32_t ntasks,
-                             const BatchTask* const_tasks, uint32_t nconst, bool split, cudaStream_t st, int num_sms) {
+                             const BatchTask* const_tasks, uint32_t nconst, bool split, uint32_t most_nodes,
+                             cudaStream_t st, int num_sms) {
     if (ntasks && split) {
         const uint32_t cap  = (uint32_t)num_sms * kSplitBlocks;
         static std::atomic<unsigned long long> attr{0};
@@ -1692,11 +1706,22 @@ int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks,
                                              split_smem<kSplitS>(kSplitThreads), st>>>(args, tasks, ntasks);
         count_launch();
     } else if (ntasks) {
-        const uint32_t cap  = (uint32_t)num_sms * kWinBatchBlocks;
-        const uint32_t grid = ntasks < cap ? ntasks : cap;
-        static std::atomic<unsigned long long> attr{0};
-        smem_limit_once(k_huff_decode_win_batch, (int)win_smem(kWinBatchThreads), attr);
-        k_huff_decode_win_batch<<<grid, kWinBatchThreads, win_smem(kWinBatchThreads), st>>>(args, tasks, ntasks);
+        static std::atomic<unsigned long long> attr{0}, attr_second{0};
+        uint32_t grid = 0;
+        auto go = [&](auto second_c, std::atomic<unsigned long long>& at) {
+            constexpr bool SECOND = decltype(second_c)::value;
+            using W               = WinShape<SECOND>;
+            const uint32_t cap    = (uint32_t)num_sms * W::kBatchBlocks;
+            grid                  = ntasks < cap ? ntasks : cap;
+            smem_limit_once(k_huff_decode_win_batch<SECOND>, (int)W::smem(W::kBatchThreads), at);
+            k_huff_decode_win_batch<SECOND><<<grid, W::kBatchThreads, W::smem(W::kBatchThreads), st>>>(args, tasks, ntasks);
+        };
+        // without the table one CTA more fits an SM, which takes a second round out of batches of that size
+        // (550 tasks of 1024-symbol trees 213 -> 189 us, 435 142 -> 189, 750 215 -> 292)
+        const bool one_round = ntasks > (uint32_t)num_sms * WinShape<true>::kBatchBlocks &&
+                               ntasks <= (uint32_t)num_sms * WinShape<false>::kBatchBlocks;
+        if (most_nodes > kWinSecondNodes || one_round) go(std::false_type{}, attr);
+        else go(std::true_type{}, attr_second);
         count_launch();
         k_huff_decode_idx_batch<<<grid, 256, 0, st>>>(args, tasks, ntasks);
         count_launch();
@@ -1997,12 +2022,18 @@ int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms) {
         count_launch();
     } else if (indexed) {
         if (a.tree_info) {
-            static std::atomic<unsigned long long> attr_win{0};
-            smem_limit_once(k_huff_decode_win, (int)win_smem(kWinThreads), attr_win);
-            // whole warps over as many SMs as there are, at most kWinThreads to a copy of the tables
-            const size_t per  = (a.nchunks + (size_t)num_sms * kWinMinBlocks - 1) / ((size_t)num_sms * kWinMinBlocks);
-            const int threads = 32 * (int)min((size_t)kWinThreads / 32, max((size_t)2, (per + 31) / 32));
-            k_huff_decode_win<<<(unsigned)((a.nchunks + threads - 1) / threads), threads, win_smem(threads), st>>>(a);
+            static std::atomic<unsigned long long> attr_win{0}, attr_second{0};
+            // whole warps over as many SMs as there are, at most kThreads to a copy of the tables
+            auto go = [&](auto second_c, std::atomic<unsigned long long>& at) {
+                constexpr bool SECOND = decltype(second_c)::value;
+                using W               = WinShape<SECOND>;
+                const size_t per  = (a.nchunks + (size_t)num_sms * W::kBlocks - 1) / ((size_t)num_sms * W::kBlocks);
+                const int threads = 32 * (int)min((size_t)W::kThreads / 32, max((size_t)2, (per + 31) / 32));
+                smem_limit_once(k_huff_decode_win<SECOND>, (int)W::smem(W::kThreads), at);
+                k_huff_decode_win<SECOND><<<(unsigned)((a.nchunks + threads - 1) / threads), threads, W::smem(threads), st>>>(a);
+            };
+            if (a.nodes > kWinSecondNodes) go(std::false_type{}, attr_win);
+            else go(std::true_type{}, attr_second);
             count_launch();
         }
         if (a.walk_smem) {

@@ -170,7 +170,8 @@ struct DLayout {
     unsigned long long* scan_status[2];  // index scan, zero scan
     uint32_t* scan_counter[2];
     size_t cleared;
-    bool split;  // fields are decoded by the split decoder
+    uint32_t most_nodes;  // the largest tree's
+    bool split;           // fields are decoded by the split decoder
     std::vector<uint32_t*> table, table2, win, child, node_sym, parent, walk, redo;
     std::vector<uint16_t*> code;
     std::vector<size_t> chunk_base;
@@ -187,13 +188,12 @@ DLayout layout_dbatch(const std::vector<DField>& fs, uint8_t* base, size_t cap) 
     L.ctl          = b.take<uint8_t>(nf * kDCtlBytes + 256);
     L.batch_status = reinterpret_cast<int*>(L.ctl ? L.ctl + nf * kDCtlBytes : nullptr);
     size_t T = 0;
-    uint32_t nodes = 0;
     for (const auto& f : fs) {
         L.chunk_base.push_back(T);
         T += f.nch;
-        nodes = std::max(nodes, f.nodes);
+        L.most_nodes = std::max(L.most_nodes, f.nodes);
     }
-    L.split = huff_split_batch(T, nodes);
+    L.split = huff_split_batch(T, L.most_nodes);
     for (int k = 0; k < 2; k++) {
         L.scan_status[k]  = b.take<unsigned long long>(scan_tmp_tiles(T) + 1);
         L.scan_counter[k] = b.take<uint32_t>(4);
@@ -277,6 +277,7 @@ struct vsz_dbatch {
     const BatchTask* tasks = nullptr;
     uint32_t idx_off = 0, idx_n = 0, dec_off = 0, dec_n = 0, const_off = 0, const_n = 0, out_off = 0, out_n = 0;
     uint32_t redo_off = 0, redo_n = 0;
+    uint32_t most_nodes = 0;
     bool split = false;
     std::vector<DqClass> classes;       // a launch each, or
     uint32_t small_off = 0, small_n = 0;  // one for all
@@ -406,6 +407,7 @@ vsz_status vsz_dbatch_create(const vsz_dbatch_field* fields, int nfields, void* 
     }
     // ---- task lists
     B->total_chunks       = L.chunk_base.empty() ? 0 : L.chunk_base.back() + fs.back().nch;
+    B->most_nodes          = L.most_nodes;
     B->split               = L.split;
     const uint64_t dec_per = L.split ? kSplitTaskChunks : kDecTaskChunks;
     B->idx_off = (uint32_t)tasks.size();
@@ -540,7 +542,7 @@ vsz_status vsz_dbatch_decompress(vsz_dbatch* B, void* stream) {
     {
         StageTimer t(kStHuffDecode, st);
         VSZ_TRY(launch_huff_decode_batch(B->dec, B->tasks + B->dec_off, B->dec_n, B->tasks + B->const_off,
-                                         B->const_n, B->split, st, sms));
+                                         B->const_n, B->split, B->most_nodes, st, sms));
     }
     {
         StageTimer t(kStZeroScan, st);

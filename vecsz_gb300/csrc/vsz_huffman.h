@@ -189,10 +189,11 @@ int launch_huff_table(HuffTableArgs a, cudaStream_t st);
 // index), split (huff_split_batch): all by the split decoder, else 256 chunks each, every field's tree by the
 // decoder of its kind (the window decoder for codewords up to 32 bits, the general one beyond); const_tasks
 // (one-symbol trees) by a constant fill.
+// most_nodes: the largest tree's.
 int launch_huff_table_batch(const HuffTableArgs* args, uint32_t nfields, cudaStream_t st, int num_sms);
 int launch_huff_decode_batch(const HuffDecodeArgs* args, const BatchTask* tasks, uint32_t ntasks,
-                             const BatchTask* const_tasks, uint32_t nconst, bool split, cudaStream_t st,
-                             int num_sms);
+                             const BatchTask* const_tasks, uint32_t nconst, bool split, uint32_t most_nodes,
+                             cudaStream_t st, int num_sms);
 int launch_huff_decode(HuffDecodeArgs a, cudaStream_t st, int num_sms);
 int launch_huff_const(uint16_t* codes, size_t n, const uint32_t* info, const int* status, cudaStream_t st, int num_sms);
 int launch_huff_sync_init(HuffSyncArgs a, cudaStream_t st);
