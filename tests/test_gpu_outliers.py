@@ -67,3 +67,21 @@ def test_without_the_index(cuda, dims, density):
     ref, _ = O.compress(x, dims, 8, 256, 0.5, False)
     y = V.decompress(ref, len(ref), 0, 256, 8)
     np.testing.assert_array_equal(y.view(np.uint32), O.decompress(ref, 8, 256, 0.0).view(np.uint32))
+
+
+@pytest.mark.parametrize("shift", [0, 1, 8])  # codes on a 16-byte boundary, off it, 16 bytes further
+@pytest.mark.parametrize("dims", [(511,), (512,), (513,), (5000,), (64, 40, 24), (37, 65)])
+def test_stage_call(cuda, dims, shift):
+    """vsz_dualquant_decompress: codes that no decoder of this library counted."""
+    from vecsz_gb300 import api
+    n = int(np.prod(dims))
+    rng = np.random.default_rng(n + shift)
+    x = np.where(rng.random(n) < 0.1, rng.integers(1000, 100000, n), rng.integers(-4, 5, n)).astype(np.float32)
+    code, dense = O.dualquant(x, dims, 8, 256, 0.5)
+    outliers = O.gather_outliers(code, dense)
+    consts, _, _ = api.eb_setup(cuda.from_numpy(x).cuda(), 0.5)
+    d_code = cuda.zeros(n + 16, dtype=cuda.int16, device="cuda")[shift: shift + n]
+    d_code.copy_(cuda.from_numpy(code.astype(np.uint16).view(np.int16)))
+    got = api.dualquant_decompress(dims, 8, 256, d_code, cuda.from_numpy(outliers).cuda(), consts)
+    want = O.xlorenzo(code, O.scatter_outliers(code, outliers), dims, 8, 256, 0.5)
+    np.testing.assert_array_equal(got.cpu().numpy().ravel()[:n].view(np.uint32), want.view(np.uint32))

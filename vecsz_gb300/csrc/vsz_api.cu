@@ -915,9 +915,10 @@ vsz_status vsz_dualquant_decompress(int ndim, const size_t dims[3], int block_si
     o.chunk_zero  = chunk_zero;
     o.chunk_off   = chunk_off;
     o.total       = total;
-    VSZ_CUDA(cudaMemsetAsync(status, 0, sizeof(int), S(stream)));
+    // the status and the scan's counter and look-back words at once
+    VSZ_CUDA(cudaMemsetAsync(status, 0, reinterpret_cast<uint8_t*>(chunk_zero) - reinterpret_cast<uint8_t*>(status), S(stream)));
     VSZ_TRY(launch_count_zeros_chunk(d_code, g.n, chunk_zero, S(stream), num_sms()));
-    VSZ_TRY(launch_scan_u32(chunk_zero, chunk_off, nch, tiles, counter, total, status, S(stream)));
+    VSZ_TRY(launch_scan_u32(chunk_zero, chunk_off, nch, tiles, counter, total, status, S(stream), true));
     VSZ_TRY(launch_outlier_scatter(o, S(stream), num_sms()));
     DqDecArgs a{};
     a.codes      = d_code;
